@@ -192,12 +192,25 @@ template <> struct Vec<double> {
   static constexpr int G = 1;
 };
 
+// FP32 vectors hold two lines as (re, re, im, im)
 __device__ __forceinline__ void vsplit(const float4 &v, float2 *a) {
-  a[0] = make_float2(v.x, v.y);
-  a[1] = make_float2(v.z, v.w);
+  a[0] = make_float2(v.x, v.z);
+  a[1] = make_float2(v.y, v.w);
 }
 __device__ __forceinline__ void vsplit(const double2 &v, double2 *a) { a[0] = v; }
-__device__ __forceinline__ float4 vmerge(const float2 *a) { return make_float4(a[0].x, a[0].y, a[1].x, a[1].y); }
+__device__ __forceinline__ float4 vmerge(const float2 *a) { return make_float4(a[0].x, a[1].x, a[0].y, a[1].y); }
+// complex value e (position * lines + line) of a buffer of vectors
+__device__ __forceinline__ float2 line_at(const float4 *b, int e) {
+  const float *p = reinterpret_cast<const float *>(b + (e >> 1)) + (e & 1);
+  return make_float2(p[0], p[2]);
+}
+__device__ __forceinline__ void line_set(float4 *b, int e, float2 v) {
+  float *p = reinterpret_cast<float *>(b + (e >> 1)) + (e & 1);
+  p[0] = v.x;
+  p[2] = v.y;
+}
+__device__ __forceinline__ double2 line_at(const double2 *b, int e) { return b[e]; }
+__device__ __forceinline__ void line_set(double2 *b, int e, double2 v) { b[e] = v; }
 __device__ __forceinline__ double2 vmerge(const double2 *a) { return a[0]; }
 
 struct LineMap {

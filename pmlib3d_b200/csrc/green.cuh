@@ -15,6 +15,11 @@
 
 namespace pmgpu {
 
+// index of (z, row, kx) in an FP64 one-component spectral array (solve.cuh: spec_vec)
+__device__ __forceinline__ size_t green_spec_at(int z, int row, int kx, int rows, int Hp) {
+  return (((size_t)z * (Hp / 4) + kx / 4) * rows + row) * 4 + (kx & 3);
+}
+
 struct GreenParams {
   int M[3];
   int bc[3];
@@ -211,14 +216,18 @@ template <typename R>
 __global__ void k_green2_split(const double2 *__restrict__ spec, int c, int M0, int M1, int M2, int H, int Hp,
                                int gM1, int gM2, double f, const int *__restrict__ yrow,
                                const int *__restrict__ zrow, R *__restrict__ S, R *__restrict__ E) {
-  const size_t total = (size_t)gM2 * gM1 * H;
+  const size_t total = (size_t)gM2 * gM1 * Hp;
   const int Mc = c == 0 ? M0 : (c == 1 ? M1 : M2);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(t % H);
-    const int iy = (int)((t / H) % gM1);
-    const int iz = (int)(t / ((size_t)H * gM1));
+    const int kx = (int)(t % Hp);
+    const int iy = (int)((t / Hp) % gM1);
+    const int iz = (int)(t / ((size_t)Hp * gM1));
+    if (kx >= H) {
+      S[t] = R(0);
+      continue;
+    }
     const int kc = c == 0 ? kx : (c == 1 ? iy : iz);
-    const double2 v = spec[((size_t)zrow[iz] * M1 + yrow[iy]) * Hp + kx];
+    const double2 v = spec[green_spec_at(zrow[iz], yrow[iy], kx, M1, Hp)];
     S[t] = (2 * kc == Mc) ? R(0) : (R)(v.y * f);
     if (kc == 0) {
       const size_t e = c == 0 ? (size_t)iz * gM1 + iy : (c == 1 ? (size_t)iz * H + kx : (size_t)iy * H + kx);
@@ -229,7 +238,7 @@ __global__ void k_green2_split(const double2 *__restrict__ spec, int c, int M0, 
 
 // The spectral kernel of the periodic-periodic-free validation program
 // (validation/poisson_ppf/sources/poisson/poisson_setup_ppf.f:160-486): written into
-// the y-transformed spectrum layout spec[z][row][kx] (kx < Hp, zero from H on; row ->
+// the y-transformed spectrum layout (z, row, kx) (kx < Hp, zero from H on; row ->
 // ky through yk, natural order when null) at the shifted z positions, so that a
 // transform along z alone completes it.  Its x and y axes hold the wavenumbers
 // (natural order) of the periodic axes; the value is the regularised 1-D Green's
@@ -284,7 +293,7 @@ __global__ void k_green_ppf(GreenParams gp, int H, int Hp, const int *__restrict
         }
       }
     }
-    spec[t] = make_double2(g, 0.0);
+    spec[green_spec_at(z, row, kx, gp.M[1], Hp)] = make_double2(g, 0.0);
   }
 }
 
@@ -377,21 +386,36 @@ __global__ void k_green_pff(GreenParams gp, int kx0, int H, int Hp, double2 *__r
         else if (zarg < 500.0) g = c_1_2pi * dev_bessel_k0(zarg) / gp.dx[0];
       }
     }
-    spec[t] = make_double2(g, 0.0);
+    spec[green_spec_at(z, y, kx, gp.M[1], Hp)] = make_double2(g, 0.0);
   }
 }
 
-// octant of the real spectrum, scaled by dx dy dz / (Mx My Mz), in the plan precision;
-// yrow / zrow: frequency -> row of the transformed spectrum along y / z
+// the multiplier of all-periodic grids, 1 / (4 pi^2 k^2 Mx My Mz) and zero at k = 0, on the
+// octant of |k| (rows of Hp, zero from kx = H on)
+template <typename R>
+__global__ void k_green_periodic(int M0, int M1, int M2, double dx, double dy, double dz, int H, int Hp, int gM1,
+                                 int gM2, R *__restrict__ out) {
+  const size_t total = (size_t)gM2 * gM1 * Hp;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    const int i = (int)(t % Hp), j = (int)((t / Hp) % gM1), k = (int)(t / ((size_t)Hp * gM1));
+    const double kx = i / (M0 * dx), ky = j / (M1 * dy), kz = k / (M2 * dz);
+    const double k2 = kx * kx + ky * ky + kz * kz, c = 4.0 * 3.14159265358979323846 * 3.14159265358979323846;
+    out[t] = i < H && k2 > 0.0 ? (R)(1.0 / (c * k2 * M0 * M1 * M2)) : R(0);
+  }
+}
+
+// octant of the real spectrum, scaled by dx dy dz / (Mx My Mz), in the plan precision, in
+// rows of Hp (zero from kx = H on); yrow / zrow: frequency -> row of the transformed
+// spectrum along y / z
 template <typename R>
 __global__ void k_green_octant(const double2 *__restrict__ spec, int M1, int H, int Hp, int gM1, int gM2, double f,
                                const int *__restrict__ yrow, const int *__restrict__ zrow, R *__restrict__ out) {
-  const size_t total = (size_t)gM2 * gM1 * H;
+  const size_t total = (size_t)gM2 * gM1 * Hp;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(t % H);
-    const int iy = (int)((t / H) % gM1);
-    const int iz = (int)(t / ((size_t)H * gM1));
-    out[t] = (R)(spec[((size_t)zrow[iz] * M1 + yrow[iy]) * Hp + kx].x * f);
+    const int kx = (int)(t % Hp);
+    const int iy = (int)((t / Hp) % gM1);
+    const int iz = (int)(t / ((size_t)Hp * gM1));
+    out[t] = kx < H ? (R)(spec[green_spec_at(zrow[iz], yrow[iy], kx, M1, Hp)].x * f) : R(0);
   }
 }
 

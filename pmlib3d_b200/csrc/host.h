@@ -43,13 +43,18 @@ int smem_attr(const void *func, size_t bytes, const char *caller);
 // shared-memory budget of one persistent pass CTA
 constexpr size_t PASS_SMEM_BUDGET = 220 * 1024;
 
+// shared memory of a line-pass CTA with four and with two CTAs on an SM (228 KB an SM, of
+// which 1 KB a CTA is the system's)
+constexpr size_t LINE_SMEM_4 = 56 * 1024;
+constexpr size_t LINE_SMEM_2 = 113 * 1024;
+
 static inline size_t tw_bytes(int ntw, size_t csize) { return (size_t)((ntw + 7) & ~7) * csize; }
 
-// kx tile of the Stockham y / z passes: the largest of 8, 4, 2, 1 whose three
-// buffers fit (FP32 needs an even line count: two lines per 16-byte vector)
+// kx tile of the Stockham y / z passes: the largest of 8 (FP32), 4, 2, 1 (FP64) whose
+// three buffers fit (FP32 vectors hold two neighbouring kx)
 static inline int pick_tk(int n, int nc, size_t csize, int ntw) {
-  for (int tk = 8; tk >= 1; tk /= 2) {
-    if (csize == 8 && (nc * tk) % 2) continue;
+  for (int tk = csize == 8 ? 8 : 4; tk >= 1; tk /= 2) {  // within a kx block
+    if (csize == 8 && tk % 2) continue;
     if (tw_bytes(ntw, csize) + 3 * (size_t)nc * tk * n * csize <= PASS_SMEM_BUDGET) return tk;
   }
   return 0;
@@ -57,44 +62,19 @@ static inline int pick_tk(int n, int nc, size_t csize, int ntw) {
 static inline size_t lines_smem(int n, int nc, int tk, size_t csize, int ntw) {
   return tw_bytes(ntw, csize) + 3 * (size_t)nc * tk * n * csize;
 }
-// register engine: twiddles w_m^q + position table + wavenumbers (+ Bluestein chirp
-// and spectrum) + one tile buffer; n = line length, m = transform length (m = n
-// unless Bluestein)
-static inline size_t reg_smem(int n, int m, int nc, int tk, size_t csize) {
-  const size_t blue = m != n ? (((size_t)(n + m) * csize + 15) & ~(size_t)15) : 0;
-  return (((size_t)m * csize + 15) & ~(size_t)15) + (((size_t)n * 4 + 15) & ~(size_t)15) +
-         (((size_t)n * csize / 2 + 15) & ~(size_t)15) + blue + (size_t)nc * tk * m * csize;
+// shared memory of a line pass: the plan's tables and one tile of TK kx lines of nc
+// components (FP32: 16-byte vectors of two lines, or single lines for TK = 1)
+static inline size_t line_smem(const LinePlan &p, int nc, int tk, size_t rsize) {
+  const size_t csize = 2 * rsize, w = rsize == 4 && tk > 1 ? 16 : csize;
+  return line_tab_bytes(p, w, csize) + (size_t)nc * tk * plan_points(p) * csize;
 }
-// shared memory per CTA that lets the register-engine kernels run as many CTAs per
-// SM as their register budget allows (FP32: 3, FP64: 2; 228 KB per SM)
-static inline size_t reg_budget(size_t rsize) { return rsize == 4 ? (size_t)74 * 1024 : (size_t)112 * 1024; }
-// the wide-radix FP32 kernels run two CTAs per SM
-static inline size_t reg_budget_wide() { return (size_t)112 * 1024; }
-// kx tile of the register engine: within the budget if possible, else one CTA per SM
-static inline int pick_tk_reg(int n, int m, int nc, size_t csize, int Hp, size_t budget1) {
-  for (size_t budget : {budget1, PASS_SMEM_BUDGET})
-    for (int tk = 8; tk >= 1; tk /= 2) {
-      if (Hp % tk) continue;
-      if (reg_smem(n, m, nc, tk, csize) <= budget) return tk;
-    }
-  return 0;
-}
-// rows per tile of the register-engine x passes (table bytes + staging + buffer),
-// two CTAs per SM if possible
-static inline size_t rx_smem(int N, int m, int H, int P0, int Hp, int nc, int rb, size_t csize, size_t rsize,
-                             bool inverse) {
-  const size_t blue = m != N ? (((size_t)(N + m) * csize + 15) & ~(size_t)15) : 0;
-  const size_t tabs = (((size_t)m * csize + 15) & ~(size_t)15) + (((size_t)H * csize + 15) & ~(size_t)15) +
-                      (((size_t)N * 4 + 15) & ~(size_t)15) + blue;
-  const size_t stage = inverse ? (size_t)rb * Hp * nc * csize : (((size_t)rb * P0 * nc * rsize + 15) / 16) * 16;
-  return tabs + stage + (size_t)nc * rb * m * csize;
-}
-static inline int pick_rb_reg(int N, int m, int H, int P0, int Hp, int nc, size_t csize, size_t rsize, bool inverse,
-                              size_t budget1) {
-  for (size_t budget : {budget1, PASS_SMEM_BUDGET})
-    for (int rb = 16; rb >= 1; rb--)
-      if (rx_smem(N, m, H, P0, Hp, nc, rb, csize, rsize, inverse) <= budget) return rb;
-  return 0;
+// shared memory of an x pass of rb rows a tile; pairs: FP32 vectors of two rows
+static inline size_t x_smem(const LinePlan &p, int N, int H, int P0, int nc, int rb, size_t rsize, bool pairs,
+                            bool inverse) {
+  const size_t csize = 2 * rsize, w = pairs ? 16 : csize;
+  const size_t rows = ((size_t)rb * 8 + 15) & ~(size_t)15;
+  const size_t stage = rows + (inverse ? rows : (((size_t)rb * P0 * nc * rsize + 15) & ~(size_t)15));
+  return x_tab_bytes(p, N, H, w, csize) + stage + (size_t)nc * rb * plan_points(p) * csize;
 }
 
 // rows per tile of the x passes
@@ -111,10 +91,13 @@ static inline int pick_rb(int n2, int P0, int Hp, int nc, size_t csize, size_t r
 // y inverse, x inverse) over the tiles of every patch, then the periodic ghost fill
 // per axis.  The descriptors are built on the host once (batch_layout) and live in
 // device memory; a solve passes the patches' arrays by value (BatchIo).
+struct BatchPart {
+  size_t desc_off = 0;  // byte offset of the part's descriptors
+  int npatch = 0, nitems = 0, chunk = 1;
+  size_t smem = 0;
+};
 struct BatchPassInfo {
-  size_t desc_off;  // byte offset of the pass's descriptors
-  int nitems, chunk, wide;
-  size_t smem;
+  BatchPart part[2];  // the patches with a compile-time plan, and the others
 };
 struct BatchGhostInfo {
   size_t desc_off;
@@ -163,8 +146,26 @@ int upload_cs_f32_1(const void *t32, const void *t64);
 int upload_cs_f32_3(const void *t32, const void *t64);
 int upload_cs_f64_1(const void *t32, const void *t64);
 int upload_cs_f64_3(const void *t32, const void *t64);
-int upload_cs_ct_f32(const void *t32, const void *t64);
-int upload_cs_ct_f64(const void *t32, const void *t64);
+int upload_cs_x_f32_3(const void *t32, const void *t64);
+int upload_cs_x_f32_1(const void *t32, const void *t64);
+int upload_cs_x_f32_s(const void *t32, const void *t64);
+int upload_cs_x_f32_b(const void *t32, const void *t64);
+int upload_cs_x_f64(const void *t32, const void *t64);
+int upload_cs_x_f64_b(const void *t32, const void *t64);
+int upload_cs_ct_yf_f32(const void *t32, const void *t64);
+int upload_cs_ct_yi_f32(const void *t32, const void *t64);
+int upload_cs_ct_z_f32(const void *t32, const void *t64);
+int upload_cs_ct_x_f32(const void *t32, const void *t64);
+int upload_cs_ct_yf_f64(const void *t32, const void *t64);
+int upload_cs_ct_yi_f64(const void *t32, const void *t64);
+int upload_cs_ct_z_f64(const void *t32, const void *t64);
+int upload_cs_ct_x_f64(const void *t32, const void *t64);
+int upload_cs_ct_xb_f32(const void *t32, const void *t64);
+int upload_cs_ct_xb_f64(const void *t32, const void *t64);
+int upload_cs_lines_f32(const void *t32, const void *t64);
+int upload_cs_lines_f32b(const void *t32, const void *t64);
+int upload_cs_lines_f64(const void *t32, const void *t64);
+int upload_cs_lines_f64b(const void *t32, const void *t64);
 
 // launches of the y / z line passes take a compile-time-plan kernel when one is
 // compiled for the plan and kx tile (0: always the run-time engine)

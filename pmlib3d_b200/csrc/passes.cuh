@@ -5,6 +5,8 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 
 #include "host.h"
 #include "solve.cuh"
@@ -18,100 +20,206 @@ template <typename K> static int persistent_grid(K kernel, size_t smem, int ntil
 }
 
 
-// kx tile of the register-engine line pass along `axis` within `slack` bytes less
-// than the usual shared-memory budget (0: the pass takes the Stockham path); wide:
-// the plan has a wide composite radix
+// Tile and CTA of a register-engine line pass along `axis`, within `slack` bytes less than
+// the shared memory (tk = 0: the pass takes the Stockham path).
+struct LineShape {
+  int tk, threads;
+};
+// Threads of a CTA with sm bytes of shared memory whose phases have `tasks` work items: the
+// multiple of 32 that keeps the most threads of an SM busy, counting the idle ones of a
+// phase's last round.  An SM holds 512 threads of 128 registers.  Loads pass through the L1
+// that the shared memory leaves, so three or more CTAs share at most 196 KB (256^3, y
+// forward, tiles of 55 KB: four CTAs of 128 threads 409 us, three of 160 298 us).
+static inline int pass_threads(size_t sm, const double *tasks, int n) {
+  const size_t cta = sm + 1024;
+  int most = (int)(196 * 1024 / cta);
+  if (most < 3) most = std::min<int>(2, std::max<int>(1, (int)(228 * 1024 / cta)));
+  int best = 256;
+  double top = 0.0;
+  for (int t = 96; t <= 256; t += 32) {
+    const int ctas = std::min(most, 512 / t);
+    double work = 0.0, spent = 0.0;
+    for (int i = 0; i < n; i++) {
+      work += tasks[i];
+      spent += std::ceil(tasks[i] / t) * t;
+    }
+    const double busy = ctas * t * work / spent;
+    if (busy > top * 1.001) {
+      top = busy;
+      best = t;
+    }
+  }
+  return best;
+}
+// of a line pass of plan pl with lg vectors a position; of an x pass, with its twist
+static inline int line_threads(const LinePlan &pl, int lg, size_t sm, double twist = 0.0) {
+  double tasks[LP_MAX + 1];
+  int n = 0;
+  for (int p = 0; p < pl.np; p++)
+    tasks[n++] = (double)lg * (p == 0 && pl.split ? pl.n : plan_points(pl)) / pl.rad[p];
+  if (twist > 0.0) tasks[n++] = twist;
+  return pass_threads(sm, tasks, n);
+}
 template <typename R, int NC>
-static int rl_pick_tk(const SolveGeom<R> &g, int axis, size_t slack, bool &wide) {
-  typedef typename cplx_t<R>::type C;
-  wide = false;
-  if (!(axis == 1 ? g.ry_ok : g.rz_ok)) return 0;
-  const int n = g.M[axis];
-  const RegPlan &rp = axis == 1 ? g.ry : g.rz;
-  const int mt = rp.n;  // transform length (Bluestein: > n)
-  for (int p = 0; p < rp.np; p++) wide = wide || reg_radix_wide(rp.rad[p]);
-  const size_t budget = (wide ? reg_budget_wide() : reg_budget(sizeof(R))) - slack;
-  int TK = axis == 1 ? g.tky : g.tkz;  // a tuned tile, if it fits
-  if (TK <= 0 || g.Hp % TK || reg_smem(n, mt, NC, TK, sizeof(C)) > PASS_SMEM_BUDGET - slack)
-    TK = pick_tk_reg(n, mt, NC, sizeof(C), g.Hp, budget);
-  if (TK > 0 && reg_smem(n, mt, NC, TK, sizeof(C)) > PASS_SMEM_BUDGET - slack) TK = 0;
-  return TK;
+static LineShape line_shape(const SolveGeom<R> &g, int axis, size_t slack) {
+  if (!(axis == 1 ? g.ry_ok : g.rz_ok)) return LineShape{0, 0};
+  const LinePlan &pl = axis == 1 ? g.ly : g.lz;
+  const int tuned = axis == 1 ? g.tky : g.tkz;
+  const int top = spec_block<R>();  // tiles lie within a kx block
+  auto bytes = [&](int tk) { return line_smem(pl, NC, tk, sizeof(R)) + slack; };
+  auto shape = [&](int tk) {
+    const int lg = NC * tk / (sizeof(R) == 4 && tk > 1 ? 2 : 1);
+    return LineShape{tk, line_threads(pl, lg, bytes(tk))};
+  };
+  if (tuned > 0 && tuned <= top && bytes(tuned) <= PASS_SMEM_BUDGET) return shape(tuned);
+  // the whole block (rows of 192 bytes) for short lines, Bluestein and the z pass, which spend
+  // their time on the transforms; half of it (three CTAs an SM) for longer y lines
+  const size_t whole = (axis == 2 || pl.bl) && slack == 0 ? LINE_SMEM_2 : LINE_SMEM_4;
+  if (bytes(top) <= whole) return shape(top);
+  for (size_t budget : {LINE_SMEM_2, PASS_SMEM_BUDGET})
+    if (bytes(top / 2) <= budget) return shape(top / 2);
+  for (int tk = top / 4; tk >= 1; tk /= 2)
+    if (bytes(tk) <= PASS_SMEM_BUDGET) return shape(tk);
+  return LineShape{0, 0};
 }
 
-// a line-pass kernel (k_rlines and its compile-time-plan instances)
+// a line-pass kernel (k_rlines); pairs: FP32 tiles of two lines a vector.  Defined in
+// the lines_*.cu units.
 template <typename R>
 using LinesKernel = void (*)(SolveGeom<R>, LineTiles, const typename cplx_t<R>::type *, typename cplx_t<R>::type *,
-                             int, int, int, int, int);
-// the compile-time-plan kernel of 3-component lines for plan rp and kx tile TK
-// (nullptr: none compiled); defined in passes_ct_*.cu
-LinesKernel<float> ct_lines_f32(const RegPlan &rp, int TK);
-LinesKernel<double> ct_lines_f64(const RegPlan &rp, int TK);
-// x passes (k_rxfwd / k_rxinv and their compile-time-plan instances)
+                             int, int, int, int, int, int);
+template <typename R> LinesKernel<R> lines_kernel(bool pairs);
+template <> LinesKernel<float> lines_kernel<float>(bool pairs);
+template <> LinesKernel<double> lines_kernel<double>(bool pairs);
+// the compile-time kernel of plan pl with lg vectors a position (k_rlines_ct), nullptr if
+// there is none; passes_ct_*.cu
+template <typename R> LinesKernel<R> lines_kernel_ct(int lmode, const LinePlan &pl, int lg);
+template <> LinesKernel<float> lines_kernel_ct<float>(int, const LinePlan &, int);
+template <> LinesKernel<double> lines_kernel_ct<double>(int, const LinePlan &, int);
+// the batched line-pass kernel (k_lines_batch)
+template <typename R> using LinesBatchKernel = void (*)(BatchWork, int, int, int);
+template <typename R> LinesBatchKernel<R> lines_batch_kernel();
+// batched kernels over the compile-time plans, and whether a plan is one of them
+typedef void (*LinesBatchCt)(BatchWork);
+template <typename R> LinesBatchCt lines_batch_ct(int lmode);
+template <> LinesBatchCt lines_batch_ct<float>(int);
+template <> LinesBatchCt lines_batch_ct<double>(int);
+template <> LinesBatchKernel<float> lines_batch_kernel<float>();
+template <> LinesBatchKernel<double> lines_batch_kernel<double>();
+// x-pass kernels (k_rxfwd, k_rxinv and their batched forms); pairs: FP32 vectors of two
+// rows.  Defined in the passes_x*.cu units.
 template <typename R>
 using RxfKernel = void (*)(SolveGeom<R>, const R *, typename cplx_t<R>::type *, int, int, int, FastDiv);
 template <typename R>
 using RxiKernel = void (*)(SolveGeom<R>, const typename cplx_t<R>::type *, R *, int, int, FastDiv);
-// the compile-time-plan x passes of 3-component fields for plan rp, rows per tile RB,
-// real row length P0 and spectrum pitch Hp (nullptr: none compiled); passes_ct_*.cu
-RxfKernel<float> ct_rxfwd_f32(const RegPlan &rp, int RB, int P0, int Hp);
-RxiKernel<float> ct_rxinv_f32(const RegPlan &rp, int RB, int P0, int Hp);
-RxfKernel<double> ct_rxfwd_f64(const RegPlan &rp, int RB, int P0, int Hp);
-RxiKernel<double> ct_rxinv_f64(const RegPlan &rp, int RB, int P0, int Hp);
+using RxBatchKernel = void (*)(BatchWork, BatchIo);
+template <typename R, int NC> RxfKernel<R> rxfwd_kernel(bool pairs);
+template <typename R, int NC> RxiKernel<R> rxinv_kernel(bool pairs);
+template <> RxfKernel<float> rxfwd_kernel<float, 1>(bool);
+template <> RxfKernel<float> rxfwd_kernel<float, 3>(bool);
+template <> RxfKernel<double> rxfwd_kernel<double, 1>(bool);
+template <> RxfKernel<double> rxfwd_kernel<double, 3>(bool);
+template <> RxiKernel<float> rxinv_kernel<float, 1>(bool);
+template <> RxiKernel<float> rxinv_kernel<float, 3>(bool);
+template <> RxiKernel<double> rxinv_kernel<double, 1>(bool);
+template <> RxiKernel<double> rxinv_kernel<double, 3>(bool);
+// compile-time kernels of 3-component x passes with lg vectors a point (nullptr: none)
+template <typename R> RxfKernel<R> rxfwd_kernel_ct(const LinePlan &pl, int lg);
+template <typename R> RxiKernel<R> rxinv_kernel_ct(const LinePlan &pl, int lg);
+template <> RxfKernel<float> rxfwd_kernel_ct<float>(const LinePlan &, int);
+template <> RxfKernel<double> rxfwd_kernel_ct<double>(const LinePlan &, int);
+template <> RxiKernel<float> rxinv_kernel_ct<float>(const LinePlan &, int);
+template <> RxiKernel<double> rxinv_kernel_ct<double>(const LinePlan &, int);
+template <typename R> RxBatchKernel rx_batch_kernel(bool inverse);
+template <typename R> RxBatchKernel rx_batch_ct(bool inverse);
+template <> RxBatchKernel rx_batch_ct<float>(bool);
+template <> RxBatchKernel rx_batch_ct<double>(bool);
+template <> RxBatchKernel rx_batch_kernel<float>(bool);
+template <> RxBatchKernel rx_batch_kernel<double>(bool);
+
+// Rows of a tile and CTA of a register-engine x pass (rb = 0: the Stockham path): at most
+// 12 vectors a point (as the line tiles), four CTAs of 128 threads an SM if the tile
+// fits, else two of 256, else one; single FP32 rows when no pair of rows fits.
+struct XShape {
+  int rb, threads;
+  bool pairs;
+};
+template <typename R, int NC> static XShape x_shape(const SolveGeom<R> &g, bool inverse, size_t slack) {
+  if (!g.rx_ok) return XShape{0, 0, false};
+  auto bytes = [&](int rb, bool pairs) {
+    return x_smem(g.lx, g.N2, g.H, g.P[0], NC, rb, sizeof(R), pairs, inverse) + slack;
+  };
+  const bool f32 = sizeof(R) == 4;
+  // rows shorter than those of the compile-time plans: more of them, to fill the CTA
+  const int most = (f32 ? 8 : 4) * (plan_points(g.lx) < 32 ? 4 : 1);
+  for (size_t budget : {LINE_SMEM_4, LINE_SMEM_2, PASS_SMEM_BUDGET})
+    for (int rb = most; rb >= (budget == PASS_SMEM_BUDGET ? (f32 ? 2 : 1) : most / 2); rb /= 2)
+      if (bytes(rb, f32) <= budget)
+        return XShape{rb, line_threads(g.lx, NC * rb / (f32 ? 2 : 1), bytes(rb, f32), (double)g.Hp * NC * rb / (f32 ? 4 : 1)),
+                      f32};
+  if (f32 && bytes(1, false) <= PASS_SMEM_BUDGET) return XShape{1, 256, false};
+  return XShape{0, 0, false};
+}
+
+// the tiles of a line pass over the spectral arrays X (P1 rows a plane) and Y (M1 rows):
+// y forward X -> Y, y inverse Y -> X, and along z (rows_y spectrum rows, rows_out z rows out)
+template <typename R> static LineTiles line_tiles(const SolveGeom<R> &g, int axis, int lmode, int rows_y, int rows_out) {
+  const long long Hp = g.Hp, B = spec_block<R>(), P1 = g.P[1], M1 = g.M[1];
+  LineTiles lt;
+  memset(&lt, 0, sizeof(lt));
+  lt.n = g.M[axis];
+  if (axis == 1) {
+    const bool fwd = lmode == L_FWD;
+    lt.rows_in = fwd ? g.P[1] : g.M[1];
+    lt.rows_out = fwd ? g.M[1] : g.P[1];
+    lt.in_os = (fwd ? P1 : M1) * Hp;
+    lt.out_os = (fwd ? M1 : P1) * Hp;
+    lt.in_kb = (fwd ? P1 : M1) * B;
+    lt.out_kb = (fwd ? M1 : P1) * B;
+    lt.in_rs = lt.out_rs = B;
+    lt.nouter = g.P[2];
+  } else {
+    lt.rows_in = g.P[2];
+    lt.rows_out = rows_out;
+    lt.in_os = lt.out_os = B;
+    lt.in_kb = lt.out_kb = M1 * B;
+    lt.in_rs = lt.out_rs = M1 * Hp;
+    lt.nouter = rows_y;
+    lt.ofast = 1;  // neighbouring tiles are neighbours in memory
+  }
+  return lt;
+}
 
 template <typename R, int NC>
 static int launch_lines(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typename cplx_t<R>::type *out, int axis,
-                        int lmode, int zmode, int reproj, int use_zeta, int rows_in, int rows_out, long long in_os,
-                        long long in_rs, long long out_os, long long out_rs, int nouter, cudaStream_t st,
+                        int lmode, int zmode, int reproj, int use_zeta, const LineTiles &tiles, cudaStream_t st,
                         const char *caller) {
   typedef typename cplx_t<R>::type C;
   const int n = g.M[axis];
-  if (axis == 1 ? g.ry_ok : g.rz_ok) {
-    const RegPlan &rp = axis == 1 ? g.ry : g.rz;
-    const int mt = rp.n;  // transform length (Bluestein: > n)
-    bool wide = false;
-    const int TK = rl_pick_tk<R, NC>(g, axis, 0, wide);
-    if (wide && sizeof(R) != 4) {
-      set_error(caller, "wide radices are FP32 only.");
-      return -1;
+  const LineShape sh = line_shape<R, NC>(g, axis, 0);
+  if (sh.tk > 0) {
+    const LinePlan &pl = axis == 1 ? g.ly : g.lz;
+    const bool pairs = sizeof(R) == 4 && sh.tk > 1;
+    LineTiles lt = tiles;
+    lt.nkt = g.Hp / sh.tk;
+    lt.TK = sh.tk;
+    lt.dLG = make_fastdiv((unsigned)(NC * sh.tk / (pairs ? 2 : 1)));
+    const size_t sm = line_smem(pl, NC, sh.tk, sizeof(R));
+    const int lg = NC * sh.tk / (pairs ? 2 : 1);
+    LinesKernel<R> kern = nullptr;
+    if constexpr (NC == 3) {
+      const bool plain = lmode != L_Z || (zmode == Z_VEL && z_plain(g, use_zeta));
+      if (g_fft_ct && plain && (pairs || sizeof(R) == 8)) kern = lines_kernel_ct<R>(lmode, pl, lg);
     }
-    if (TK > 0) {
-      LineTiles lt;
-      lt.n = n;
-      lt.rows_in = rows_in;
-      lt.rows_out = rows_out;
-      lt.in_os = in_os;
-      lt.in_rs = in_rs;
-      lt.out_os = out_os;
-      lt.out_rs = out_rs;
-      lt.nouter = nouter;
-      lt.nkt = g.Hp / TK;
-      lt.TK = TK;
-      lt.dLG = make_fastdiv((unsigned)(NC * TK / RVec<R>::G));
-      const size_t sm = reg_smem(n, mt, NC, TK, sizeof(C));
-      auto launch = [&](auto kern) -> int {
-        if (smem_attr((const void *)kern, sm, caller)) return -1;
-        int per = 1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, RL_THREADS, sm) != cudaSuccess || per < 1)
-          per = 1;
-        const int grid = std::max(1, std::min(lt.nouter * lt.nkt, per * num_sms()));
-        kern<<<grid, RL_THREADS, sm, st>>>(g, lt, in, out, axis, lmode, zmode, reproj, use_zeta);
-        PM_LAUNCHED();
-        CKL(caller);
-        return 0;
-      };
-      if constexpr (NC == 3) {
-        if (g_fft_ct) {
-          LinesKernel<R> ck;
-          if constexpr (sizeof(R) == 4) ck = ct_lines_f32(rp, TK);
-          else ck = ct_lines_f64(rp, TK);
-          if (ck) return launch(ck);
-        }
-      }
-      if constexpr (sizeof(R) == 4) {
-        if (wide) return launch(k_rlines<R, NC, true>);
-      }
-      return launch(k_rlines<R, NC, false>);
-    }
+    if (!kern) kern = lines_kernel<R>(pairs);
+    if (smem_attr((const void *)kern, sm, caller)) return -1;
+    int per = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, sh.threads, sm) != cudaSuccess || per < 1) per = 1;
+    const int grid = std::max(1, std::min(lt.nouter * lt.nkt, per * num_sms()));
+    kern<<<grid, sh.threads, sm, st>>>(g, lt, in, out, NC, axis, lmode, zmode, reproj, use_zeta);
+    PM_LAUNCHED();
+    CKL(caller);
+    return 0;
   }
   const int ntw = (axis == 1) ? g.fy.ntw : g.fz.ntw;
   const int TK = pick_tk(n, NC, sizeof(C), ntw);
@@ -119,17 +227,10 @@ static int launch_lines(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typ
     set_error(caller, "FFT length too large for the shared-memory transform.");
     return -1;
   }
-  LineTiles lt;
-  lt.n = n;
-  lt.rows_in = rows_in;
-  lt.rows_out = rows_out;
-  lt.in_os = in_os;
-  lt.in_rs = in_rs;
-  lt.out_os = out_os;
-  lt.out_rs = out_rs;
-  lt.nouter = nouter;
+  LineTiles lt = tiles;
   lt.nkt = g.Hp / TK;
   lt.TK = TK;
+  lt.ofast = 0;
   const size_t sm = lines_smem(n, NC, TK, sizeof(C), ntw);
   if (smem_attr((const void *)k_lines<R, NC>, sm, caller)) return -1;
   const int grid = persistent_grid(k_lines<R, NC>, sm, lt.nouter * lt.nkt);
@@ -145,36 +246,31 @@ int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename c
   typedef typename cplx_t<R>::type C;
   const bool vec16r = cs == NC && ((size_t)g.ext[0] * NC * sizeof(R)) % 16 == 0 &&
                       ((size_t)g.off[0] * NC * sizeof(R)) % 16 == 0 && ((size_t)g.P[0] * NC * sizeof(R)) % 16 == 0;
-  if (g.rx_ok) {
-    const int RB = pick_rb_reg(g.N2, g.rx.n, g.H, g.P[0], g.Hp, NC, sizeof(C), sizeof(R), false, reg_budget(sizeof(R)));
-    if (RB > 0) {
-      const size_t sm = rx_smem(g.N2, g.rx.n, g.H, g.P[0], g.Hp, NC, RB, sizeof(C), sizeof(R), false);
-      RxfKernel<R> kern = k_rxfwd<R, NC>;
-      if constexpr (NC == 3) {
-        if (g_fft_ct && !g.rx.bl) {
-          RxfKernel<R> ck;
-          if constexpr (sizeof(R) == 4) ck = ct_rxfwd_f32(g.rx, RB, g.P[0], (int)g.Hp);
-          else ck = ct_rxfwd_f64(g.rx, RB, g.P[0], (int)g.Hp);
-          if (ck) kern = ck;
-        }
-      }
+  const XShape sh = x_shape<R, NC>(g, false, 0);
+  if (sh.rb > 0) {
+    const size_t sm = x_smem(g.lx, g.N2, g.H, g.P[0], NC, sh.rb, sizeof(R), sh.pairs, false);
+    auto launch = [&](auto kern, int G) -> int {
       if (smem_attr((const void *)kern, sm, caller)) return -1;
-      const int rows = g.P[1] * g.P[2];
-      const int ntiles = (rows + RB - 1) / RB;
+      const int ntiles = (g.P[1] * g.P[2] + sh.rb - 1) / sh.rb;
       int per = 1;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, RL_THREADS, sm) != cudaSuccess || per < 1)
-        per = 1;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, sh.threads, sm) != cudaSuccess || per < 1) per = 1;
       const int grid = std::max(1, std::min(ntiles, per * num_sms()));
-      { KTimer kt_(KC_XFWD, st);
-        kern<<<grid, RL_THREADS, sm, st>>>(g, in, X, RB, cs, vec16r ? 1 : 0,
-                                           make_fastdiv((unsigned)(NC * RB / RVec<R>::G))); }
+      KTimer kt_(KC_XFWD, st);
+      kern<<<grid, sh.threads, sm, st>>>(g, in, X, sh.rb, cs, vec16r ? 1 : 0, make_fastdiv((unsigned)(NC * sh.rb / G)));
       PM_LAUNCHED();
       CKL(caller);
-      const long long Hp = g.Hp;
-      KTimer kt_(KC_YFWD, st);
-      return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, g.P[1], g.M[1], (long long)g.P[1] * Hp, Hp,
-                                 (long long)g.M[1] * Hp, Hp, g.P[2], st, caller);
+      return 0;
+    };
+    auto kern = rxfwd_kernel<R, NC>(sh.pairs);
+    if constexpr (NC == 3) {
+      if (g_fft_ct && (sh.pairs || sizeof(R) == 8)) {
+        const auto ck = rxfwd_kernel_ct<R>(g.lx, NC * sh.rb / (sh.pairs ? 2 : 1));
+        if (ck) kern = ck;
+      }
     }
+    if (launch(kern, sh.pairs ? 2 : 1)) return -1;
+    KTimer kt_(KC_YFWD, st);
+    return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, line_tiles(g, 1, L_FWD, 0, 0), st, caller);
   }
   const int ntwx = g.fx.ntw + g.fx.next;
   const int RB = pick_rb(g.N2, g.P[0], g.Hp, NC, sizeof(C), sizeof(R), ntwx, false);
@@ -193,69 +289,63 @@ int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename c
     k_xfwd<R, NC><<<persistent_grid(k_xfwd<R, NC>, sm, ntiles), PASS_THREADS, sm, st>>>(g, in, X, RB, cs, vec16 ? 1 : 0); }
   PM_LAUNCHED();
   CKL(caller);
-  const long long Hp = g.Hp;
   KTimer kt_(KC_YFWD, st);
-  return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, g.P[1], g.M[1], (long long)g.P[1] * Hp, Hp,
-                             (long long)g.M[1] * Hp, Hp, g.P[2], st, caller);
+  return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, line_tiles(g, 1, L_FWD, 0, 0), st, caller);
 }
 
 // one forward (or inverse) pass along y over the X layout -> Y layout, as in fwd_xy
 template <typename R, int NC>
 int ypass(SolveGeom<R> &g, const typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y, int inverse,
           cudaStream_t st, const char *caller) {
-  const long long Hp = g.Hp;
   if (inverse)
-    return launch_lines<R, NC>(g, Y, (typename cplx_t<R>::type *)X, 1, L_INV, 0, 0, 0, g.M[1], g.P[1],
-                               (long long)g.M[1] * Hp, Hp, (long long)g.P[1] * Hp, Hp, g.P[2], st, caller);
-  return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, g.P[1], g.M[1], (long long)g.P[1] * Hp, Hp,
-                             (long long)g.M[1] * Hp, Hp, g.P[2], st, caller);
+    return launch_lines<R, NC>(g, Y, (typename cplx_t<R>::type *)X, 1, L_INV, 0, 0, 0, line_tiles(g, 1, L_INV, 0, 0), st,
+                               caller);
+  return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, line_tiles(g, 1, L_FWD, 0, 0), st, caller);
 }
 
 template <typename R, int NC>
 int zpass(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typename cplx_t<R>::type *out, int mode,
                  int reproj, int use_zeta, int rows_y, cudaStream_t st, const char *caller) {
-  const long long Hp = g.Hp;
   // Z_FORWARD: forward transform only, P rows in (the rest zero), M rows out
-  const int rows_in = g.P[2], rows_out = (mode == Z_FORWARD) ? g.M[2] : g.P[2];
+  const int rows_out = (mode == Z_FORWARD) ? g.M[2] : g.P[2];
   KTimer kt_(KC_ZPASS, st);
-  return launch_lines<R, NC>(g, in, out, 2, mode == Z_FORWARD ? L_FWD : L_Z, mode, reproj, use_zeta, rows_in,
-                             rows_out, Hp, (long long)g.M[1] * Hp, Hp, (long long)g.M[1] * Hp, rows_y, st, caller);
+  return launch_lines<R, NC>(g, in, out, 2, mode == Z_FORWARD ? L_FWD : L_Z, mode, reproj, use_zeta,
+                             line_tiles(g, 2, L_Z, rows_y, rows_out), st, caller);
 }
 
 template <typename R, int NC>
 int inv_yx(SolveGeom<R> &g, const pmgpu_topo *topo, typename cplx_t<R>::type *Y,
            typename cplx_t<R>::type *X, R *out, cudaStream_t st, const char *caller, int cs, bool ghosts) {
   typedef typename cplx_t<R>::type C;
-  const long long Hp = g.Hp;
   {
     KTimer kt_(KC_YINV, st);
-    if (launch_lines<R, NC>(g, Y, X, 1, L_INV, 0, 0, 0, g.M[1], g.P[1], (long long)g.M[1] * Hp, Hp,
-                            (long long)g.P[1] * Hp, Hp, g.P[2], st, caller))
+    if (launch_lines<R, NC>(g, Y, X, 1, L_INV, 0, 0, 0, line_tiles(g, 1, L_INV, 0, 0), st, caller))
       return -1;
   }
   const int rows = g.P[1] * g.P[2];
-  const int RBr = g.rx_ok ? pick_rb_reg(g.N2, g.rx.n, g.H, g.P[0], g.Hp, NC, sizeof(C), sizeof(R), true, reg_budget(sizeof(R))) : 0;
-  if (RBr > 0) {
-    const size_t sm = rx_smem(g.N2, g.rx.n, g.H, g.P[0], g.Hp, NC, RBr, sizeof(C), sizeof(R), true);
-    RxiKernel<R> kern = k_rxinv<R, NC>;
+  const XShape sh = x_shape<R, NC>(g, true, 0);
+  if (sh.rb > 0) {
+    const size_t sm = x_smem(g.lx, g.N2, g.H, g.P[0], NC, sh.rb, sizeof(R), sh.pairs, true);
+    auto launch = [&](auto kern, int G) -> int {
+      if (smem_attr((const void *)kern, sm, caller)) return -1;
+      const int ntiles = (rows + sh.rb - 1) / sh.rb;
+      int per = 1;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, sh.threads, sm) != cudaSuccess || per < 1) per = 1;
+      const int grid = std::max(1, std::min(ntiles, per * num_sms()));
+      KTimer kt_(KC_XINV, st);
+      kern<<<grid, sh.threads, sm, st>>>(g, X, out, sh.rb, cs, make_fastdiv((unsigned)(NC * sh.rb / G)));
+      PM_LAUNCHED();
+      CKL(caller);
+      return 0;
+    };
+    auto kern = rxinv_kernel<R, NC>(sh.pairs);
     if constexpr (NC == 3) {
-      if (g_fft_ct && !g.rx.bl) {
-        RxiKernel<R> ck;
-        if constexpr (sizeof(R) == 4) ck = ct_rxinv_f32(g.rx, RBr, g.P[0], (int)g.Hp);
-        else ck = ct_rxinv_f64(g.rx, RBr, g.P[0], (int)g.Hp);
+      if (g_fft_ct && (sh.pairs || sizeof(R) == 8)) {
+        const auto ck = rxinv_kernel_ct<R>(g.lx, NC * sh.rb / (sh.pairs ? 2 : 1));
         if (ck) kern = ck;
       }
     }
-    if (smem_attr((const void *)kern, sm, caller)) return -1;
-    const int ntiles = (rows + RBr - 1) / RBr;
-    int per = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, RL_THREADS, sm) != cudaSuccess || per < 1)
-      per = 1;
-    const int grid = std::max(1, std::min(ntiles, per * num_sms()));
-    { KTimer kt_(KC_XINV, st);
-      kern<<<grid, RL_THREADS, sm, st>>>(g, X, out, RBr, cs, make_fastdiv((unsigned)(NC * RBr / RVec<R>::G))); }
-    PM_LAUNCHED();
-    CKL(caller);
+    if (launch(kern, sh.pairs ? 2 : 1)) return -1;
   } else {
     const int ntwx = g.fx.ntw + g.fx.next;
     const int RB = pick_rb(g.N2, g.P[0], g.Hp, NC, sizeof(C), sizeof(R), ntwx, true);
@@ -302,89 +392,66 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
   if (n <= 0 || n > BATCH_MAX) return -1;
   lay = BatchLayout();
   lay.npatch = n;
-  std::vector<PassDesc<R>> d[5];
-  for (int f = 0; f < 5; f++) {
-    d[f].resize(n);
-    memset(d[f].data(), 0, sizeof(PassDesc<R>) * n);
-    lay.pass[f].nitems = 0;
-    lay.pass[f].smem = 0;
-    lay.pass[f].wide = 0;
-  }
+  std::vector<PassDesc<R>> d[5][2];  // by pass family and part
+  // the descriptor of patch i in family f: in the part of its plan
+  auto add = [&](int f, int i, int cls, size_t smem, PassDesc<R> &q) {
+    const int part = cls ? 0 : 1;
+    BatchPart &bp = lay.pass[f].part[part];
+    q.patch = i;
+    q.cls = cls;
+    q.first = bp.nitems;
+    bp.nitems += q.ntiles;
+    bp.npatch++;
+    bp.smem = std::max(bp.smem, smem);
+    d[f][part].push_back(q);
+  };
   std::vector<GhostDesc> gd[3];
   for (int i = 0; i < n; i++) {
     const SolveGeom<R> &gi = g[i];
     if (!gi.rx_ok || !gi.ry_ok || !gi.rz_ok) return -1;
-    const long long Hp = gi.Hp;
     // x forward and x inverse (rows per tile as the single-plan passes, within the slack)
     for (int inv = 0; inv < 2; inv++) {
       const int f = inv ? 4 : 0;
-      const int RB = pick_rb_reg(gi.N2, gi.rx.n, gi.H, gi.P[0], gi.Hp, NC, sizeof(C), sizeof(R), inv != 0,
-                                 reg_budget(sizeof(R)) - BATCH_SMEM_SLACK);
-      if (RB <= 0) return -1;
-      const size_t sm = rx_smem(gi.N2, gi.rx.n, gi.H, gi.P[0], gi.Hp, NC, RB, sizeof(C), sizeof(R), inv != 0);
-      if (sm > PASS_SMEM_BUDGET - BATCH_SMEM_SLACK) return -1;
-      PassDesc<R> &q = d[f][i];
+      const XShape sh = x_shape<R, NC>(gi, inv != 0, BATCH_SMEM_SLACK);
+      if (sh.rb <= 0 || sh.pairs != (sizeof(R) == 4)) return -1;
+      const int RB = sh.rb;
+      const size_t sm = x_smem(gi.lx, gi.N2, gi.H, gi.P[0], NC, RB, sizeof(R), sh.pairs, inv != 0);
+      PassDesc<R> q;
+      memset(&q, 0, sizeof(q));
       q.g = gi;
       q.RB = RB;
       q.cs = NC;
       q.vec16 = ((size_t)gi.ext[0] * NC * sizeof(R)) % 16 == 0 && ((size_t)gi.off[0] * NC * sizeof(R)) % 16 == 0 &&
                 ((size_t)gi.P[0] * NC * sizeof(R)) % 16 == 0;
-      q.dLG = make_fastdiv((unsigned)(NC * RB / RVec<R>::G));
+      q.dLG = make_fastdiv((unsigned)(NC * RB / (sizeof(R) == 4 ? 2 : 1)));
       q.in = inv ? X[i] : nullptr;   // x forward reads the caller's vorticity
       q.out = inv ? nullptr : X[i];  // x inverse writes the caller's velocity
       q.ntiles = (gi.P[1] * gi.P[2] + RB - 1) / RB;
-      q.first = lay.pass[f].nitems;
-      lay.pass[f].nitems += q.ntiles;
-      lay.pass[f].smem = std::max(lay.pass[f].smem, sm);
+      const int lg = NC * RB / (sizeof(R) == 4 ? 2 : 1);
+      const bool ct = g_fft_ct && (inv ? rxinv_kernel_ct<R>(gi.lx, lg) != nullptr : rxfwd_kernel_ct<R>(gi.lx, lg) != nullptr);
+      add(f, i, ct ? plan_class(gi.lx.n, gi.lx.split, lg) : 0, sm, q);
     }
     // y forward, z pass, y inverse (run_solve's launch_lines arguments)
     for (int f = 1; f <= 3; f++) {
       const int axis = f == 2 ? 2 : 1;
-      bool wide = false;
-      const int TK = rl_pick_tk<R, NC>(gi, axis, BATCH_SMEM_SLACK, wide);
-      if (TK <= 0 || (wide && sizeof(R) != 4)) return -1;
-      const RegPlan &rp = axis == 1 ? gi.ry : gi.rz;
-      PassDesc<R> &q = d[f][i];
+      const LineShape sh = line_shape<R, NC>(gi, axis, BATCH_SMEM_SLACK);
+      const int TK = sh.tk;
+      if (TK <= (sizeof(R) == 4 ? 1 : 0)) return -1;
+      const LinePlan &pl = axis == 1 ? gi.ly : gi.lz;
+      PassDesc<R> q;
+      memset(&q, 0, sizeof(q));
       q.g = gi;
       LineTiles &lt = q.lt;
-      lt.n = gi.M[axis];
+      lt = line_tiles(gi, axis, f == 3 ? L_INV : f == 2 ? L_Z : L_FWD, gi.M[1], gi.P[2]);
       lt.TK = TK;
       lt.nkt = gi.Hp / TK;
-      lt.dLG = make_fastdiv((unsigned)(NC * TK / RVec<R>::G));
-      lt.nouter = f == 2 ? gi.M[1] : gi.P[2];
-      if (f == 1) {  // X -> Y
-        lt.rows_in = gi.P[1];
-        lt.rows_out = gi.M[1];
-        lt.in_os = (long long)gi.P[1] * Hp;
-        lt.in_rs = Hp;
-        lt.out_os = (long long)gi.M[1] * Hp;
-        lt.out_rs = Hp;
-        q.in = X[i];
-        q.out = Y[i];
-      } else if (f == 2) {  // Y -> Y, fused multiply
-        lt.rows_in = gi.P[2];
-        lt.rows_out = gi.P[2];
-        lt.in_os = Hp;
-        lt.in_rs = (long long)gi.M[1] * Hp;
-        lt.out_os = Hp;
-        lt.out_rs = (long long)gi.M[1] * Hp;
-        q.in = Y[i];
-        q.out = Y[i];
-      } else {  // Y -> X
-        lt.rows_in = gi.M[1];
-        lt.rows_out = gi.P[1];
-        lt.in_os = (long long)gi.M[1] * Hp;
-        lt.in_rs = Hp;
-        lt.out_os = (long long)gi.P[1] * Hp;
-        lt.out_rs = Hp;
-        q.in = Y[i];
-        q.out = X[i];
-      }
+      lt.dLG = make_fastdiv((unsigned)(NC * TK / (sizeof(R) == 4 ? 2 : 1)));
+      q.in = f == 1 ? X[i] : Y[i];
+      q.out = f == 3 ? X[i] : Y[i];
       q.ntiles = lt.nouter * lt.nkt;
-      q.first = lay.pass[f].nitems;
-      lay.pass[f].nitems += q.ntiles;
-      lay.pass[f].smem = std::max(lay.pass[f].smem, reg_smem(lt.n, rp.n, NC, TK, sizeof(C)));
-      lay.pass[f].wide |= wide ? 1 : 0;
+      const int lmode = f == 3 ? L_INV : f == 2 ? L_Z : L_FWD, lg = NC * TK / (sizeof(R) == 4 ? 2 : 1);
+      const bool ct = g_fft_ct && (f != 2 || z_plain(gi, 0)) && lines_kernel_ct<R>(lmode, pl, lg) != nullptr;
+      add(f, i, ct ? plan_class(pl.n, pl.split, lg) : 0, line_smem(pl, NC, TK, sizeof(R)), q);
     }
     // periodic ghosts of the velocity (x, then y, then z)
     for (int a = 0; a < 3; a++) {
@@ -406,13 +473,15 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
   }
   // chunks of work items: about eight per CTA slot of the GPU
   size_t off = 0;
-  for (int f = 0; f < 5; f++) {
-    lay.pass[f].desc_off = off;
-    off += sizeof(PassDesc<R>) * n;
-    off = (off + 255) & ~(size_t)255;
-    const int slots = num_sms() * 3;
-    lay.pass[f].chunk = std::max(1, std::min(16, lay.pass[f].nitems / (8 * slots)));
-  }
+  for (int f = 0; f < 5; f++)
+    for (int k = 0; k < 2; k++) {
+      BatchPart &bp = lay.pass[f].part[k];
+      bp.desc_off = off;
+      off += sizeof(PassDesc<R>) * bp.npatch;
+      off = (off + 255) & ~(size_t)255;
+      const int slots = num_sms() * 3;
+      bp.chunk = std::max(1, std::min(16, bp.nitems / (8 * slots)));
+    }
   for (int a = 0; a < 3; a++) {
     lay.ghost[a].desc_off = off;
     lay.ghost[a].npatch = (int)gd[a].size();
@@ -421,7 +490,10 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
   }
   lay.bytes = off;
   desc.assign(off, 0);
-  for (int f = 0; f < 5; f++) memcpy(desc.data() + lay.pass[f].desc_off, d[f].data(), sizeof(PassDesc<R>) * n);
+  for (int f = 0; f < 5; f++)
+    for (int k = 0; k < 2; k++)
+      if (!d[f][k].empty())
+        memcpy(desc.data() + lay.pass[f].part[k].desc_off, d[f][k].data(), sizeof(PassDesc<R>) * d[f][k].size());
   for (int a = 0; a < 3; a++)
     if (!gd[a].empty()) memcpy(desc.data() + lay.ghost[a].desc_off, gd[a].data(), sizeof(GhostDesc) * gd[a].size());
   return 0;
@@ -438,40 +510,42 @@ int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters,
     vin.p[i] = vort[i];
     vout.p[i] = vel[i];
   }
-  CK(cudaMemsetAsync(counters, 0, 5 * sizeof(unsigned), st), caller);
+  CK(cudaMemsetAsync(counters, 0, 10 * sizeof(unsigned), st), caller);
   const char *base = reinterpret_cast<const char *>(d_desc);
-  auto work = [&](int f) {
+  // one part of a pass family; a family's patches differ in their phases: four CTAs of 128
+  // threads where they fit
+  auto launch = [&](auto kern, int f, int k, auto... args) -> int {
+    const BatchPart &bp = lay.pass[f].part[k];
+    if (bp.npatch == 0) return 0;
     BatchWork bw;
-    bw.desc = base + lay.pass[f].desc_off;
-    bw.npatch = n;
-    bw.nitems = lay.pass[f].nitems;
-    bw.chunk = lay.pass[f].chunk;
+    bw.desc = base + bp.desc_off;
+    bw.npatch = bp.npatch;
+    bw.nitems = bp.nitems;
+    bw.chunk = bp.chunk;
     bw.pad = 0;
-    bw.counter = counters + f;
-    return bw;
-  };
-  auto launch = [&](auto kern, int f, auto... args) -> int {
-    const size_t sm = lay.pass[f].smem;
-    if (smem_attr((const void *)kern, sm, caller)) return -1;
+    bw.counter = counters + 2 * f + k;
+    const size_t cta = bp.smem + BATCH_SMEM_SLACK + 1024;
+    const int threads = 4 * cta <= 196 * 1024 ? 128 : 3 * cta <= 196 * 1024 ? 160 : 256;
+    if (smem_attr((const void *)kern, bp.smem, caller)) return -1;
     int per = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, RL_THREADS, sm) != cudaSuccess || per < 1) per = 1;
-    const int grid = std::max(1, std::min(lay.pass[f].nitems, per * num_sms()));
-    kern<<<grid, RL_THREADS, sm, st>>>(work(f), args...);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, bp.smem) != cudaSuccess || per < 1) per = 1;
+    const int grid = std::max(1, std::min(bp.nitems, per * num_sms()));
+    kern<<<grid, threads, bp.smem, st>>>(bw, args...);
     PM_LAUNCHED();
     CKL(caller);
     return 0;
   };
   auto lines = [&](int f, int axis, int lmode, int zmode) -> int {
-    if constexpr (sizeof(R) == 4) {
-      if (lay.pass[f].wide) return launch(k_rlines_batch<R, NC, true>, f, axis, lmode, zmode, 0, 0);
-    }
-    return launch(k_rlines_batch<R, NC, false>, f, axis, lmode, zmode, 0, 0);
+    return launch(lines_batch_ct<R>(lmode), f, 0) || launch(lines_batch_kernel<R>(), f, 1, axis, lmode, zmode) ? -1 : 0;
   };
-  { KTimer kt_(KC_XFWD, st); if (launch(k_rxfwd_batch<R, NC>, 0, vin)) return -1; }
+  auto xpass = [&](int f, bool inverse, const BatchIo &io) -> int {
+    return launch(rx_batch_ct<R>(inverse), f, 0, io) || launch(rx_batch_kernel<R>(inverse), f, 1, io) ? -1 : 0;
+  };
+  { KTimer kt_(KC_XFWD, st); if (xpass(0, false, vin)) return -1; }
   { KTimer kt_(KC_YFWD, st); if (lines(1, 1, L_FWD, 0)) return -1; }
   { KTimer kt_(KC_ZPASS, st); if (lines(2, 2, L_Z, Z_VEL)) return -1; }
   { KTimer kt_(KC_YINV, st); if (lines(3, 1, L_INV, 0)) return -1; }
-  { KTimer kt_(KC_XINV, st); if (launch(k_rxinv_batch<R, NC>, 4, vout)) return -1; }
+  { KTimer kt_(KC_XINV, st); if (xpass(4, true, vout)) return -1; }
   for (int a = 0; a < 3; a++) {
     if (lay.ghost[a].npatch == 0) continue;
     const long long total = lay.ghost[a].total;
@@ -485,7 +559,7 @@ int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters,
   return 0;
 }
 
-// copies the DFT constant tables into this unit's constant memory// copies the DFT constant tables into this unit's constant memory
+// copies the DFT constant tables into this unit's constant memory
 static int upload_cs_local(const void *t32, const void *t64) {
   if (cudaMemcpyToSymbol(c_cs32, t32, sizeof(c_cs32)) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_cs64, t64, sizeof(c_cs64)) != cudaSuccess) return -1;

@@ -123,8 +123,18 @@ static int ensure_device(const char *caller) {
       t32[R][m][0] = (float)cosl(a);
       t32[R][m][1] = (float)sinl(a);
     }
-  if (upload_cs_f32_1(t32, t64) || upload_cs_f32_3(t32, t64) || upload_cs_f64_1(t32, t64) ||
-      upload_cs_f64_3(t32, t64) || upload_cs_ct_f32(t32, t64) || upload_cs_ct_f64(t32, t64)) {
+  int (*const up[])(const void *, const void *) = {
+      upload_cs_ct_xb_f32, upload_cs_ct_xb_f64, upload_cs_ct_yf_f32, upload_cs_ct_yi_f32, upload_cs_ct_z_f32, upload_cs_ct_x_f32,
+      upload_cs_ct_yf_f64, upload_cs_ct_yi_f64, upload_cs_ct_z_f64, upload_cs_ct_x_f64,
+      upload_cs_f32_1, upload_cs_f32_3, upload_cs_f64_1,
+      upload_cs_f64_3, upload_cs_x_f32_3, upload_cs_x_f32_1,
+      upload_cs_x_f32_s, upload_cs_x_f32_b, upload_cs_x_f64,
+      upload_cs_x_f64_b, upload_cs_lines_f32, upload_cs_lines_f32b,
+      upload_cs_lines_f64, upload_cs_lines_f64b,
+  };
+  bool sent = true;
+  for (auto f : up) sent = sent && f(t32, t64) == 0;
+  if (!sent) {
     set_error(caller, "could not upload the DFT constant tables.");
     return -1;
   }
@@ -272,132 +282,6 @@ template <typename R> static int upload_tw(const std::vector<cld> &tw, DevBuf &b
   return 0;
 }
 
-// ------------------------------------------------------------------ register-engine plans
-// Factor n into at most three register radices; the score models per-point work
-// (a shared-memory round trip + twiddles per phase, plus the DFT of the radix).
-static double radix_cost(int r) {
-  switch (r) {
-    case 2: return 1.0;
-    case 3: return 1.3;
-    case 4: return 1.1;
-    case 5: return 1.7;
-    case 6: return 1.4;
-    case 7: return 2.3;
-    case 8: return 1.2;
-    case 9: return 1.7;
-    case 10: return 1.6;
-    case 11: return 3.2;
-    case 12: return 1.5;
-    case 13: return 3.6;
-    case 16: return 2.3;  // 16 and 17 exceed the register budget of two vectors a thread: spills
-    case 17: return 5.4;
-    default: return 1e9;
-  }
-}
-
-// a plan from an explicit radix sequence (outermost first)
-static void regplan_from(int n, const int *r, int np, RegPlan &pl) {
-  memset(&pl, 0, sizeof(pl));
-  pl.n = n;
-  pl.np = np;
-  int B = n;
-  for (int p = 0; p < np; p++) {
-    pl.rad[p] = r[p];
-    pl.blk[p] = B;
-    pl.str[p] = B / r[p];
-    pl.twm[p] = n / B;
-    pl.dstr[p] = make_fastdiv((unsigned)pl.str[p]);
-    B /= r[p];
-  }
-}
-
-// radix sequences of at most three register radices whose product is n, best model
-// score first
-struct RadixSeq {
-  int np;
-  int r[3];
-  double cost;
-};
-static std::vector<RadixSeq> regplan_candidates(int n) {
-  static const int S[] = {16, 17, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-  std::vector<RadixSeq> out;
-  auto add = [&](int np, int a, int b, int c) {
-    RadixSeq q;
-    q.np = np;
-    q.r[0] = a;
-    q.r[1] = b;
-    q.r[2] = c;
-    q.cost = 0.0;
-    for (int i = 0; i < np; i++) q.cost += 1.5 + radix_cost(q.r[i]);
-    if (a % 2) q.cost += 0.5;  // the zero half of a padded line is skipped only with an even first radix
-    out.push_back(q);
-  };
-  for (int a : S) {
-    if (n % a) continue;
-    const int n1 = n / a;
-    if (n1 == 1) {
-      add(1, a, 0, 0);
-      continue;
-    }
-    for (int b : S) {
-      if (n1 % b) continue;
-      const int n2 = n1 / b;
-      if (n2 == 1) add(2, a, b, 0);
-      else if (reg_radix(n2)) add(3, a, b, n2);
-    }
-  }
-  std::stable_sort(out.begin(), out.end(), [](const RadixSeq &x, const RadixSeq &y) { return x.cost < y.cost; });
-  return out;
-}
-
-// two-phase sequences with at least one wide composite radix (the wide FP32 kernel
-// variant), fewest points per thread first; only the autotuner tries them
-static std::vector<RadixSeq> regplan_candidates_wide(int n) {
-  static const int S[] = {24, 22, 20, 18, 17, 16, 13, 12, 11, 10, 9, 8};
-  std::vector<RadixSeq> out;
-  for (int a : S) {
-    if (n % a) continue;
-    const int b = n / a;
-    if (!(reg_radix(b) || reg_radix_wide(b)) || !(reg_radix_wide(a) || reg_radix_wide(b))) continue;
-    RadixSeq q;
-    q.np = 2;
-    q.r[0] = a;
-    q.r[1] = b;
-    q.r[2] = 0;
-    q.cost = (double)std::max(a, b) + (a % 2 ? 0.5 : 0.0);
-    out.push_back(q);
-  }
-  std::stable_sort(out.begin(), out.end(), [](const RadixSeq &x, const RadixSeq &y) { return x.cost < y.cost; });
-  return out;
-}
-
-// The same radices ordered for the fused middle of the z pass: the smallest radix
-// that the registers take last, an even radix first where there is one (the zero half
-// of a padded line is then skipped); any order of the radices is a valid plan.
-static RadixSeq z_order(const RadixSeq &c, int rsize) {
-  RadixSeq q = c;
-  if (c.np < 2) return q;
-  const int lim = rsize == 4 ? 8 : 6;
-  int best = -1;
-  for (int i = 0; i < c.np; i++)
-    if (c.r[i] <= lim && (best < 0 || c.r[i] < c.r[best])) best = i;
-  if (best < 0) return q;
-  int rest[2], nr = 0;
-  for (int i = 0; i < c.np; i++)
-    if (i != best) rest[nr++] = c.r[i];
-  if (nr == 2 && rest[0] % 2 && !(rest[1] % 2)) std::swap(rest[0], rest[1]);
-  for (int i = 0; i < nr; i++) q.r[i] = rest[i];
-  q.r[nr] = c.r[best];
-  return q;
-}
-
-static bool make_regplan(int n, RegPlan &pl) {
-  const std::vector<RadixSeq> c = regplan_candidates(n);
-  if (c.empty()) return false;
-  regplan_from(n, c[0].r, c[0].np, pl);
-  return true;
-}
-
 // Autotuned schedules: (length, precision, axis) -> radix sequence and kx tile, the
 // fastest measured forward pass among the candidates (process-wide, filled when
 // plans are created while tuning is on).
@@ -410,21 +294,225 @@ struct TunedSchedule {
 static std::map<std::tuple<int, int, int>, TunedSchedule> g_tuned;
 static int g_tune = 0;
 
-// position -> frequency index of the digit-reversed output of a plan
-static std::vector<int> regplan_positions(const RegPlan &pl) {
-  std::vector<int> k(pl.n);
-  for (int q = 0; q < pl.n; q++) {
-    int rem = q, mul = 1, f = 0;
-    for (int p = 0; p < pl.np; p++) {
-      const int sub = pl.blk[p] / pl.rad[p];
-      const int d = rem / sub;
-      rem -= d * sub;
-      f += mul * d;
-      mul *= pl.rad[p];
-    }
-    k[q] = f;
+// ------------------------------------------------------------------ line plans (y and z)
+struct RadixSeq {
+  int np;
+  int r[3];
+  double cost;
+};
+// Packed instructions per point of a register DFT (linefft.cuh's codelets), counted.
+static double line_radix_ops(int r) {
+  switch (r) {
+    case 1: return 0.0;
+    case 2: return 2.0;
+    case 3: return 4.7;
+    case 4: return 4.0;
+    case 5: return 7.2;
+    case 6: return 6.7;
+    case 7: return 9.4;
+    case 8: return 7.0;
+    case 9: return 11.8;
+    case 10: return 9.2;
+    case 11: return 13.6;
+    case 12: return 8.7;
+    case 13: return 15.7;
+    case 16: return 10.0;
+    case 17: return 19.8;
+    case 18: return 13.8;
+    case 20: return 11.2;
+    case 22: return 15.6;
+    case 24: return 11.7;
+    default: return 1e9;
   }
-  return k;
+}
+static int gcd_i(int a, int b) { return b ? gcd_i(b, a % b) : a; }
+
+// The plan of digits r[0..np) (outermost first) over n = prod r points; split: see
+// linefft.cuh.  one_group: natural order inside (Bluestein), else the finest partition of
+// the consecutive digits into groups of pairwise coprime sizes.
+static void lineplan_from(int n, int split, const int *r, int np, bool one_group, LinePlan &pl) {
+  memset(&pl, 0, sizeof(pl));
+  pl.n = n;
+  pl.split = split;
+  pl.np = np;
+  int grp[LP_MAX] = {0, 0, 0};  // group of each digit
+  if (!one_group) {
+    auto share = [&](int i, int j) { return j < np && gcd_i(r[i], r[j]) > 1; };
+    const bool ends = share(0, 2);
+    grp[1] = share(0, 1) || ends ? 0 : 1;
+    grp[2] = share(1, 2) || ends ? grp[1] : grp[1] + 1;
+  }
+  int gsize[LP_MAX] = {1, 1, 1};
+  for (int i = 0; i < np; i++) gsize[grp[i]] *= r[i];
+  int str = n;
+  for (int p = 0; p < np; p++) {
+    pl.rad[p] = r[p];
+    str /= r[p];
+    pl.str[p] = str;
+    pl.dstr[p] = make_fastdiv((unsigned)str);
+    int tin = 1, inner = 1;  // digits of later groups; later digits of this group
+    for (int q = p + 1; q < np; q++) (grp[q] == grp[p] ? inner : tin) *= r[q];
+    pl.tin[p] = tin;
+    pl.dtin[p] = make_fastdiv((unsigned)tin);
+    // decimation in frequency inside the group: w_B^(rg k) with B = r[p] inner
+    pl.tmul[p] = inner > 1 ? n / (r[p] * inner) : 0;
+  }
+  int inner0 = 1;
+  for (int q = 1; q < np; q++)
+    if (grp[q] == grp[0]) inner0 *= r[q];
+  pl.rstep = np ? (n / gsize[grp[0]]) * inner0 % n : 0;
+}
+
+// groups of a plan, recovered from its twiddles (a phase without twiddles ends a group)
+static std::vector<std::vector<int>> lineplan_groups(const LinePlan &pl) {
+  std::vector<std::vector<int>> g(1);
+  for (int p = 0; p < pl.np; p++) {
+    g.back().push_back(p);
+    if (pl.tmul[p] == 0 && p + 1 < pl.np) g.emplace_back();
+  }
+  return g;
+}
+
+// frequency of every position (both halves of a split plan) and input row of every
+// butterfly of phase 0 at digit 0
+static void lineplan_tables(const LinePlan &pl, std::vector<int> &freq, std::vector<int> &rbase) {
+  const auto groups = lineplan_groups(pl);
+  const int n = pl.n;
+  std::vector<int> inverse(groups.size());  // of n / size modulo the group's size
+  for (size_t i = 0; i < groups.size(); i++) {
+    int size = 1;
+    for (int p : groups[i]) size *= pl.rad[p];
+    while (((long long)(n / size) * inverse[i]) % size != 1 % size) inverse[i]++;
+  }
+  std::vector<int> f1(n), row(n);
+  for (int q = 0; q < n; q++) {
+    long long rw = 0, f = 0;
+    for (size_t i = 0; i < groups.size(); i++) {
+      const auto &g = groups[i];
+      int size = 1;
+      for (int p : g) size *= pl.rad[p];
+      int idx = 0, fr = 0, mul = 1;
+      for (int p : g) {
+        const int d = (q / pl.str[p]) % pl.rad[p];
+        idx = idx * pl.rad[p] + d;  // natural index: first digit slowest
+        fr += d * mul;              // its transform sits digit-reversed
+        mul *= pl.rad[p];
+      }
+      const int rest = n / size;
+      rw += (long long)rest * idx;
+      // Chinese remainder: the multiple of `rest` that is fr modulo size
+      f += (long long)rest * ((long long)inverse[i] * fr % size);
+    }
+    row[q] = (int)(rw % n);
+    f1[q] = (int)(f % n);
+  }
+  rbase.assign(row.begin(), row.begin() + n / pl.rad[0]);
+  freq.resize(plan_points(pl));
+  for (int q = 0; q < n; q++) {
+    if (pl.split) {
+      freq[q] = 2 * f1[q];
+      freq[n + q] = 2 * f1[q] + 1;
+    } else {
+      freq[q] = f1[q];
+    }
+  }
+}
+
+// Digit sequences for n points, best first.  The score counts packed instructions a point:
+// the radix DFTs, 5 for a twiddle (product and table load), and 16 for the
+// shared-memory round trip of a phase beyond the first (eight wavefronts a warp against
+// half a cycle of the SM an instruction).  Along z (axis 2) the last digit is done
+// together with the multiply when it is small enough (z_mid_radix): worth its round
+// trip; an even one pays four instructions for its bank conflicts.  Split plans hold
+// both halves of a first-phase butterfly, so digit 0 is at most 12 (FP64: 8).
+static std::vector<RadixSeq> line_candidates(int n, int split, int axis, int rsize, bool one_group = false) {
+  static const int S[] = {24, 22, 20, 18, 17, 16, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  std::vector<RadixSeq> out;
+  auto add = [&](int np, int a, int b, int c) {
+    RadixSeq q;
+    q.np = np;
+    q.r[0] = a;
+    q.r[1] = b;
+    q.r[2] = c;
+    if (split && a > (rsize == 4 || axis == 0 ? 12 : 8)) return;
+    LinePlan pl;
+    lineplan_from(n, split, q.r, np, one_group, pl);
+    q.cost = 0.0;
+    for (int i = 0; i < np; i++) q.cost += line_radix_ops(q.r[i]) + (pl.tmul[i] ? 5.0 : 0.0) + (i ? 16.0 : 0.0);
+    if (axis == 2) {
+      const int last = q.r[np - 1];
+      if (np < 2 || !z_mid_radix(last)) q.cost += 16.0;
+      else if (last % 2 == 0) q.cost += 4.0;
+    }
+    // long butterflies spill beyond 128 registers a thread (the last of two digits does not)
+    for (int i = 0; i < np; i++) {
+      if (q.r[i] > 13 && !(axis != 2 && i > 0 && np == 2)) q.cost += q.r[i] == 16 ? 6.0 : 20.0;
+      if (split && i == 0 && q.r[i] > 8) q.cost += axis != 2 && q.r[i] <= 11 ? 6.0 : 20.0;
+    }
+    out.push_back(q);
+  };
+  auto ok = [&](int r) { return reg_radix(r) || ((rsize == 4 || one_group) && axis != 0 && reg_radix_wide(r)); };
+  for (int a : S) {
+    if (n % a || !ok(a)) continue;
+    const int n1 = n / a;
+    if (n1 == 1) {
+      add(1, a, 0, 0);
+      continue;
+    }
+    for (int b : S) {
+      if (n1 % b || !ok(b)) continue;
+      const int n2 = n1 / b;
+      if (n2 == 1) add(2, a, b, 0);
+      else if (ok(n2)) add(3, a, b, n2);
+    }
+  }
+  std::stable_sort(out.begin(), out.end(), [](const RadixSeq &x, const RadixSeq &y) { return x.cost < y.cost; });
+  return out;
+}
+
+// The digits of a schedule (radices of the whole line, as the schedule table holds them)
+// for a split plan: the padding's factor 2 comes off the first radix if that leaves a
+// digit, else off the largest even radix, which then comes first.
+static bool schedule_digits(const int *r, int np, int split, int *d, int &nd) {
+  nd = 0;
+  if (!split) {
+    for (int i = 0; i < np; i++) d[nd++] = r[i];
+    return true;
+  }
+  int h = -1;
+  if (r[0] % 2 == 0 && r[0] > 2) h = 0;
+  else
+    for (int i = 0; i < np; i++)
+      if (r[i] % 2 == 0 && (h < 0 || r[i] > r[h])) h = i;
+  if (h < 0) return false;
+  if (r[h] > 2) d[nd++] = r[h] / 2;
+  for (int i = 0; i < np; i++)
+    if (i != h) d[nd++] = r[i];
+  return nd > 0;
+}
+
+// the plan of a line of M points along `axis`; half: the second half is zero padding
+static bool make_lineplan(int M, bool half, int axis, int rsize, LinePlan &pl) {
+  const int split = half && M >= 4 ? 1 : 0, n = split ? M / 2 : M;
+  // a plan with compile-time kernels
+  static const struct { int axis, rsize, split, n, r[3]; } ct[] = {
+#define PMGPU_PLAN_X_F32(S, N, A, B, C) {0, 4, S, N, {A, B, C}},
+#define PMGPU_PLAN_X_F64(S, N, A, B, C) {0, 8, S, N, {A, B, C}},
+#define PMGPU_PLAN_Y_F32(S, N, A, B, C) {1, 4, S, N, {A, B, C}},
+#define PMGPU_PLAN_Y_F64(S, N, A, B, C) {1, 8, S, N, {A, B, C}},
+#define PMGPU_PLAN_Z_F32(S, N, A, B, C) {2, 4, S, N, {A, B, C}},
+#define PMGPU_PLAN_Z_F64(S, N, A, B, C) {2, 8, S, N, {A, B, C}},
+#include "line_plans.inc"
+  };
+  for (const auto &q : ct)
+    if (q.axis == axis && q.rsize == rsize && q.split == split && q.n == n) {
+      lineplan_from(n, split, q.r, q.r[2] > 1 ? 3 : q.r[1] > 1 ? 2 : 1, false, pl);
+      return true;
+    }
+  const std::vector<RadixSeq> c = line_candidates(n, split, axis, rsize);
+  if (c.empty()) return false;
+  lineplan_from(n, split, c[0].r, c[0].np, false, pl);
+  return true;
 }
 
 // forward DFT in long double, any length whose prime factors are small (mixed radix,
@@ -452,23 +540,28 @@ static void host_dft(std::vector<cld> &a) {
   }
 }
 
-// Bluestein plan for a line of length n: the convolution length m is the smallest
-// m >= 2n - 1 with a register plan
-static bool make_bluestein(int n, RegPlan &pl) {
-  for (int m = 2 * n - 1; m <= 4 * n; m++)
-    if (make_regplan(m, pl)) {
-      pl.bl = 1;
-      pl.bn = n;
-      return true;
-    }
-  return false;
+// Bluestein plan for a line of length n with `rows` data points: of the convolution lengths
+// from n + rows - 1 on (up to a third more), the one with the least work
+static bool make_bluestein(int n, int rows, int axis, int rsize, LinePlan &pl) {
+  const int least = n + rows - 1;
+  double best = 1e30;
+  for (int m = least; m <= 2 * least && (m <= least + least / 3 || best > 1e29); m++) {
+    const std::vector<RadixSeq> c = line_candidates(m, 0, axis ? 1 : 0, rsize, true);
+    if (c.empty() || m * (c[0].cost + 16.0) >= best) continue;
+    best = m * (c[0].cost + 16.0);
+    lineplan_from(m, 0, c[0].r, c[0].np, true, pl);
+    pl.bl = 1;
+    pl.bn = n;
+    pl.brows = rows;
+  }
+  return best < 1e29;
 }
 
-// chirp c[j] = exp(-i pi j^2 / n) and B = DFT_m of conj(c) wrapped (B[q] at the
-// plan's position q)
+// chirp c[j] = exp(-i pi j^2 / n) and, B[q] at position q (kp: position -> frequency), the
+// DFT_m of conj(c) wrapped from 1 - rows on (forward) and from 1 - n on (inverse)
 template <typename C, typename R>
-static void bluestein_tables(const RegPlan &pl, std::vector<C> &chirp, std::vector<C> &bpos) {
-  const int n = pl.bn, m = pl.n;
+static void bluestein_tables(int n, int rows, int m, const std::vector<int> &kp, std::vector<C> &chirp,
+                             std::vector<C> &bpos) {
   const long double pi = acosl(-1.0L);
   std::vector<cld> c(n), b(m, cld(0.0L, 0.0L));
   for (int j = 0; j < n; j++) {
@@ -476,14 +569,17 @@ static void bluestein_tables(const RegPlan &pl, std::vector<C> &chirp, std::vect
     const long double a = -pi * (long double)q / (long double)n;
     c[j] = cld(cosl(a), sinl(a));
   }
-  b[0] = std::conj(c[0]);
-  for (int j = 1; j < n; j++) b[j] = b[m - j] = std::conj(c[j]);
+  for (int j = 0; j < n; j++) b[j] = std::conj(c[j]);
+  for (int j = 1; j < rows; j++) b[m - j] = std::conj(c[j]);
   host_dft(b);
-  const std::vector<int> kp = regplan_positions(pl);
   chirp.resize(n);
-  bpos.resize(m);
+  bpos.resize(2 * (size_t)m);
   for (int j = 0; j < n; j++) chirp[j] = mk((R)c[j].real(), (R)c[j].imag());
-  for (int q = 0; q < m; q++) bpos[q] = mk((R)b[kp[q]].real(), (R)b[kp[q]].imag());
+  for (int q = 0; q < m; q++) {
+    const cld f = b[kp[q]], v = b[(m - kp[q]) % m];  // the inverse wrap is the mirrored sequence
+    bpos[q] = mk((R)f.real(), (R)f.imag());
+    bpos[m + q] = mk((R)v.real(), (R)v.imag());
+  }
 }
 
 static std::mutex g_attr_mu;
@@ -559,9 +655,10 @@ struct pmgpu_plan {
   DevBuf X, Y, Y2, Y3;
   // register-engine plans along y and z (in-place, digit-reversed spectra)
   int rx_ok, ry_ok, rz_ok;
-  RegPlan rx, ry, rz;
+  LinePlan lx, ly, lz;
   int tky = 0, tkz = 0;  // tuned kx tiles (0: chosen by shared memory)
-  DevBuf rtwx, rtwy, rtwz, yk, zk, rextx, xpos;
+  DevBuf rtwx, rtwy, rtwz, rtsx, rtsy, rtsz, rbx0, rby0, rbz0, yk, zk, rextx, xpos;
+  DevBuf kxv, kzv, zoff;  // multiplier tables of the plain velocity solve
   DevBuf rchx, rchy, rchz, rbx, rby, rbz;  // Bluestein chirps and spectra
   // the register-engine tables above are views of device tables shared by the plans
   // of the same transform length, precision and schedule; these keep them alive
@@ -575,9 +672,11 @@ struct pmgpu_plan {
   ~pmgpu_plan() {
     DevBuf *bs[] = {&twx, &twy, &twz, &kxt, &kyt, &kzt, &X, &Y, &Y2, &Y3, &mesh_w, &mesh_u,
                     &mesh_a, &mesh_b, &h_pos, &h_val, &h_out, &key, &val, &key2, &val2, &counts,
-                    &start, &spart, &hist, &rtwx, &rtwy, &rtwz, &yk, &zk, &rextx, &xpos,
+                    &start, &spart, &hist, &rtwx, &rtwy, &rtwz, &rtsx, &rtsy, &rtsz, &rbx0, &rby0, &rbz0, &yk, &zk, &rextx, &xpos,
+                    &kxv, &kzv, &zoff,
                     &rchx, &rchy, &rchz, &rbx, &rby, &rbz};
     for (DevBuf *b : bs) b->release();
+    green.release();  // (a view unless all axes are periodic)
   }
 };
 
@@ -841,16 +940,26 @@ template <typename R> static SolveGeom<R> solve_geom(const pmgpu_plan *pl) {
   g.tky = pl->tky;
   g.tkz = pl->tkz;
   g.rx_ok = pl->rx_ok;
-  g.rx = pl->rx;
+  g.lx = pl->lx;
+  g.rtsx = pl->rtsx.as<C>();
+  g.rbx0 = pl->rbx0.as<int>();
   g.rtwx = pl->rtwx.as<C>();
   g.rextx = pl->rextx.as<C>();
   g.xpos = pl->xpos.as<int>();
   g.ry_ok = pl->ry_ok;
   g.rz_ok = pl->rz_ok;
-  g.ry = pl->ry;
-  g.rz = pl->rz;
+  g.ly = pl->ly;
+  g.lz = pl->lz;
   g.rtwy = pl->rtwy.as<C>();
   g.rtwz = pl->rtwz.as<C>();
+  g.rtsy = pl->rtsy.as<C>();
+  g.rtsz = pl->rtsz.as<C>();
+  g.rby0 = pl->rby0.as<int>();
+  g.rbz0 = pl->rbz0.as<int>();
+  g.kxv = pl->kxv.as<R>();
+  g.kzv = pl->kzv.as<R>();
+  g.zoff = pl->zoff.as<int>();
+  g.gH = pl->g.Hp;
   g.yk = pl->ry_ok ? pl->yk.as<int>() : nullptr;
   g.zk = pl->rz_ok ? pl->zk.as<int>() : nullptr;
   return g;
@@ -947,9 +1056,18 @@ template <typename R> static int reg_tables(pmgpu_plan *pl, const char *caller, 
 
 template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller) {
   const Geometry &G = pl->g;
-  pl->gM1 = G.M[1] / 2 + 1;
-  pl->gM2 = G.M[2] / 2 + 1;
-  if (G.allper) return 0;
+  if (G.allper) {
+    // the plain velocity solve's multiplier 1 / (4 pi^2 k^2 Mx My Mz), as an octant
+    const size_t noct = (size_t)pl->gM2 * pl->gM1 * G.Hp;
+    if (pl->green.ensure(sizeof(R) * noct, caller)) return -1;
+    const unsigned nb = (unsigned)std::min<size_t>((noct + 255) / 256, 148 * 64);
+    k_green_periodic<R><<<nb, 256>>>(G.M[0], G.M[1], G.M[2], pl->patch.dx[0], pl->patch.dx[1], pl->patch.dx[2], G.H,
+                                     G.Hp, pl->gM1, pl->gM2, pl->green.as<R>());
+    PM_LAUNCHED();
+    CKL(caller);
+    CK(cudaStreamSynchronize(0), caller);
+    return 0;
+  }
   const std::string key = green_key(pl);
   {
     auto it = g_green_cache.find(key);
@@ -1031,7 +1149,7 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
     if (gr.ensure(sizeof(double) * npts, caller) || gX.ensure(sizeof(double2) * nspec, caller) ||
         gY.ensure(sizeof(double2) * nspec, caller))
       break;
-    const size_t noct = (size_t)pl->gM2 * pl->gM1 * G.H;
+    const size_t noct = (size_t)pl->gM2 * pl->gM1 * G.Hp;
     const double f = pl->patch.dx[0] * pl->patch.dx[1] * pl->patch.dx[2] /
                      ((double)G.M[0] * (double)G.M[1] * (double)G.M[2]);
     const unsigned nb_real = (unsigned)std::min<size_t>((npts + 255) / 256, 148 * 64);
@@ -1127,8 +1245,72 @@ template <typename R> static int upload_wavenumbers(pmgpu_plan *pl, const char *
     }
     if (bufs[e]->ensure(sizeof(R) * cnt, caller)) return -1;
     CK(cudaMemcpy(bufs[e]->p, h.data(), sizeof(R) * cnt, cudaMemcpyHostToDevice), caller);
+    if (e == 0) {
+      std::vector<R> v(pl->g.Hp, R(0));
+      for (int i = 0; i < cnt; i++)
+        if (2 * i != M) v[i] = (R)(2.0 * 3.14159265358979323846 * (double)i * dk);
+      if (pl->kxv.ensure(sizeof(R) * v.size(), caller)) return -1;
+      CK(cudaMemcpy(pl->kxv.p, v.data(), sizeof(R) * v.size(), cudaMemcpyHostToDevice), caller);
+    }
   }
   return 0;
+}
+
+// Host tables of a line plan: w_n^q, w_{2n}^q (split plans), the frequency of every
+// position and the rows of phase 0's butterflies; of the velocity multiplier along z:
+// 2 pi kz (Nyquist component zero) and the octant plane's offset, by position.
+template <typename C, typename R> static void line_twiddles(int n, int num, std::vector<C> &tw) {
+  const long double twopi = 2.0L * acosl(-1.0L);
+  tw.resize(num);
+  for (int q = 0; q < num; q++) {
+    const long double a = twopi * (long double)q / (long double)n;
+    tw[q] = mk((R)cosl(a), (R)-sinl(a));
+  }
+}
+template <typename R>
+static void zvel_tables(const pmgpu_plan *pl, const std::vector<int> &freq, std::vector<R> &kzv,
+                        std::vector<int> &zoff) {
+  const int M = pl->g.M[2];
+  const double dk = 2.0 * 3.14159265358979323846 / ((double)M * pl->patch.dx[2]);
+  kzv.resize(M);
+  zoff.resize(M);
+  for (int q = 0; q < M; q++) {
+    const int z = freq[q];
+    kzv[q] = 2 * z == M ? R(0) : (R)((double)(2 * z < M ? z : z - M) * dk);
+    zoff[q] = std::min(z, M - z) * pl->gM1 * pl->g.Hp;
+  }
+}
+
+struct LineBufs {
+  DevBuf tw, tws, rbase, freq, kzv, zoff;
+  std::vector<int> hfreq;
+  ~LineBufs() {
+    for (DevBuf *b : {&tw, &tws, &rbase, &freq, &kzv, &zoff}) b->release();
+  }
+};
+template <typename T> static int put_table(DevBuf &b, const std::vector<T> &h, const char *caller) {
+  if (b.ensure(sizeof(T) * std::max<size_t>(h.size(), 1), caller)) return -1;
+  if (!h.empty()) CK(cudaMemcpy(b.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice), caller);
+  return 0;
+}
+template <typename R> static int line_upload(const LinePlan &lp, LineBufs &t, const char *caller) {
+  typedef typename cplx_t<R>::type C;
+  std::vector<C> tw, tws;
+  std::vector<int> rbase;
+  line_twiddles<C, R>(lp.n, lp.n, tw);
+  if (lp.split) line_twiddles<C, R>(2 * lp.n, lp.n, tws);
+  lineplan_tables(lp, t.hfreq, rbase);
+  return put_table(t.tw, tw, caller) || put_table(t.tws, tws, caller) || put_table(t.rbase, rbase, caller) ||
+                 put_table(t.freq, t.hfreq, caller)
+             ? -1
+             : 0;
+}
+template <typename R>
+static int zvel_upload(const pmgpu_plan *pl, const LinePlan &, LineBufs &t, const char *caller) {
+  std::vector<R> kzv;
+  std::vector<int> zoff;
+  zvel_tables<R>(pl, t.hfreq, kzv, zoff);
+  return put_table(t.kzv, kzv, caller) || put_table(t.zoff, zoff, caller) ? -1 : 0;
 }
 
 // Times the pass along `axis` of this plan's geometry (y: the forward pass; z: the
@@ -1139,25 +1321,11 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
   typedef typename cplx_t<R>::type C;
   const Geometry &G = pl->g;
   const int n = G.M[axis];
-  std::vector<RadixSeq> cands = regplan_candidates(n);
-  if (cands.size() > 5) cands.resize(5);
-  if (axis == 2) {
-    // the same radices ordered for the fused middle of the z pass
-    const size_t nc = cands.size();
-    for (size_t i = 0; i < nc; i++) {
-      const RadixSeq q = z_order(cands[i], (int)sizeof(R));
-      bool dup = false;
-      for (const RadixSeq &o : cands)
-        dup = dup || (o.np == q.np && o.r[0] == q.r[0] && o.r[1] == q.r[1] && o.r[2] == q.r[2]);
-      if (!dup) cands.push_back(q);
-    }
-  }
-  if (sizeof(R) == 4) {
-    std::vector<RadixSeq> w = regplan_candidates_wide(n);
-    if (w.size() > 3) w.resize(3);
-    cands.insert(cands.end(), w.begin(), w.end());
-  }
-  DevBuf A, B, tw, kp;
+  const int split = G.M[axis] == 2 * G.P[axis] && n >= 4 ? 1 : 0, m = split ? n / 2 : n;
+  std::vector<RadixSeq> cands = line_candidates(m, split, axis, (int)sizeof(R));
+  if (cands.size() > 8) cands.resize(8);
+  DevBuf A, B;
+  LineBufs tabs;
   const size_t nx = (size_t)G.P[1] * G.P[2] * G.Hp * 3;
   const size_t ny = (size_t)G.M[1] * G.P[2] * G.Hp * 3;
   if ((axis == 1 && A.ensure(sizeof(C) * nx, caller)) || B.ensure(sizeof(C) * ny, caller)) return -1;
@@ -1168,34 +1336,31 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
   CK(cudaEventCreate(&e1), caller);
   best.ms = 1e30;
   best.np = 0;
-  const long double twopi = 2.0L * acosl(-1.0L);
   for (const RadixSeq &c : cands) {
-    RegPlan rp;
-    regplan_from(n, c.r, c.np, rp);
-    std::vector<C> t(n);
-    for (int q = 0; q < n; q++) {
-      const long double a = twopi * (long double)q / (long double)n;
-      t[q] = mk((R)cosl(a), (R)-sinl(a));
-    }
-    const std::vector<int> pos = regplan_positions(rp);
-    if (tw.ensure(sizeof(C) * n, caller) || kp.ensure(sizeof(int) * n, caller)) break;
-    if (!cuda_ok(cudaMemcpy(tw.p, t.data(), sizeof(C) * n, cudaMemcpyHostToDevice), caller) ||
-        !cuda_ok(cudaMemcpy(kp.p, pos.data(), sizeof(int) * n, cudaMemcpyHostToDevice), caller))
-      break;
+    LinePlan lp;
+    lineplan_from(m, split, c.r, c.np, false, lp);
+    if (line_upload<R>(lp, tabs, caller)) break;
     for (int tk : {8, 4, 2}) {
-      if (G.Hp % tk || reg_smem(n, n, 3, tk, sizeof(C)) > PASS_SMEM_BUDGET) continue;
+      if (tk > spec_block<R>() || line_smem(lp, 3, tk, sizeof(R)) > PASS_SMEM_BUDGET) continue;
       SolveGeom<R> g = solve_geom<R>(pl);
       if (axis == 1) {
-        g.ry = rp;
+        g.ly = lp;
         g.ry_ok = 1;
-        g.rtwy = tw.as<C>();
-        g.yk = kp.as<int>();
+        g.rtwy = tabs.tw.as<C>();
+        g.rtsy = tabs.tws.as<C>();
+        g.rby0 = tabs.rbase.as<int>();
+        g.yk = tabs.freq.as<int>();
         g.tky = tk;
       } else {
-        g.rz = rp;
+        if (zvel_upload<R>(pl, lp, tabs, caller)) break;
+        g.lz = lp;
         g.rz_ok = 1;
-        g.rtwz = tw.as<C>();
-        g.zk = kp.as<int>();
+        g.rtwz = tabs.tw.as<C>();
+        g.rtsz = tabs.tws.as<C>();
+        g.rbz0 = tabs.rbase.as<int>();
+        g.zk = tabs.freq.as<int>();
+        g.kzv = tabs.kzv.as<R>();
+        g.zoff = tabs.zoff.as<int>();
         g.tkz = tk;
       }
       auto run = [&]() {
@@ -1213,7 +1378,9 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
       if (ms / 3 < best.ms) {
         best.ms = ms / 3;
         best.np = c.np;
-        for (int i = 0; i < 3; i++) best.r[i] = c.r[i];
+        // the table holds radices of the whole line
+        for (int i = 0; i < 3; i++) best.r[i] = i < c.np ? c.r[i] : 0;
+        if (split) best.r[0] *= 2;
         best.tk = tk;
       }
     }
@@ -1237,10 +1404,10 @@ static std::map<std::string, std::weak_ptr<DevBuf>> g_tab_cache;
 static std::deque<std::shared_ptr<DevBuf>> &g_tab_recent = *new std::deque<std::shared_ptr<DevBuf>>();
 constexpr size_t TAB_RECENT = 512;
 
-static std::string regplan_key(const char *kind, int prec_bytes, int n, int extra, const RegPlan &rp) {
+static std::string lineplan_key(int prec_bytes, const LinePlan &lp) {
   char b[160];
-  snprintf(b, sizeof(b), "%s|%d|%d|%d|%d:%d,%d,%d|%d,%d", kind, prec_bytes, n, extra, rp.np, rp.rad[0],
-           rp.np > 1 ? rp.rad[1] : 0, rp.np > 2 ? rp.rad[2] : 0, rp.bl, rp.bn);
+  snprintf(b, sizeof(b), "l|%d|%d|%d|%d:%d,%d,%d|%d,%d,%d|%d,%d", prec_bytes, lp.n, lp.split, lp.np, lp.rad[0],
+           lp.np > 1 ? lp.rad[1] : 0, lp.np > 2 ? lp.rad[2] : 0, lp.tmul[0], lp.tmul[1], lp.tmul[2], lp.bl, lp.bn * 4 + (lp.brows < lp.bn ? 1 : 0));
   return std::string(b);
 }
 
@@ -1276,23 +1443,16 @@ template <typename R> static int reg_tables(pmgpu_plan *pl, const char *caller, 
   typedef typename cplx_t<R>::type C;
   pl->rx_ok = pl->ry_ok = pl->rz_ok = 0;
   if (g_force_stockham) return 0;
-  const long double twopi = 2.0L * acosl(-1.0L);
   const int pb = (int)sizeof(R);
-  // twiddles w_m^q of a plan's transform length m
-  auto twiddles = [&](int mm, std::vector<C> &tw) {
-    tw.resize(mm);
-    for (int q = 0; q < mm; q++) {
-      const long double a = twopi * (long double)q / (long double)mm;
-      tw[q] = mk((R)cosl(a), (R)-sinl(a));
-    }
-  };
   // Bluestein chirp and spectrum of a plan (nothing for a direct plan)
-  auto upload_blue = [&](const std::string &key, const RegPlan &rp, DevBuf &ch, DevBuf &bp) -> int {
-    if (!rp.bl) return 0;
+  auto upload_blue = [&](const std::string &key, const LinePlan &lp, DevBuf &ch, DevBuf &bp) -> int {
+    if (!lp.bl) return 0;
     std::vector<C> c, b;
     bool made = false;
     auto make = [&]() {
-      if (!made) bluestein_tables<C, R>(rp, c, b);
+      std::vector<int> kp, rbase;
+      if (!made) lineplan_tables(lp, kp, rbase);
+      if (!made) bluestein_tables<C, R>(lp.bn, lp.brows, lp.n, kp, c, b);
       made = true;
     };
     if (shared_table<C>(pl, key + "|ch", ch, [&](std::vector<C> &h) { make(); h = c; }, caller)) return -1;
@@ -1301,81 +1461,106 @@ template <typename R> static int reg_tables(pmgpu_plan *pl, const char *caller, 
   pl->tab_keep.clear();
   {
     // x passes: half-length complex transform N = Mx / 2
-    RegPlan rp;
+    LinePlan lp;
     const int N = pl->g.N2, H = pl->g.H, Mx = pl->g.M[0];
-    if (make_regplan(N, rp) || make_bluestein(N, rp)) {
-      const std::string key = regplan_key("x", pb, N, Mx, rp);
-      if (shared_table<C>(pl, key + "|tw", pl->rtwx, [&](std::vector<C> &h) { twiddles(rp.n, h); }, caller) ||
-          shared_table<C>(pl, key + "|ext", pl->rextx,
+    // a free axis of even length: exactly the second half of the packed points is zero
+    const bool half = Mx == 2 * pl->g.P[0] && pl->g.P[0] % 2 == 0;
+    if (make_lineplan(N, half, 0, pb, lp) ||
+        make_bluestein(N, Mx == 2 * pl->g.P[0] ? (pl->g.P[0] + 1) / 2 : N, 0, pb, lp)) {
+      const std::string key = "x" + lineplan_key(pb, lp);
+      std::vector<int> freq, rbase;
+      auto made = [&]() {  // the tables, when one is missing
+        if (freq.empty()) lineplan_tables(lp, freq, rbase);
+      };
+      if (shared_table<C>(pl, key + "|tw", pl->rtwx, [&](std::vector<C> &h) { line_twiddles<C, R>(lp.n, lp.n, h); },
+                          caller) ||
+          shared_table<C>(pl, key + "|ts", pl->rtsx,
                           [&](std::vector<C> &h) {
-                            h.resize(H);
-                            for (int k = 0; k < H; k++) {
-                              const long double a = twopi * (long double)k / (long double)Mx;
-                              h[k] = mk((R)cosl(a), (R)-sinl(a));
-                            }
+                            if (lp.split) line_twiddles<C, R>(2 * lp.n, lp.n, h);
                           },
+                          caller) ||
+          shared_table<int>(pl, key + "|rb", pl->rbx0, [&](std::vector<int> &h) { made(); h = rbase; }, caller) ||
+          shared_table<C>(pl, key + "|ext", pl->rextx, [&](std::vector<C> &h) { line_twiddles<C, R>(Mx, H, h); },
                           caller) ||
           shared_table<int>(pl, key + "|pos", pl->xpos,
                             [&](std::vector<int> &h) {
                               h.resize(N);
-                              if (rp.bl) {
-                                for (int q = 0; q < N; q++) h[q] = q;  // natural order
-                              } else {
-                                const std::vector<int> kp = regplan_positions(rp);
-                                for (int q = 0; q < N; q++) h[kp[q]] = q;
+                              made();
+                              for (int q = 0; q < N; q++) {
+                                if (lp.bl) h[q] = q;  // natural order
+                                else h[freq[q]] = q;
                               }
                             },
                             caller) ||
-          upload_blue(key, rp, pl->rchx, pl->rbx))
+          upload_blue(key, lp, pl->rchx, pl->rbx))
         return -1;
-      pl->rx = rp;
+      pl->lx = lp;
       pl->rx_ok = 1;
     }
   }
   for (int axis = 1; axis <= 2; axis++) {
-    RegPlan rp;
+    LinePlan lp;
     const int n = pl->g.M[axis];
-    if (!make_regplan(n, rp) && !make_bluestein(n, rp)) continue;
-    bool tuned = false;
-    if (!rp.bl && tune_ok) {
-      // a schedule measured earlier for this length
-      auto it = g_tuned.find(std::make_tuple(n, (int)sizeof(R), axis));
-      if (it != g_tuned.end()) {
-        regplan_from(n, it->second.r, it->second.np, rp);
+    const bool half = n == 2 * pl->g.P[axis];
+    if (!make_lineplan(n, half, axis, pb, lp) && !make_bluestein(n, half ? n / 2 : n, axis, pb, lp)) continue;
+    if (!lp.bl && tune_ok) {
+      // a schedule measured or set earlier for this length
+      auto it = g_tuned.find(std::make_tuple(n, pb, axis));
+      int d[LP_MAX], nd = 0;
+      if (it != g_tuned.end() && schedule_digits(it->second.r, it->second.np, lp.split, d, nd)) {
+        lineplan_from(lp.n, lp.split, d, nd, false, lp);
         (axis == 1 ? pl->tky : pl->tkz) = it->second.tk;
-        tuned = true;
       }
     }
-    if (!rp.bl && !tuned && axis == 2) {
-      // untuned z plans: the model's radices ordered for the fused middle
-      RadixSeq c;
-      c.np = rp.np;
-      for (int i = 0; i < 3; i++) c.r[i] = i < rp.np ? rp.rad[i] : 0;
-      c.cost = 0.0;
-      const RadixSeq q = z_order(c, (int)sizeof(R));
-      regplan_from(n, q.r, q.np, rp);
-    }
-    const std::string key = regplan_key("l", pb, n, 0, rp);
-    DevBuf &tb = axis == 1 ? pl->rtwy : pl->rtwz;
-    DevBuf &kb = axis == 1 ? pl->yk : pl->zk;
-    if (shared_table<C>(pl, key + "|tw", tb, [&](std::vector<C> &h) { twiddles(rp.n, h); }, caller) ||
-        shared_table<int>(pl, key + "|pos", kb,
+    const std::string key = lineplan_key(pb, lp);
+    std::vector<int> freq, rbase;
+    auto made = [&]() {  // the tables, when one is missing
+      if (freq.empty()) lineplan_tables(lp, freq, rbase);
+    };
+    if (shared_table<C>(pl, key + "|tw", axis == 1 ? pl->rtwy : pl->rtwz,
+                        [&](std::vector<C> &h) { line_twiddles<C, R>(lp.n, lp.n, h); }, caller) ||
+        shared_table<C>(pl, key + "|ts", axis == 1 ? pl->rtsy : pl->rtsz,
+                        [&](std::vector<C> &h) {
+                          if (lp.split) line_twiddles<C, R>(2 * lp.n, lp.n, h);
+                        },
+                        caller) ||
+        shared_table<int>(pl, key + "|rb", axis == 1 ? pl->rby0 : pl->rbz0,
                           [&](std::vector<int> &h) {
-                            if (rp.bl) {
+                            made();
+                            h = rbase;
+                          },
+                          caller) ||
+        shared_table<int>(pl, key + "|pos", axis == 1 ? pl->yk : pl->zk,
+                          [&](std::vector<int> &h) {
+                            if (lp.bl) {
                               h.resize(n);
                               for (int q = 0; q < n; q++) h[q] = q;  // natural order
                             } else {
-                              h = regplan_positions(rp);
+                              made();
+                              h = freq;
                             }
                           },
                           caller) ||
-        upload_blue(key, rp, axis == 1 ? pl->rchy : pl->rchz, axis == 1 ? pl->rby : pl->rbz))
+        upload_blue(key, lp, axis == 1 ? pl->rchy : pl->rchz, axis == 1 ? pl->rby : pl->rbz))
       return -1;
+    if (axis == 2 && !lp.bl && tune_ok) {
+      char zk[96];
+      snprintf(zk, sizeof(zk), "|%a|%d|%d", pl->patch.dx[2], pl->gM1, pl->g.Hp);
+      std::vector<R> kzv;
+      std::vector<int> zoff;
+      auto zmade = [&]() {
+        made();
+        if (kzv.empty()) zvel_tables<R>(pl, freq, kzv, zoff);
+      };
+      if (shared_table<R>(pl, key + zk + "|kzv", pl->kzv, [&](std::vector<R> &h) { zmade(); h = kzv; }, caller) ||
+          shared_table<int>(pl, key + zk + "|zoff", pl->zoff, [&](std::vector<int> &h) { zmade(); h = zoff; }, caller))
+        return -1;
+    }
     if (axis == 1) {
-      pl->ry = rp;
+      pl->ly = lp;
       pl->ry_ok = 1;
     } else {
-      pl->rz = rp;
+      pl->lz = lp;
       pl->rz_ok = 1;
     }
   }
@@ -1388,8 +1573,7 @@ template <typename R> static int apply_tuning(pmgpu_plan *pl, const char *caller
   if (!g_tune || g_force_stockham) return 0;
   bool fresh = false;
   for (int axis = 1; axis <= 2; axis++) {
-    const RegPlan &rp = axis == 1 ? pl->ry : pl->rz;
-    if (!(axis == 1 ? pl->ry_ok : pl->rz_ok) || rp.bl) continue;
+    if (!(axis == 1 ? pl->ry_ok : pl->rz_ok) || (axis == 1 ? pl->ly : pl->lz).bl) continue;
     const auto key = std::make_tuple(pl->g.M[axis], (int)sizeof(R), axis);
     if (g_tuned.count(key)) continue;
     TunedSchedule ts;
@@ -1408,6 +1592,8 @@ template <typename R> static int plan_tables(pmgpu_plan *pl, const char *caller)
   if (!make_fft(pl->g.M[1], 0, pl->fy, tw) || upload_tw<R>(tw, pl->twy, caller)) return -1;
   if (!make_fft(pl->g.M[2], 0, pl->fz, tw) || upload_tw<R>(tw, pl->twz, caller)) return -1;
   if (upload_wavenumbers<R>(pl, caller)) return -1;
+  pl->gM1 = pl->g.M[1] / 2 + 1;
+  pl->gM2 = pl->g.M[2] / 2 + 1;
   if (reg_tables<R>(pl, caller, true)) return -1;
   if (setup_green<R>(pl, caller)) return -1;
   // the work spectra of a three-component solve, so that a plan's first solve (often
@@ -2297,7 +2483,7 @@ template <typename R> static int batch_fuse(pmgpu_batch *b, const char *caller) 
   }
   std::vector<unsigned char> host;
   if (batch_layout<R, 3>(n, geo.data(), X.data(), Y.data(), topo.data(), host, b->lay, caller)) return 0;
-  if (b->desc.ensure(host.size(), caller) || b->counters.ensure(5 * sizeof(unsigned), caller)) return -1;
+  if (b->desc.ensure(host.size(), caller) || b->counters.ensure(10 * sizeof(unsigned), caller)) return -1;
   CK(cudaMemcpy(b->desc.p, host.data(), host.size(), cudaMemcpyHostToDevice), caller);
   b->fused = true;
   return 0;

@@ -22,7 +22,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
-#include "regfft.cuh"
+#include "linefft.cuh"
 
 namespace pmgpu {
 
@@ -45,10 +45,13 @@ template <typename R> struct SolveGeom {
   R eps2pi;                  // 2 pi epsilon (filter argument scale)
   int order;                 // filter order (poisson order or reg_order)
   int allper;                // all axes periodic: spectral Green's function
-  // in-place register FFTs along y and z (when the lengths factor into register radices)
+  // in-place register FFTs (when the lengths factor into register radices, or Bluestein)
   int rx_ok, ry_ok, rz_ok;
-  RegPlan rx, ry, rz;        // rx: the half-length complex transform of the x passes
+  LinePlan lx;               // the half-length complex transform of the x passes
+  LinePlan ly, lz;
   const C *rtwx, *rtwy, *rtwz;  // w_n^q, q < n
+  const C *rtsx, *rtsy, *rtsz;      // split plans: w_{2n}^q, q < n
+  const int *rbx0, *rby0, *rbz0;    // input row of every butterfly of phase 0 at digit 0
   const C *rextx;            // exp(-2 pi i k / Mx), k < H
   const int *xpos;           // frequency -> position of the x transform
   int tky, tkz;              // kx tile of the y / z register passes (0: chosen by shared memory)
@@ -56,6 +59,12 @@ template <typename R> struct SolveGeom {
   const C *rbx, *rby, *rbz;     // Bluestein plans: FFT of the wrapped chirp, by position
   const int *yk;             // row of the y spectrum -> ky index (nullptr: natural order)
   const int *zk;             // position of the z transform -> kz index
+  // the plain velocity solve's multiplier tables: 2 pi kx (Nyquist component zero, zero
+  // from H on, Hp entries), and by z position 2 pi kz (Nyquist component zero) and the
+  // offset of the octant plane |kz|
+  const R *kxv, *kzv;
+  const int *zoff;
+  int gH;                    // row pitch of the octants (kx entries beyond H are zero)
 };
 
 enum ZMode { Z_VEL = 0, Z_VORT = 1, Z_VECPOT = 2, Z_REGULARISE = 3, Z_FORWARD = 4 };
@@ -134,9 +143,30 @@ struct LineTiles {
   int rows_in;    // rows read (the rest is zero padding)
   int rows_out;   // rows written (truncation)
   long long in_os, in_rs, out_os, out_rs;
+  long long in_kb, out_kb;  // strides between kx blocks
   int nouter, nkt, TK;
+  int ofast;      // consecutive tiles: outer index fastest (z pass) or kx tile fastest
   FastDiv dLG;    // division by the line vectors per row (register engine)
 };
+// kx of a block of the spectral arrays: 192 bytes of three components
+template <typename R> __host__ __device__ constexpr int spec_block() { return sizeof(R) == 4 ? 8 : 4; }
+// tile -> (outer index, first kx)
+__device__ __forceinline__ void line_tile_at(const LineTiles &lt, int tile, int TK, int &o, int &k0) {
+  if (lt.ofast) {
+    const int kt = tile / lt.nouter;
+    o = tile - kt * lt.nouter;
+    k0 = kt * TK;
+  } else {
+    o = tile / lt.nkt;
+    k0 = (tile - o * lt.nkt) * TK;
+  }
+}
+// complex offset (to be multiplied by the components) of kx index k0 in a row whose
+// blocks lie kb apart
+template <typename R> __device__ __forceinline__ long long spec_off(long long row, long long kb, int k0) {
+  constexpr int B = spec_block<R>();
+  return row + (long long)(k0 / B) * kb + (k0 & (B - 1));
+}
 
 enum LMode { L_FWD = 0, L_INV = 1, L_Z = 2 };
 
@@ -202,9 +232,9 @@ __device__ __forceinline__ void z_point(const SolveGeom<R> &g, typename cplx_t<R
       // i S_c + (-1)^(k_c) E_c, S_c odd along axis c and even along the others
       // (stored for |ky|, |kz| with the sign of the odd axis applied here), E_c the
       // spectrum of the kernel's plane at -M_c/2 dx_c
-      const size_t noct = (size_t)g.gM2 * g.gM1 * g.H;
+      const size_t noct = (size_t)g.gM2 * g.gM1 * g.gH;
       const int iz = min(z, g.M[2] - z);
-      const size_t oc = ((size_t)iz * g.gM1 + iy) * g.H + kx_i;
+      const size_t oc = ((size_t)iz * g.gM1 + iy) * g.gH + kx_i;
       const R *E = g.green + 3 * noct;
       R sx = g.green[oc], sy = g.green[noct + oc], sz = g.green[2 * noct + oc];
       if (2 * y > g.M[1]) sy = -sy;
@@ -273,171 +303,138 @@ __device__ __forceinline__ void z_point(const SolveGeom<R> &g, typename cplx_t<R
   }
 }
 
-// z-pass spectral multiply of one tile held in buffer V (complex view C).
-// zpos: position -> kz index (nullptr: natural order); kzs: kz wavenumbers (shared
-// copy of g.kzt, or nullptr)
-template <typename R, int NC>
-__device__ __forceinline__ void z_multiply(const SolveGeom<R> &g, typename cplx_t<R>::type *Cb, int L, int TK, int k0,
-                                           int y, int zmode, int reproj, int use_zeta, const int *zpos,
-                                           const R *kzs = nullptr) {
-  typedef typename cplx_t<R>::type C;
-  const R twopi = R(6.283185307179586476925286766559);
-  const int N = g.M[2];
+// One complex value of a line vector, and back.
+__device__ __forceinline__ float2 lane_get(const LV<float2> &a, int h) {
+  return h ? make_float2(a.re.y, a.im.y) : make_float2(a.re.x, a.im.x);
+}
+__device__ __forceinline__ void lane_set(LV<float2> &a, int h, float2 v) {
+  if (h) { a.re.y = v.x; a.im.y = v.y; }
+  else { a.re.x = v.x; a.im.x = v.y; }
+}
+__device__ __forceinline__ float2 lane_get(const LV<float> &a, int) { return make_float2(a.re, a.im); }
+__device__ __forceinline__ void lane_set(LV<float> &a, int, float2 v) { a.re = v.x; a.im = v.y; }
+__device__ __forceinline__ double2 lane_get(const LV<double> &a, int) { return make_double2(a.re, a.im); }
+__device__ __forceinline__ void lane_set(LV<double> &a, int, double2 v) { a.re = v.x; a.im = v.y; }
+
+// The spectral multiply (any mode) of a tile of LG vectors per position: TK kx of NC
+// components from kx index k0, spectrum row y.  zpos: position -> kz index (nullptr:
+// natural order)
+template <typename T, int NC>
+__device__ __forceinline__ void z_multiply(const SolveGeom<typename LineT<T>::R> &g, typename LineT<T>::V *buf, int LG,
+                                           int k0, int y, int zmode, int reproj, int use_zeta, const int *zpos) {
+  typedef typename LineT<T>::R R;
+  constexpr int G = LineT<T>::G;
+  const int N = g.M[2], nk = LG / NC;
   const R ky = g.kyt[y];
   const R kyc = (2 * y == g.M[1]) ? R(0) : ky;  // Nyquist component dropped in the curl
   const int iy = min(y, g.M[1] - y);
-  const int tks = __ffs(TK) - 1;  // TK is a power of two
-  const R *kzt = kzs ? kzs : g.kzt;
-  // a thread's points are taken U at a time: the Green's function values and
-  // wavenumbers of all U are loaded before any is used, so that their global-memory
-  // latencies overlap
   const bool pre = NC == 3 && zmode != Z_REGULARISE && !g.allper && !g.kernel2;
-  auto point = [&](int t, R kxp, R Gp) {
-    const int q = t >> tks, kk = t - (q << tks);
+  const int nks = __ffs(nk) - 1;  // a power of two
+  for (int t = threadIdx.x; t < N * nk; t += blockDim.x) {
+    const int q = t >> nks, kk = t - (q << nks);
     const int z = zpos ? zpos[q] : q;
-    const int kx_i = k0 + kk;
-    C *v = Cb + q * L + kk * NC;
-    z_point<R, NC>(g, v, kx_i, kxp, Gp, ky, kyc, y, iy, z, kzt[z], zmode, reproj, use_zeta);
-  };
-  constexpr int U = 4;
-  const int total = N * TK;
-  for (int t0 = threadIdx.x; t0 < total; t0 += U * blockDim.x) {
-    R kxv[U], Gv[U];
+    typename LineT<T>::V *p = buf + (size_t)q * LG + kk * NC;
+    LV<T> a[NC];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int t = t0 + u * (int)blockDim.x;
-      kxv[u] = R(0);
-      Gv[u] = R(0);
-      if (t < total) {
-        const int q = t >> tks, kk = t - (q << tks);
-        const int kx_i = k0 + kk;
-        if (kx_i < g.H) {
-          kxv[u] = g.kxt[kx_i];
-          if (pre) {
-            const int z = zpos ? zpos[q] : q;
-            Gv[u] = g.green[((size_t)min(z, g.M[2] - z) * g.gM1 + iy) * g.H + kx_i];
-          }
-        }
-      }
+    for (int c = 0; c < NC; c++) a[c] = vget(p[c]);
+#pragma unroll
+    for (int h = 0; h < G; h++) {
+      const int kx_i = k0 + kk * G + h;
+      const R kxp = kx_i < g.H ? g.kxt[kx_i] : R(0);
+      const R Gp = pre ? g.green[((size_t)min(z, g.M[2] - z) * g.gM1 + iy) * g.gH + kx_i] : R(0);
+      typename cplx_t<R>::type v[NC];
+#pragma unroll
+      for (int c = 0; c < NC; c++) v[c] = lane_get(a[c], h);
+      z_point<R, NC>(g, v, kx_i, kxp, Gp, ky, kyc, y, iy, z, g.kzt[z], zmode, reproj, use_zeta);
+#pragma unroll
+      for (int c = 0; c < NC; c++) lane_set(a[c], h, v[c]);
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int t = t0 + u * (int)blockDim.x;
-      if (t < total) point(t, kxv[u], Gv[u]);
-    }
+    for (int c = 0; c < NC; c++) p[c] = vput(a[c]);
   }
 }
 
-// ---------------------------------------------------------------- fused middle of the z pass
-// Largest last radix of a z plan whose last forward phase, spectral multiply and first
-// inverse phase run in registers (three component lines of RL points a thread).
-__host__ __device__ inline bool z_fusable(const RegPlan &pl, int rsize) {
-  if (pl.bl || pl.np < 2) return false;
-  const int r = pl.rad[pl.np - 1];
-  return r >= 2 && r <= (rsize == 4 ? 8 : 6);
-}
-
-// The z pass's last forward phase, spectral multiply and first inverse phase in
-// registers: a thread takes one block of RL consecutive (digit-reversed) positions of
-// the NC component lines of one kx, runs the RL-point forward DFT of each (the last
-// decimation-in-frequency phase has no twiddles), multiplies every point, runs the
-// inverse DFTs (the first decimation-in-time phase has none either) and writes the
-// block back in place.  The arithmetic is that of the two phases and the multiply
-// done apart, so the result is the same; two shared-memory round trips and two
-// barriers per tile are saved.  Ends with a barrier.
-// NCT, TKC: the transform length and the kx tile when known at compile time (0: read
-// from pl and TK)
-template <int RL, typename R, int NC, int NCT = 0, int TKC = 0>
-__device__ __forceinline__ void z_fused_mid_r(const SolveGeom<R> &g, const RegPlan &pl,
-                                              typename cplx_t<R>::type *Cb, int L, int TK, int k0, int y, int zmode,
-                                              int reproj, int use_zeta, const int *zpos, const R *kzs) {
-  typedef typename cplx_t<R>::type C;
-  const int nblk = NCT ? NCT / RL : pl.n / RL;
-  const R ky = g.kyt[y];
-  const R kyc = (2 * y == g.M[1]) ? R(0) : ky;  // Nyquist component dropped in the curl
-  const int iy = min(y, g.M[1] - y);
-  const bool pre = NC == 3 && zmode != Z_REGULARISE && !g.allper && !g.kernel2;
-  const int tks = TKC ? (TKC == 1 ? 0 : TKC == 2 ? 1 : TKC == 4 ? 2 : TKC == 8 ? 3 : 4) : __ffs(TK) - 1;  // TK: 2^k
-  if (TKC) L = NC * TKC;
-  const int total = nblk * (TKC ? TKC : TK);
+// The plain velocity solve's middle of the z pass in registers: a thread takes one block
+// of RL consecutive positions of the three component lines of one kx group, runs the
+// last forward phase (it has no twiddles), multiplies by i G (k x w) with 2 pi folded into
+// k, runs the first inverse phase and writes the block back in place.  A block's vectors
+// start RL * LG apart, so with an odd RL (and LG = 12, 6 or 3) the eight lanes of a
+// quarter-warp fall in distinct banks; even RL share banks two to four times.
+__device__ __forceinline__ float2 ld_lines(const float *p, float2) { return __ldg(reinterpret_cast<const float2 *>(p)); }
+__device__ __forceinline__ float ld_lines(const float *p, float) { return __ldg(p); }
+__device__ __forceinline__ double ld_lines(const double *p, double) { return __ldg(p); }
+template <int RL, typename T>
+__device__ __forceinline__ void z_mid_vel(const SolveGeom<typename LineT<T>::R> &g, typename LineT<T>::V *buf, int LG,
+                                          int k0, int y, int npts) {
+  typedef typename LineT<T>::R R;
+  constexpr int G = LineT<T>::G;
+  const int nk = LG / 3, nks = __ffs(nk) - 1;
+  const T ky = pset(T(), (2 * y == g.M[1]) ? R(0) : R(6.283185307179586476925286766559) * g.kyt[y]);
+  const R *green = g.green + (size_t)min(y, g.M[1] - y) * g.gH + k0;
+  const int total = (npts / RL) << nks;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    const int beta = t >> tks, kk = t - (beta << tks);
-    const int kx_i = k0 + kk;
-    C *base = Cb + (size_t)beta * RL * L + kk * NC;
-    int zs[RL];
-    R Gv[RL];
-    const R kxp = kx_i < g.H ? g.kxt[kx_i] : R(0);
+    const int beta = t >> nks, kk = t - (beta << nks);
+    typename LineT<T>::V *p = buf + (size_t)(beta * RL) * LG + kk * 3;
+    const T kx = ld_lines(g.kxv + k0 + kk * G, T());
+    T Gv[RL];
+    R kzs[RL];
 #pragma unroll
     for (int k = 0; k < RL; k++) {
-      zs[k] = zpos[beta * RL + k];
-      Gv[k] = R(0);
-      if (pre && kx_i < g.H) Gv[k] = g.green[((size_t)min(zs[k], g.M[2] - zs[k]) * g.gM1 + iy) * g.H + kx_i];
+      Gv[k] = ld_lines(green + __ldg(g.zoff + beta * RL + k) + kk * G, T());
+      kzs[k] = __ldg(g.kzv + beta * RL + k);
     }
-    C a[NC][RL];
-    // FP32, compile-time kx tile 8, three components and RL = 4: the four blocks of a
-    // warp sit a multiple of 16 complex apart, so the same position of every block
-    // falls in the same banks.  Threads of odd blocks walk their positions rotated
-    // by one (position j + 1 at step j), which puts the warp's two block parities 8
-    // complex apart: two wavefronts per access instead of four.  Only the order of
-    // the loads and stores changes.  (FP64 accesses need four wavefronts anyway.)
-    constexpr bool ROT = sizeof(R) == 4 && RL == 4 && TKC == 8 && NC == 3;
-    const int rot = ROT ? (beta & 1) : 0;
+    LV<T> a[3][RL];
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-      if constexpr (ROT) {
-        C tmp[RL];
+    for (int c = 0; c < 3; c++) {
 #pragma unroll
-        for (int j = 0; j < RL; j++) tmp[j] = base[((j + rot) & (RL - 1)) * L + c];
-#pragma unroll
-        for (int j = 0; j < RL; j++) a[c][j] = rot ? tmp[(j + RL - 1) & (RL - 1)] : tmp[j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < RL; j++) a[c][j] = base[j * L + c];
-      }
-      dft<RL, false>(a[c]);
+      for (int j = 0; j < RL; j++) a[c][j] = vget(p[j * LG + c]);
+      ldft<RL, false, T>(a[c]);
     }
 #pragma unroll
     for (int k = 0; k < RL; k++) {
-      C v[NC];
-#pragma unroll
-      for (int c = 0; c < NC; c++) v[c] = a[c][k];
-      z_point<R, NC>(g, v, kx_i, kxp, Gv[k], ky, kyc, y, iy, zs[k], kzs[zs[k]], zmode, reproj, use_zeta);
-#pragma unroll
-      for (int c = 0; c < NC; c++) a[c][k] = v[c];
+      const T kz = pset(T(), kzs[k]), f = Gv[k], fm = pneg(Gv[k]);
+      const LV<T> w1 = a[0][k], w2 = a[1][k], w3 = a[2][k];
+      const T c1r = pfmap(w3.re, ky, pneg(pmulp(w2.re, kz))), c1i = pfmap(w3.im, ky, pneg(pmulp(w2.im, kz)));
+      const T c2r = pfmap(w1.re, kz, pneg(pmulp(w3.re, kx))), c2i = pfmap(w1.im, kz, pneg(pmulp(w3.im, kx)));
+      const T c3r = pfmap(w2.re, kx, pneg(pmulp(w1.re, ky))), c3i = pfmap(w2.im, kx, pneg(pmulp(w1.im, ky)));
+      a[0][k] = {pmulp(fm, c1i), pmulp(f, c1r)};
+      a[1][k] = {pmulp(fm, c2i), pmulp(f, c2r)};
+      a[2][k] = {pmulp(fm, c3i), pmulp(f, c3r)};
     }
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-      dft<RL, true>(a[c]);
-      if constexpr (ROT) {
+    for (int c = 0; c < 3; c++) {
+      ldft<RL, true, T>(a[c]);
 #pragma unroll
-        for (int j = 0; j < RL; j++) base[((j + rot) & (RL - 1)) * L + c] = rot ? a[c][(j + 1) & (RL - 1)] : a[c][j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < RL; j++) base[j * L + c] = a[c][j];
-      }
+      for (int j = 0; j < RL; j++) p[j * LG + c] = vput(a[c][j]);
     }
   }
-  __syncthreads();
+}
+// the velocity multiplier is G(k) times the curl: kernel 1, or all axes periodic (either
+// kernel) unless the filter goes with it
+template <typename R> __host__ __device__ inline bool z_plain(const SolveGeom<R> &g, int use_zeta) {
+  return g.allper ? !use_zeta : !g.kernel2;
+}
+// radices of a last phase that z_mid_vel takes
+__host__ __device__ constexpr bool z_mid_radix(int r) { return r >= 2 && r <= 6; }
+// block of the multiply of a plan whose last radix is r
+__host__ __device__ constexpr int z_mid_block(int r) { return z_mid_radix(r) ? r : 1; }
+template <typename T>
+__device__ __forceinline__ void z_mid_vel_any(const SolveGeom<typename LineT<T>::R> &g, typename LineT<T>::V *buf,
+                                              int LG, int k0, int y, int npts, int rl) {
+  switch (rl) {
+    case 2: z_mid_vel<2, T>(g, buf, LG, k0, y, npts); break;
+    case 3: z_mid_vel<3, T>(g, buf, LG, k0, y, npts); break;
+    case 4: z_mid_vel<4, T>(g, buf, LG, k0, y, npts); break;
+    case 5: z_mid_vel<5, T>(g, buf, LG, k0, y, npts); break;
+    case 6: z_mid_vel<6, T>(g, buf, LG, k0, y, npts); break;
+    default: z_mid_vel<1, T>(g, buf, LG, k0, y, npts); break;
+  }
 }
 
-template <typename R, int NC>
-__device__ __forceinline__ void z_fused_mid(const SolveGeom<R> &g, const RegPlan &pl, typename cplx_t<R>::type *Cb,
-                                            int L, int TK, int k0, int y, int zmode, int reproj, int use_zeta,
-                                            const int *zpos, const R *kzs) {
-  switch (pl.rad[pl.np - 1]) {
-    case 2: z_fused_mid_r<2, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs); break;
-    case 3: z_fused_mid_r<3, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs); break;
-    case 4: z_fused_mid_r<4, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs); break;
-    case 5: z_fused_mid_r<5, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs); break;
-    case 6: z_fused_mid_r<6, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs); break;
-    default:
-      if constexpr (sizeof(R) == 4) {
-        if (pl.rad[pl.np - 1] == 7) z_fused_mid_r<7, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs);
-        else z_fused_mid_r<8, R, NC>(g, pl, Cb, L, TK, k0, y, zmode, reproj, use_zeta, zpos, kzs);
-      }
-      break;
-  }
-}
+// the Stockham passes' vectors: FP32 pairs, FP64 single lines
+template <typename R> struct StockLine;
+template <> struct StockLine<float> { typedef float2 T; };
+template <> struct StockLine<double> { typedef double T; };
 
 // lines along y (lmode L_FWD / L_INV) or the fused z pass (L_Z, or L_FWD along z
 // for the Green's function transform).  axis: 1 = y, 2 = z.
@@ -469,7 +466,8 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_lines(SolveGeom<R> g, LineT
   const int ntiles = lt.nouter * lt.nkt;
   auto load = [&](int tile) {
     const int o = tile / lt.nkt, kt = tile - o * lt.nkt;
-    tile_rows_load<R>(reinterpret_cast<C *>(S), in, o * lt.in_os + (long long)kt * TK, lt.in_rs, lt.rows_in, L, NC);
+    tile_rows_load<R>(reinterpret_cast<C *>(S), in, spec_off<R>(o * lt.in_os, lt.in_kb, kt * TK), lt.in_rs, lt.rows_in, L,
+                      NC);
     cp_async_commit();
   };
   int tile = blockIdx.x;
@@ -488,183 +486,261 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_lines(SolveGeom<R> g, LineT
     } else {
       res = vfft_chain<false, R>(S, A, B, LG, sd, tw, lm, hook);
       if (lmode == L_Z) {
-        z_multiply<R, NC>(g, reinterpret_cast<C *>(res), L, TK, kt * TK, g.yk ? g.yk[o] : o, zmode, reproj,
-                          use_zeta, nullptr);
+        typedef typename StockLine<R>::T T;
+        z_multiply<T, NC>(g, reinterpret_cast<typename LineT<T>::V *>(res), LG, kt * TK, g.yk ? g.yk[o] : o, zmode,
+                          reproj, use_zeta, nullptr);
         __syncthreads();
         res = vfft_chain<true, R>(res, A, B, LG, sd, tw, lm, NoHook());
       }
     }
-    tile_rows_store<R>(out, reinterpret_cast<C *>(res), o * lt.out_os + (long long)kt * TK, lt.out_rs, lt.rows_out,
-                       L, NC);
+    tile_rows_store<R>(out, reinterpret_cast<C *>(res), spec_off<R>(o * lt.out_os, lt.out_kb, kt * TK), lt.out_rs,
+                       lt.rows_out, L, NC);
     __syncthreads();
   }
   cp_async_wait_all();
 }
 
-// Register-engine version of k_lines (lmode L_FWD along y, L_INV along y, L_Z):
-// one tile buffer per CTA, transformed in place; the first phase reads the rows
-// from global memory (zero padding not read) and the last phase writes them back
-// (truncation not written).  Forward y output rows are stored in digit-reversed
-// order (row -> ky through g.yk); the z pass keeps its spectrum digit-reversed in
-// shared memory (position -> kz through g.zk).  Several CTAs share an SM so that
-// one CTA's loads overlap another's transforms.
-constexpr int RL_THREADS = 256;
+// Register-engine line pass (lmode L_FWD along y or z, L_INV along y, L_Z): one tile
+// buffer per CTA, transformed in place (linefft.cuh).  The y spectrum rows are stored by
+// position (row -> ky through g.yk); the z pass keeps its spectrum by position in shared
+// memory (position -> kz through g.zk).  Several CTAs share an SM so that one CTA's loads
+// overlap another's transforms.
+constexpr int LINE_THREADS_MAX = 256;   // 128 or 256 threads, at most 128 registers
+constexpr int LINE_CTAS = 2;
 
-// shared memory of a line pass: tables of the geometry, then the tile buffer
-template <typename R> struct RlSmem {
-  typename cplx_t<R>::type *tw, *chirp, *bpos;
-  int *zpos;
-  R *kzs;
-  typename RVec<R>::V *buf;
+struct LineSmem {
+  LineTabs tabs;
+  unsigned chirp, bpos;
 };
+__host__ __device__ inline bool plan_twiddles(const LinePlan &p) {
+  bool t = false;
+  for (int i = 0; i < p.np; i++) t = t || p.tmul[i] != 0;
+  return t;
+}
+// bytes of the tables of a line pass in shared memory; wsize / csize: a twiddle, a
+// complex value
+__host__ __device__ inline size_t line_tab_bytes(const LinePlan &p, size_t wsize, size_t csize) {
+  size_t b = 0;
+  if (plan_twiddles(p)) b += (size_t)p.n * wsize;
+  if (p.split) b += (size_t)p.n * wsize;
+  b = (b + 15) & ~(size_t)15;
+  if (!p.bl) b += ((size_t)(p.n / p.rad[0]) * sizeof(int) + 15) & ~(size_t)15;
+  else b += ((size_t)(p.bn + p.n) * csize + 15) & ~(size_t)15;
+  return b;
+}
 
-// carves the shared memory of a line pass of geometry g and stages its tables (the
-// caller synchronises before the first tile)
-template <typename R>
-__device__ __forceinline__ RlSmem<R> rl_setup(const SolveGeom<R> &g, const LineTiles &lt, int axis, int lmode,
-                                              unsigned char *smem_raw) {
-  typedef typename cplx_t<R>::type C;
-  typedef typename RVec<R>::V V;
-  const RegPlan &pl = (axis == 1) ? g.ry : g.rz;
-  const int m = pl.n, nl = lt.n;
-  const bool blue = pl.bl != 0;
-  RlSmem<R> s;
-  unsigned char *sp = smem_raw;
-  s.tw = reinterpret_cast<C *>(sp);
-  sp += ((size_t)m * sizeof(C) + 15) & ~(size_t)15;
-  s.zpos = reinterpret_cast<int *>(sp);
-  sp += ((size_t)nl * sizeof(int) + 15) & ~(size_t)15;
-  s.kzs = reinterpret_cast<R *>(sp);
-  sp += ((size_t)nl * sizeof(R) + 15) & ~(size_t)15;
-  s.chirp = reinterpret_cast<C *>(sp);
-  s.bpos = s.chirp + nl;
-  if (blue) sp += ((size_t)(nl + m) * sizeof(C) + 15) & ~(size_t)15;
-  s.buf = reinterpret_cast<V *>(sp);
-  const C *twg = (axis == 1) ? g.rtwy : g.rtwz;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) s.tw[i] = twg[i];
-  if (lmode == L_Z)
-    for (int i = threadIdx.x; i < nl; i += blockDim.x) {
-      s.zpos[i] = g.zk[i];
-      s.kzs[i] = g.kzt[i];
-    }
-  if (blue) {
-    const C *cg = (axis == 1) ? g.rchy : g.rchz, *bg = (axis == 1) ? g.rby : g.rbz;
-    for (int i = threadIdx.x; i < nl; i += blockDim.x) s.chirp[i] = cg[i];
-    for (int i = threadIdx.x; i < m; i += blockDim.x) s.bpos[i] = bg[i];
+// carves the tables of plan pl out of shared memory and stages them (Bluestein: the product
+// table of one direction; the caller
+// synchronises before the first tile); tabs.buf: the first byte after them
+template <typename T, typename C>
+__device__ __forceinline__ LineSmem line_tables(const LinePlan &pl, const C *rtw, const C *rts, const int *rb0,
+                                                const C *cg, const C *bg, bool inverse) {
+  typedef typename LineT<T>::W W;
+  const int n = pl.n;
+  LineSmem s;
+  unsigned at = 0;
+  s.tabs.tw = s.tabs.tws = s.tabs.rbase = s.chirp = s.bpos = 0;
+  if (plan_twiddles(pl)) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) line_smem_at<W>(at)[i] = wput<T>(rtw[i]);
+    s.tabs.tw = at;
+    at += (unsigned)(n * sizeof(W));
   }
+  if (pl.split) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) line_smem_at<W>(at)[i] = wput<T>(rts[i]);
+    s.tabs.tws = at;
+    at += (unsigned)(n * sizeof(W));
+  }
+  at = (at + 15) & ~15u;
+  if (!pl.bl) {
+    const int m = n / pl.rad[0];
+    for (int i = threadIdx.x; i < m; i += blockDim.x) line_smem_at<int>(at)[i] = rb0[i];
+    s.tabs.rbase = at;
+    at += ((unsigned)m * sizeof(int) + 15) & ~15u;
+  } else {
+    s.chirp = at;
+    s.bpos = at + (unsigned)(pl.bn * sizeof(C));
+    for (int i = threadIdx.x; i < pl.bn; i += blockDim.x) line_smem_at<C>(s.chirp)[i] = cg[i];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) line_smem_at<C>(s.bpos)[i] = bg[inverse ? n + i : i];
+    at += (unsigned)((pl.bn + n) * sizeof(C) + 15) & ~15u;
+  }
+  s.tabs.buf = at;
   return s;
+}
+template <typename T>
+__device__ __forceinline__ LineSmem line_setup(const SolveGeom<typename LineT<T>::R> &g, int axis, int lmode) {
+  return axis == 1 ? line_tables<T>(g.ly, g.rtwy, g.rtsy, g.rby0, g.rchy, g.rby, lmode == L_INV)
+                   : line_tables<T>(g.lz, g.rtwz, g.rtsz, g.rbz0, g.rchz, g.rbz, lmode == L_INV);
+}
+
+// the rows of tile (o, k0) of a line pass
+template <typename T>
+__device__ __forceinline__ LineIo<T> line_io(const LineTiles &lt, const typename cplx_t<typename LineT<T>::R>::type *in,
+                                             typename cplx_t<typename LineT<T>::R>::type *out, int nc, int o, int k0) {
+  typedef typename LineT<T>::R R;
+  typedef typename LineT<T>::V V;
+  typedef typename cplx_t<R>::type C;
+  constexpr int G = LineT<T>::G;
+  LineIo<T> io;
+  const long long bi = spec_off<R>(o * lt.in_os, lt.in_kb, k0) * nc, bo = spec_off<R>(o * lt.out_os, lt.out_kb, k0) * nc;
+  if constexpr (sizeof(T) == 4) {
+    // single FP32 line: the first word of its pair, plus the kx parity
+    const int odd = k0 & 1;
+    io.in = reinterpret_cast<const V *>(reinterpret_cast<const R *>(in + bi - odd * nc) + odd);
+    io.out = reinterpret_cast<V *>(reinterpret_cast<R *>(out + bo - odd * nc) + odd);
+  } else {
+    io.in = reinterpret_cast<const V *>(in + bi);
+    io.out = reinterpret_cast<V *>(out + bo);
+  }
+  io.rs_in = lt.in_rs * nc / G;
+  io.rs_out = lt.out_rs * nc / G;
+  io.rows_in = lt.rows_in;
+  io.rows_out = lt.rows_out;
+  return io;
 }
 
 // one tile of a line pass (ends with a barrier)
-template <typename R, int NC, bool WIDE>
-__device__ __forceinline__ void rl_tile(const SolveGeom<R> &g, const LineTiles &lt, const typename cplx_t<R>::type *in,
-                                        typename cplx_t<R>::type *out, int axis, int lmode, int zmode, int reproj,
-                                        int use_zeta, const RlSmem<R> &s, int tile) {
-  typedef typename cplx_t<R>::type C;
-  constexpr int G = RVec<R>::G;
-  const RegPlan &pl = (axis == 1) ? g.ry : g.rz;
-  const int nl = lt.n, TK = lt.TK, L = NC * TK, LG = L / G;
+template <typename T>
+__device__ __forceinline__ void line_tile(const SolveGeom<typename LineT<T>::R> &g, const LineTiles &lt,
+                                          const typename cplx_t<typename LineT<T>::R>::type *in,
+                                          typename cplx_t<typename LineT<T>::R>::type *out, int nc, int axis, int lmode,
+                                          int zmode, int reproj, int use_zeta, const LineSmem &s, int tile) {
+  typedef typename LineT<T>::V V;
+  typedef LineIo<T> IO;
+  const LinePlan &pl = (axis == 1) ? g.ly : g.lz;
+  const int LG = nc * lt.TK / LineT<T>::G;
+  const RtPlan rp{pl, LG, lt.dLG};
   const bool blue = pl.bl != 0;
-  const int o = tile / lt.nkt, kt = tile - o * lt.nkt;
-  PhaseGlobal gl;
-  gl.in = in + (o * lt.in_os + (long long)kt * TK) * NC;
-  gl.out = out + (o * lt.out_os + (long long)kt * TK) * NC;
-  gl.rs_in = lt.in_rs * NC;
-  gl.rs_out = lt.out_rs * NC;
-  gl.rows_in = lt.rows_in;
-  gl.rows_out = lt.rows_out;
-  if (lmode == L_FWD) {
-    if (blue) bfft<R, false>(pl, s.buf, LG, lt.dLG, s.tw, s.chirp, s.bpos, true, true, gl, lt.rows_in, nl);
-    else rfft_fwd<R, WIDE>(pl, s.buf, LG, lt.dLG, s.tw, true, true, gl);
-  } else if (lmode == L_INV) {
-    if (blue) bfft<R, true>(pl, s.buf, LG, lt.dLG, s.tw, s.chirp, s.bpos, true, true, gl, nl, lt.rows_out);
-    else rfft_inv<R, WIDE>(pl, s.buf, LG, lt.dLG, s.tw, true, true, gl);
-  } else if (!blue && NC == 3 && z_fusable(pl, (int)sizeof(R))) {
-    rfft_fwd<R, WIDE>(pl, s.buf, LG, lt.dLG, s.tw, true, false, gl, -1, pl.np - 1);
-    z_fused_mid<R, NC>(g, pl, reinterpret_cast<C *>(s.buf), L, TK, kt * TK, g.yk ? g.yk[o] : o, zmode, reproj,
-                       use_zeta, s.zpos, s.kzs);
-    rfft_inv<R, WIDE>(pl, s.buf, LG, lt.dLG, s.tw, false, true, gl, pl.np - 2);
-  } else {
-    if (blue) bfft<R, false>(pl, s.buf, LG, lt.dLG, s.tw, s.chirp, s.bpos, true, false, gl, lt.rows_in, nl);
-    else rfft_fwd<R, WIDE>(pl, s.buf, LG, lt.dLG, s.tw, true, false, gl);
-    z_multiply<R, NC>(g, reinterpret_cast<C *>(s.buf), L, TK, kt * TK, g.yk ? g.yk[o] : o, zmode, reproj, use_zeta,
-                      blue ? nullptr : s.zpos, s.kzs);
-    __syncthreads();
-    if (blue) bfft<R, true>(pl, s.buf, LG, lt.dLG, s.tw, s.chirp, s.bpos, false, true, gl, nl, lt.rows_out);
-    else rfft_inv<R, WIDE>(pl, s.buf, LG, lt.dLG, s.tw, false, true, gl);
-  }
-}
-
-template <typename R, int NC, bool WIDE = false>
-__global__ void __launch_bounds__(RL_THREADS, WIDE ? 2 : RMinBlocks<R>::v) k_rlines(SolveGeom<R> g, LineTiles lt,
-                                                          const typename cplx_t<R>::type *in,
-                                                          typename cplx_t<R>::type *out, int axis, int lmode,
-                                                          int zmode, int reproj, int use_zeta) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const RlSmem<R> s = rl_setup<R>(g, lt, axis, lmode, smem_raw);
-  __syncthreads();
-  const int ntiles = lt.nouter * lt.nkt;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    rl_tile<R, NC, WIDE>(g, lt, in, out, axis, lmode, zmode, reproj, use_zeta, s, tile);
-}
-
-// ---------------------------------------------------------------- compile-time line passes
-// rl_tile for a plan P (no Bluestein) and a kx tile TK known at compile time: the
-// same phases, multiply and fused middle, so the results equal those of rl_tile bit
-// for bit.
-template <typename P, typename R> __host__ __device__ constexpr bool ct_z_fusable() {
-  return P::np >= 2 && P::rad(P::np - 1) >= 2 && P::rad(P::np - 1) <= (sizeof(R) == 4 ? 8 : 6);
-}
-
-template <typename R, int NC, typename P, int TK>
-__device__ __forceinline__ void rl_tile_ct(const SolveGeom<R> &g, const LineTiles &lt,
-                                           const typename cplx_t<R>::type *in, typename cplx_t<R>::type *out,
-                                           int lmode, int zmode, int reproj, int use_zeta, const RlSmem<R> &s,
-                                           int tile) {
-  typedef typename cplx_t<R>::type C;
-  constexpr int L = NC * TK, LG = L / RVec<R>::G;
-  const int o = tile / lt.nkt, kt = tile - o * lt.nkt;
-  PhaseGlobal gl;
-  gl.in = in + (o * lt.in_os + (long long)kt * TK) * NC;
-  gl.out = out + (o * lt.out_os + (long long)kt * TK) * NC;
-  gl.rs_in = lt.in_rs * NC;
-  gl.rs_out = lt.out_rs * NC;
-  gl.rows_in = lt.rows_in;
-  gl.rows_out = lt.rows_out;
-  if (lmode == L_FWD) {
-    rfft_fwd_ct<P, R, LG, true, true, P::np>(s.buf, s.tw, gl);
-  } else if (lmode == L_INV) {
-    rfft_inv_ct<P, R, LG, true, true, P::np - 1>(s.buf, s.tw, gl);
-  } else {
-    const int y = g.yk ? g.yk[o] : o;
-    if constexpr (NC == 3 && ct_z_fusable<P, R>()) {
-      rfft_fwd_ct<P, R, LG, true, false, P::np - 1>(s.buf, s.tw, gl);
-      z_fused_mid_r<P::rad(P::np - 1), R, NC, P::n, TK>(g, RegPlan(), reinterpret_cast<C *>(s.buf), L, TK, kt * TK,
-                                                        y, zmode, reproj, use_zeta, s.zpos, s.kzs);
-      rfft_inv_ct<P, R, LG, false, true, P::np - 2>(s.buf, s.tw, gl);
-    } else {
-      rfft_fwd_ct<P, R, LG, true, false, P::np>(s.buf, s.tw, gl);
-      z_multiply<R, NC>(g, reinterpret_cast<C *>(s.buf), L, TK, kt * TK, y, zmode, reproj, use_zeta, s.zpos,
-                        s.kzs);
+  int o, k0;
+  line_tile_at(lt, tile, lt.TK, o, k0);
+  const IO io = line_io<T>(lt, in, out, nc, o, k0);
+  V *const buf = line_smem_at<V>(s.tabs.buf);
+  const int y = g.yk ? g.yk[o] : o;  // z pass: the spectrum row's ky
+  const bool zvel = lmode == L_Z && zmode == Z_VEL && nc == 3 && z_plain(g, use_zeta);
+  const bool mid = zvel && !blue && pl.np >= 2 && z_mid_radix(pl.rad[pl.np - 1]);
+  const int nrep = lmode == L_Z && blue ? 2 : 1;
+  for (int rep = 0; rep < nrep; rep++) {
+    const bool binv = lmode == L_INV || rep == 1;
+    if (blue) {
+      lchirp_in<T, IO>(s.tabs.buf, pl.n, LG, lt.dLG, s.chirp, rep == 0 && lmode != L_INV ? lt.rows_in : pl.bn, binv,
+                       rep == 0, io);
       __syncthreads();
-      rfft_inv_ct<P, R, LG, false, true, P::np - 1>(s.buf, s.tw, gl);
+    }
+    if (blue || lmode != L_INV) {
+      const int pe = mid ? pl.np - 1 : pl.np;
+      for (int p = 0; p < pe; p++) {
+        lphase_any<false, true, T, IO>(rp, p, s.tabs, io, !blue, false, !blue && lmode == L_FWD && p == pl.np - 1);
+        __syncthreads();
+      }
+    }
+    if (blue) {
+      // (the z pass's inverse table stays in global memory)
+      typedef typename cplx_t<typename LineT<T>::R>::type C;
+      lchirp_mul<T>(s.tabs.buf, pl.n, LG, lt.dLG, rep == 1 ? g.rbz + pl.n : line_smem_at<C>(s.bpos));
+      __syncthreads();
+    } else if (lmode == L_Z) {
+      if (zvel) z_mid_vel_any<T>(g, buf, LG, k0, y, plan_points(pl), mid ? pl.rad[pl.np - 1] : 1);
+      else if (nc == 3) z_multiply<T, 3>(g, buf, LG, k0, y, zmode, reproj, use_zeta, g.zk);
+      else z_multiply<T, 1>(g, buf, LG, k0, y, zmode, reproj, use_zeta, g.zk);
+      __syncthreads();
+    }
+    if (blue || lmode != L_FWD) {
+      for (int p = mid ? pl.np - 2 : pl.np - 1; p >= 0; p--) {
+        lphase_any<true, true, T, IO>(rp, p, s.tabs, io, !blue, !blue && lmode == L_INV && p == pl.np - 1, false);
+        __syncthreads();
+      }
+    }
+    if (blue) {
+      const bool last = rep == nrep - 1;
+      lchirp_out<T, IO>(s.tabs.buf, pl.n, LG, lt.dLG, s.chirp, last && lmode != L_FWD ? lt.rows_out : pl.bn, binv,
+                        last, io);
+      __syncthreads();
+      if (!last) {
+        if (nc == 3) z_multiply<T, 3>(g, buf, LG, k0, y, zmode, reproj, use_zeta, nullptr);
+        else z_multiply<T, 1>(g, buf, LG, k0, y, zmode, reproj, use_zeta, nullptr);
+        __syncthreads();
+      }
     }
   }
 }
 
-// k_rlines for the compile-time plan (N; R0, R1, R2) and kx tile TK
-template <typename R, int NC, bool WIDE, int N, int R0, int R1, int R2, int TK>
-__global__ void __launch_bounds__(RL_THREADS, WIDE ? 2 : RMinBlocks<R>::v) k_rlines_ct(SolveGeom<R> g, LineTiles lt,
-                                                          const typename cplx_t<R>::type *in,
-                                                          typename cplx_t<R>::type *out, int axis, int lmode,
-                                                          int zmode, int reproj, int use_zeta) {
-  static_assert(RL_THREADS == REG_THREADS, "the compile-time phases stride by REG_THREADS");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const RlSmem<R> s = rl_setup<R>(g, lt, axis, lmode, smem_raw);
+template <typename T>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS)
+    k_rlines(SolveGeom<typename LineT<T>::R> g, LineTiles lt, const typename cplx_t<typename LineT<T>::R>::type *in,
+             typename cplx_t<typename LineT<T>::R>::type *out, int nc, int axis, int lmode, int zmode, int reproj,
+             int use_zeta) {
+  const LineSmem s = line_setup<T>(g, axis, lmode);
   __syncthreads();
   const int ntiles = lt.nouter * lt.nkt;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    rl_tile_ct<R, NC, CtPlan<N, R0, R1, R2>, TK>(g, lt, in, out, lmode, zmode, reproj, use_zeta, s, tile);
+    line_tile<T>(g, lt, in, out, nc, axis, lmode, zmode, reproj, use_zeta, s, tile);
+}
+
+// ---------------------------------------------------------------- compile-time line passes
+// forward phases P .. PE - 1 and inverse phases P .. 0 of a compile-time plan, each with its
+// barrier
+template <typename T, typename PL, int P, int PE, bool GOUT>
+__device__ __forceinline__ void ct_forward(const LineTabs &tb, const LineIo<T> &io) {
+  if constexpr (P < PE) {
+    lphase<PL::rad(P), false, T, LineIo<T>, PL>(PL(), P, tb, io, true, false, GOUT && P == PL::NP - 1);
+    __syncthreads();
+    ct_forward<T, PL, P + 1, PE, GOUT>(tb, io);
+  }
+}
+template <typename T, typename PL, int P, bool GIN>
+__device__ __forceinline__ void ct_inverse(const LineTabs &tb, const LineIo<T> &io) {
+  if constexpr (P >= 0) {
+    lphase<PL::rad(P), true, T, LineIo<T>, PL>(PL(), P, tb, io, true, GIN && P == PL::NP - 1, false);
+    __syncthreads();
+    ct_inverse<T, PL, P - 1, GIN>(tb, io);
+  }
+}
+// asks for a tile's input rows (`bytes` each) to be brought into L2
+template <typename T> __device__ __forceinline__ void line_prefetch(const LineIo<T> &io, int rows, unsigned bytes) {
+  for (int r = threadIdx.x; r < rows; r += blockDim.x)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(io.in + (long long)r * io.rs_in)),
+                 "r"(bytes)
+                 : "memory");
+}
+// k_rlines for a compile-time plan PL of three-component lines, one mode each (L_Z: the
+// plain velocity solve with the last digit in the multiply)
+template <typename T, int LMODE, typename PL>
+__device__ __forceinline__ void line_tile_ct(const SolveGeom<typename LineT<T>::R> &g, const LineIo<T> &io,
+                                             const LineTabs &tb, int o, int k0) {
+  typedef typename LineT<T>::V V;
+  if constexpr (LMODE == L_FWD) {
+    ct_forward<T, PL, 0, PL::NP, true>(tb, io);
+  } else if constexpr (LMODE == L_INV) {
+    ct_inverse<T, PL, PL::NP - 1, true>(tb, io);
+  } else {
+    constexpr int RL = PL::NP > 1 ? z_mid_block(PL::rad(PL::NP - 1)) : 1;
+    constexpr int PE = RL > 1 ? PL::NP - 1 : PL::NP;
+    ct_forward<T, PL, 0, PE, false>(tb, io);
+    z_mid_vel<RL, T>(g, line_smem_at<V>(tb.buf), PL::LG(), k0, g.yk ? g.yk[o] : o,
+                     PL::split() ? 2 * PL::n() : PL::n());
+    __syncthreads();
+    ct_inverse<T, PL, PE - 1, false>(tb, io);
+  }
+}
+template <typename T, int LMODE, typename PL>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS)
+    k_rlines_ct(SolveGeom<typename LineT<T>::R> g, LineTiles lt, const typename cplx_t<typename LineT<T>::R>::type *in,
+                typename cplx_t<typename LineT<T>::R>::type *out, int, int axis, int, int, int, int) {
+  constexpr int TK = PL::LG() * LineT<T>::G / 3;
+  const LineSmem s = line_setup<T>(g, axis, LMODE);
+  __syncthreads();
+  const int ntiles = lt.nouter * lt.nkt;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    int o, k0;
+    line_tile_at(lt, tile, TK, o, k0);
+    const LineIo<T> io = line_io<T>(lt, in, out, 3, o, k0);
+    if (LMODE == L_Z && tile + (int)gridDim.x < ntiles) {
+      // the next tile's rows on their way to L2 while this one is transformed
+      int no, nk;
+      line_tile_at(lt, tile + gridDim.x, TK, no, nk);
+      line_prefetch<T>(line_io<T>(lt, in, out, 3, no, nk), PL::n(), PL::LG() * 16);
+    }
+    line_tile_ct<T, LMODE, PL>(g, io, s.tabs, o, k0);
+  }
 }
 
 // ---------------------------------------------------------------- batches of patches
@@ -685,8 +761,12 @@ template <typename R> struct PassDesc {
   int vec16;        // x forward: rows are staged in 16-byte chunks
   int first;        // first work item of the patch
   FastDiv dLG;      // x passes: division by the line vectors of a tile
-  int ntiles, pad;
+  int ntiles;
+  int patch;        // index into the caller's arrays
+  int cls;          // compile-time plan (plan_class), 0: run-time plan
 };
+// key of a compile-time plan in the batched kernels
+__host__ __device__ constexpr int plan_class(int n, int split, int lg) { return n * 4 + split * 2 + (lg == 12 ? 1 : 0); }
 struct BatchWork {
   const void *desc;   // PassDesc<R>[npatch]
   int npatch, nitems, chunk, pad;
@@ -732,86 +812,135 @@ __device__ __forceinline__ bool batch_patch(const BatchWork &bw, int item, PassD
   return true;
 }
 
-template <typename R, int NC, bool WIDE = false>
-__global__ void __launch_bounds__(RL_THREADS, WIDE ? 2 : RMinBlocks<R>::v) k_rlines_batch(BatchWork bw, int axis,
-                                                                int lmode, int zmode, int reproj, int use_zeta) {
+template <typename R>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS) k_lines_batch(BatchWork bw, int axis, int lmode, int zmode) {
   typedef typename cplx_t<R>::type C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef typename StockLine<R>::T T;
   __shared__ PassDesc<R> sd;
-  RlSmem<R> s;
+  LineSmem s;
   int cur = -1, i0, i1;
   while (batch_next(bw, i0, i1)) {
     for (int it = i0; it < i1; it++) {
       if (batch_patch<R>(bw, it, sd, cur)) {
-        s = rl_setup<R>(sd.g, sd.lt, axis, lmode, smem_raw);
+        s = line_setup<T>(sd.g, axis, lmode);
         __syncthreads();
       }
-      rl_tile<R, NC, WIDE>(sd.g, sd.lt, reinterpret_cast<const C *>(sd.in), reinterpret_cast<C *>(sd.out), axis,
-                           lmode, zmode, reproj, use_zeta, s, it - sd.first);
+      line_tile<T>(sd.g, sd.lt, reinterpret_cast<const C *>(sd.in), reinterpret_cast<C *>(sd.out), 3, axis, lmode,
+                   zmode, 0, 0, s, it - sd.first);
     }
   }
 }
 
 // ---------------------------------------------------------------- x passes, register engine
-// As k_xfwd / k_xinv below (R2C / C2R through a half-length complex transform),
-// with the transform done in place by the register engine: the packed line has
-// its second half zero (not read), and the digit-reversed spectrum is addressed
-// through the frequency -> position table.
-template <typename R> struct RxSmem {
-  typename cplx_t<R>::type *tw, *ext, *chirp, *bpos;
-  int *xpos;
-  void *stage;  // raw rows (forward: reals, inverse: spectrum rows)
-  typename RVec<R>::V *buf;
+// R2C / C2R of real rows through a half-length complex transform: the packed points
+// z[m] = x[2m] + i x[2m+1], m < N = Mx/2, give the Mx-point spectrum by
+//   X[k] = (Z[k] + conj Z[N-k] - i W^k (Z[k] - conj Z[N-k])) / 2,   W = exp(-2 pi i / Mx),
+// and back by Z[k] = X[k] + conj X[N-k] + i W^-k (X[k] - conj X[N-k]).  The lines are
+// transformed as line vectors (linefft.cuh): in FP32 a vector holds one component of two
+// rows.  A free axis of even length has exactly the second half of its packed points
+// zero: a split plan.  A tile is RB rows of NC components, LG = NC RB / G vectors a
+// point, vector g = rho NC + c for row group rho.  The forward pass stages its raw rows in
+// shared memory (the next tile's rows stream in while this one is transformed) and its first
+// phase packs from there; the inverse pass reads the spectrum rows straight into the
+// twist and its last phase writes the real rows.
+struct XSmem {
+  LineTabs tabs;
+  unsigned chirp, bpos;
+  unsigned ext, xpos;
+  unsigned srow;   // first vector of every row of the tile in the spectral array
+  unsigned stage;  // forward: raw rows
+  unsigned rows;   // inverse: offset of every row of the tile in the real field, -1: none
 };
 
-// carves the shared memory of an x pass of geometry g with RB rows per tile and
-// stages its tables; inverse: the staged rows are spectrum rows of Hp complex
-template <typename R, int NC>
-__device__ __forceinline__ RxSmem<R> rx_setup(const SolveGeom<R> &g, int RB, bool inverse, unsigned char *smem_raw) {
-  typedef typename cplx_t<R>::type C;
-  typedef typename RVec<R>::V V;
-  const RegPlan &pl = g.rx;
-  const bool blue = pl.bl != 0;
-  const int N = blue ? pl.bn : pl.n, m = pl.n, H = g.H;
-  RxSmem<R> s;
-  unsigned char *sp = smem_raw;
-  s.tw = reinterpret_cast<C *>(sp);
-  sp += ((size_t)m * sizeof(C) + 15) & ~(size_t)15;
-  s.ext = reinterpret_cast<C *>(sp);
-  sp += ((size_t)H * sizeof(C) + 15) & ~(size_t)15;
-  s.xpos = reinterpret_cast<int *>(sp);
-  sp += ((size_t)N * sizeof(int) + 15) & ~(size_t)15;
-  s.chirp = reinterpret_cast<C *>(sp);
-  s.bpos = s.chirp + N;
-  if (blue) sp += ((size_t)(N + m) * sizeof(C) + 15) & ~(size_t)15;
-  s.stage = sp;
-  if (inverse) sp += (size_t)RB * g.Hp * NC * sizeof(C);
-  else sp += ((size_t)RB * g.P[0] * NC * sizeof(R) + 15) & ~(size_t)15;
-  s.buf = reinterpret_cast<V *>(sp);
-  for (int i = threadIdx.x; i < m; i += blockDim.x) s.tw[i] = g.rtwx[i];
-  for (int i = threadIdx.x; i < N; i += blockDim.x) s.xpos[i] = g.xpos[i];
-  for (int i = threadIdx.x; i < H; i += blockDim.x) s.ext[i] = g.rextx[i];
-  if (blue) {
-    for (int i = threadIdx.x; i < N; i += blockDim.x) s.chirp[i] = g.rchx[i];
-    for (int i = threadIdx.x; i < m; i += blockDim.x) s.bpos[i] = g.rbx[i];
+// input of the forward transform: packed point m of the staged rows (rows of P0 NC reals)
+template <typename T, int NC> struct XStageIo {
+  typedef typename LineT<T>::R R;
+  unsigned stage;
+  int P0;
+  int rows_in, rows_out;
+  __device__ __forceinline__ LV<T> load(int m, int g) const {
+    const int rho = g / NC, c = g - rho * NC;
+    const bool odd = 2 * m + 1 < P0;
+    const R *p = line_smem_at<R>(stage) + rho * LineT<T>::G * P0 * NC + 2 * m * NC + c;
+    if constexpr (LineT<T>::G == 2) {
+      const R *q = p + P0 * NC;
+      return {make_float2(p[0], q[0]), make_float2(odd ? p[NC] : R(0), odd ? q[NC] : R(0))};
+    } else {
+      return {p[0], odd ? p[NC] : R(0)};
+    }
   }
+  __device__ __forceinline__ void store(int, int, const LV<T> &) const {}
+};
+// output of the inverse transform: packed point m to the real rows (component stride cs)
+template <typename T, int NC> struct XRowIo {
+  typedef typename LineT<T>::R R;
+  R *out;
+  unsigned rows;
+  int P0, cs;
+  int rows_in, rows_out;
+  __device__ __forceinline__ LV<T> load(int, int) const { return lzero<T>(); }
+  __device__ __forceinline__ void put(int row, int m, int c, R a, R b) const {
+    const long long o = line_smem_at<long long>(rows)[row];
+    if (o < 0) return;
+    R *p = out + o + (size_t)(2 * m) * cs + c;
+    p[0] = a;
+    if (2 * m + 1 < P0) p[cs] = b;
+  }
+  __device__ __forceinline__ void store(int m, int g, const LV<T> &v) const {
+    const int rho = g / NC, c = g - rho * NC;
+    if constexpr (LineT<T>::G == 2) {
+      put(2 * rho, m, c, v.re.x, v.im.x);
+      put(2 * rho + 1, m, c, v.re.y, v.im.y);
+    } else {
+      put(rho, m, c, v.re, v.im);
+    }
+  }
+};
+
+// shared memory of an x pass of RB rows a tile (G rows a vector, wsize bytes a twiddle)
+__host__ __device__ inline size_t x_tab_bytes(const LinePlan &p, int N, int H, size_t wsize, size_t csize) {
+  return line_tab_bytes(p, wsize, csize) + (((size_t)H * csize + 15) & ~(size_t)15) +
+         (((size_t)N * sizeof(int) + 15) & ~(size_t)15);
+}
+
+template <typename T, int NC>
+__device__ __forceinline__ XSmem x_setup(const SolveGeom<typename LineT<T>::R> &g, int RB, bool inverse) {
+  typedef typename LineT<T>::R R;
+  typedef typename cplx_t<R>::type C;
+  XSmem s;
+  const LineSmem l = line_tables<T>(g.lx, g.rtwx, g.rtsx, g.rbx0, g.rchx, g.rbx, inverse);
+  s.tabs = l.tabs;
+  s.chirp = l.chirp;
+  s.bpos = l.bpos;
+  unsigned at = l.tabs.buf;
+  s.ext = at;
+  at += (unsigned)(g.H * sizeof(C) + 15) & ~15u;
+  s.xpos = at;
+  at += (unsigned)(g.N2 * sizeof(int) + 15) & ~15u;
+  for (int i = threadIdx.x; i < g.H; i += blockDim.x) line_smem_at<C>(s.ext)[i] = g.rextx[i];
+  for (int i = threadIdx.x; i < g.N2; i += blockDim.x) line_smem_at<int>(s.xpos)[i] = g.xpos[i];
+  s.srow = at;
+  at += (unsigned)(RB * sizeof(long long) + 15) & ~15u;
+  s.stage = s.rows = at;
+  if (inverse) at += (unsigned)(RB * sizeof(long long) + 15) & ~15u;
+  else at += (unsigned)(RB * g.P[0] * NC * sizeof(R) + 15) & ~15u;
+  s.tabs.buf = at;
   return s;
 }
 
 // x forward: raw rows of tile `tile` into the stage (cp.async, committed)
 template <typename R, int NC>
 __device__ __forceinline__ void rxf_load(const SolveGeom<R> &g, const R *__restrict__ in, int RB, int cs, int vec16,
-                                         const RxSmem<R> &s, int tile) {
+                                         R *stage, int tile) {
   const int P0 = g.P[0];
   const int nrows = g.P[1] * g.P[2];
-  R *Sr = reinterpret_cast<R *>(s.stage);
   const int row0 = tile * RB;
   for (int rr = 0; rr < RB; rr++) {
     const int row = row0 + rr;
     if (row >= nrows) break;
     const int y = row % g.P[1], z = row / g.P[1];
     const R *src = in + (((size_t)(z + g.off[2]) * g.ext[1] + (y + g.off[1])) * g.ext[0] + g.off[0]) * cs;
-    R *dst = Sr + (size_t)rr * P0 * NC;
+    R *dst = stage + (size_t)rr * P0 * NC;
     if (vec16) {
       const int nch = (P0 * NC * (int)sizeof(R)) / 16;
       for (int c = threadIdx.x; c < nch; c += blockDim.x)
@@ -827,98 +956,159 @@ __device__ __forceinline__ void rxf_load(const SolveGeom<R> &g, const R *__restr
   cp_async_commit();
 }
 
-// x forward of a staged tile (the caller waited for its copies and synchronised);
-// `prefetch` runs once the stage has been read.  Ends with a barrier.
-template <typename R, int NC, typename Prefetch>
-__device__ __forceinline__ void rxf_tile(const SolveGeom<R> &g, typename cplx_t<R>::type *__restrict__ X, int RB,
-                                         const FastDiv &dLG, const RxSmem<R> &s, int tile, Prefetch prefetch) {
-  typedef typename cplx_t<R>::type C;
-  constexpr int G = RVec<R>::G;
-  const RegPlan &pl = g.rx;
-  const bool blue = pl.bl != 0;
-  const int N = blue ? pl.bn : pl.n, L = NC * RB, LG = L / G, H = g.H;
-  const int P0 = g.P[0];
-  const int nrows = g.P[1] * g.P[2];
-  const int npk = (P0 + 1) / 2;  // packed points that hold data
-  const R *Sr = reinterpret_cast<const R *>(s.stage);
-  C *Bc = reinterpret_cast<C *>(s.buf);
-  const int row0 = tile * RB;
-  for (int t = threadIdx.x; t < RB * npk; t += blockDim.x) {
-    const int rr = t / npk, m = t - rr * npk;
-    const R *xr = Sr + (size_t)rr * P0 * NC;
-    const int x0 = 2 * m, x1 = 2 * m + 1;
-    const bool ok = row0 + rr < nrows;
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-      const R a = ok ? xr[x0 * NC + c] : R(0);
-      const R b = (ok && x1 < P0) ? xr[x1 * NC + c] : R(0);
-      Bc[m * L + rr * NC + c] = mk(a, b);
-    }
-  }
+// Vector v of spectral row `row` (z P1 + y): the rows of a z plane lie block by block of kx,
+// so that a y line tile is contiguous.
+template <typename R, int NC>
+__device__ __forceinline__ size_t spec_vec(const SolveGeom<R> &g, int row, int v) {
+  constexpr int XG = sizeof(R) == 4 ? 2 : 1, BV = spec_block<R>() * NC / XG;  // vectors of a block row
+  const int z = row / g.P[1], y = row - z * g.P[1];
+  const int kb = v / BV, nkb = g.Hp / spec_block<R>();
+  return (((size_t)z * nkb + kb) * g.P[1] + y) * BV + (v - kb * BV);
+}
+
+// the first vector of a row's block 0, and the stride between its blocks
+template <typename R, int NC> __device__ __forceinline__ long long spec_row0(const SolveGeom<R> &g, int row) {
+  return (long long)spec_vec<R, NC>(g, row, 0);
+}
+template <typename R, int NC> __device__ __forceinline__ long long spec_kb(const SolveGeom<R> &g) {
+  return (long long)g.P[1] * (spec_block<R>() * NC / (sizeof(R) == 4 ? 2 : 1));
+}
+
+// forward / inverse phases of the x transforms: all in shared memory but the outer end
+template <typename T, typename IO, typename PL, bool INV, int P>
+__device__ __forceinline__ void x_phase_ct(const LineTabs &tb, const IO &io) {
+  lphase<PL::rad(P), INV, T, IO, PL>(PL(), P, tb, io, true, false, false);
   __syncthreads();
-  prefetch();
-  PhaseGlobal gl;
-  gl.in = nullptr;
-  gl.out = nullptr;
-  gl.rs_in = gl.rs_out = 0;
-  gl.rows_in = gl.rows_out = N;
-  if (blue) bfft<R, false>(pl, s.buf, LG, dLG, s.tw, s.chirp, s.bpos, false, false, gl, npk, N);
-  else rfft_fwd<R>(pl, s.buf, LG, dLG, s.tw, false, false, gl, npk);
-  for (int t = threadIdx.x; t < RB * g.Hp; t += blockDim.x) {
-    const int rr = t / g.Hp, k = t - rr * g.Hp;
-    const int row = row0 + rr;
-    if (row >= nrows) continue;
-    C o[NC];
-    if (k < H) {
-      const int kk = (k == N) ? 0 : k;
-      const int km = (k == 0 || k == N) ? 0 : N - k;
-      const int pk = s.xpos[kk], pm = s.xpos[km];
-      const C w = s.ext[k];
-#pragma unroll
-      for (int c = 0; c < NC; c++) {
-        const C zk = Bc[pk * L + rr * NC + c];
-        const C zn = cconj(Bc[pm * L + rr * NC + c]);
-        const C a = cadd(zk, zn), bb = csub(zk, zn);
-        const C wb = cmul(w, bb);
-        o[c] = mk(R(0.5) * (a.x + wb.y), R(0.5) * (a.y - wb.x));  // (a - i W^k b) / 2
-      }
-    } else {
-#pragma unroll
-      for (int c = 0; c < NC; c++) o[c] = mk(R(0), R(0));
+}
+
+// row groups of a tile of a compile-time x plan
+template <typename PL, int NC> __device__ constexpr int x_groups() {
+  if constexpr (PL::RT) return 1;
+  else return PL::LG() / NC;
+}
+
+// x forward of a staged tile (the caller waited for its copies and synchronised);
+// `prefetch` runs once the stage has been read.  Ends with a barrier.  PL: a compile-time
+// plan, or RtPlan for the run-time one.
+template <typename T, int NC, typename PL, typename Prefetch>
+__device__ __forceinline__ void rxf_tile(const SolveGeom<typename LineT<T>::R> &g,
+                                         typename cplx_t<typename LineT<T>::R>::type *__restrict__ X, int RB,
+                                         const FastDiv &dLG, const XSmem &s, int tile, Prefetch prefetch) {
+  typedef typename LineT<T>::R R;
+  typedef typename cplx_t<R>::type C;
+  constexpr int G = LineT<T>::G;
+  constexpr int XG = sizeof(R) == 4 ? 2 : 1;  // kx of a spectral vector
+  const LinePlan &pl = g.lx;
+  const bool blue = pl.bl != 0;
+  const int N = g.N2, LG = NC * RB / G, P0 = g.P[0];
+  const RtPlan rp{pl, LG, dLG};
+  const int *xpos = line_smem_at<int>(s.xpos);
+  const C *ext = line_smem_at<C>(s.ext);
+  XStageIo<T, NC> io;
+  io.stage = s.stage;
+  io.P0 = P0;
+  io.rows_in = (P0 + 1) / 2;
+  io.rows_out = N;
+  const int nrows = g.P[1] * g.P[2], row0 = tile * RB;
+  long long *srow = line_smem_at<long long>(s.srow);
+  for (int rr = threadIdx.x; rr < RB; rr += blockDim.x)
+    srow[rr] = row0 + rr < nrows ? spec_row0<R, NC>(g, row0 + rr) : -1;
+  if constexpr (!PL::RT) {
+    x_phase_ct<T, XStageIo<T, NC>, PL, false, 0>(s.tabs, io);
+    prefetch();
+    if constexpr (PL::NP > 1) x_phase_ct<T, XStageIo<T, NC>, PL, false, 1>(s.tabs, io);
+    if constexpr (PL::NP > 2) x_phase_ct<T, XStageIo<T, NC>, PL, false, 2>(s.tabs, io);
+  } else {
+  if (blue) {
+    lchirp_in<T>(s.tabs.buf, pl.n, LG, dLG, s.chirp, io.rows_in, false, true, io);
+    __syncthreads();
+    prefetch();
+  }
+  for (int p = 0; p < pl.np; p++) {
+    lphase_any<false, false, T>(rp, p, s.tabs, io, !blue, false, false);
+    __syncthreads();
+    if (p == 0 && !blue) prefetch();
+  }
+  if (blue) {
+    lchirp_mul<T>(s.tabs.buf, pl.n, LG, dLG, line_smem_at<C>(s.bpos));
+    __syncthreads();
+    for (int p = pl.np - 1; p >= 0; p--) {
+      lphase_any<true, false, T>(rp, p, s.tabs, io, false, false, false);
+      __syncthreads();
     }
+    lchirp_out<T>(s.tabs.buf, pl.n, LG, dLG, s.chirp, N, false, false, io);
+    __syncthreads();
+  }
+  }
+  // the twist.  Consecutive threads: the vectors of a block row, then the tile's rows, then
+  // the next block: RB rows of 192 bytes lie together
+  const T half = pset(T(), R(0.5));
+  constexpr int BV = spec_block<R>() * NC / XG;
+  const int nrg = PL::RT ? RB / G : x_groups<PL, NC>(), nrs = __ffs(nrg) - 1;  // a power of two
+  const int nt = g.Hp / XG * NC * nrg;
+  const long long kbs = spec_kb<R, NC>(g);
+  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+    const int w0 = t / BV, kb = w0 >> nrs, rho = w0 - (kb << nrs), bv = t - w0 * BV;
+    const int v = kb * BV + bv;
+    if (srow[rho * G] < 0) continue;
+    const int kv = v / NC, c = v - kv * NC;
+    const typename LineT<T>::V *b = line_smem_at<typename LineT<T>::V>(s.tabs.buf) + rho * NC + c;
+    LV<T> o[XG];
 #pragma unroll
-    for (int c = 0; c < NC; c++) X[((size_t)row * g.Hp + k) * NC + c] = o[c];
+    for (int h = 0; h < XG; h++) {
+      const int k = kv * XG + h;
+      o[h] = lzero<T>();
+      if (k < g.H) {
+        const LV<T> zk = vget(b[xpos[k == N ? 0 : k] * LG]);
+        const LV<T> zn = vget(b[xpos[k == 0 || k == N ? 0 : N - k] * LG]);
+        const C w = ext[k];
+        const LV<T> a = {padd(zk.re, zn.re), psub(zk.im, zn.im)}, d = {psub(zk.re, zn.re), padd(zk.im, zn.im)};
+        const LV<T> t2 = lmul<T>(d, pset(T(), w.x), pset(T(), w.y));
+        o[h] = lsub_i(a, t2);  // a - i W^k d
+        o[h].re = pmulp(o[h].re, half);
+        o[h].im = pmulp(o[h].im, half);
+      }
+    }
+    const long long at = kb * kbs + bv;
+    if constexpr (G == 2) {
+      float4 *x = reinterpret_cast<float4 *>(X) + at;
+      x[srow[2 * rho]] = make_float4(o[0].re.x, o[1].re.x, o[0].im.x, o[1].im.x);
+      if (srow[2 * rho + 1] >= 0) x[srow[2 * rho + 1]] = make_float4(o[0].re.y, o[1].re.y, o[0].im.y, o[1].im.y);
+    } else if constexpr (XG == 2) {
+      reinterpret_cast<float4 *>(X)[srow[rho] + at] = make_float4(o[0].re, o[1].re, o[0].im, o[1].im);
+    } else {
+      X[srow[rho] + at] = vput(o[0]);
+    }
   }
   __syncthreads();
 }
 
-template <typename R, int NC>
-__global__ void __launch_bounds__(RL_THREADS, RMinBlocks<R>::v) k_rxfwd(SolveGeom<R> g, const R *__restrict__ in,
-                                                         typename cplx_t<R>::type *__restrict__ X, int RB, int cs,
-                                                         int vec16, FastDiv dLG) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const RxSmem<R> s = rx_setup<R, NC>(g, RB, false, smem_raw);
+template <typename T, int NC, typename PL = RtPlan>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS)
+    k_rxfwd(SolveGeom<typename LineT<T>::R> g, const typename LineT<T>::R *__restrict__ in,
+            typename cplx_t<typename LineT<T>::R>::type *__restrict__ X, int RB, int cs, int vec16, FastDiv dLG) {
+  const XSmem s = x_setup<T, NC>(g, RB, false);
   const int nrows = g.P[1] * g.P[2];
   const int ntiles = (nrows + RB - 1) / RB;
   int tile = blockIdx.x;
-  if (tile < ntiles) rxf_load<R, NC>(g, in, RB, cs, vec16, s, tile);
+  if (tile < ntiles) rxf_load<typename LineT<T>::R, NC>(g, in, RB, cs, vec16, line_smem_at<typename LineT<T>::R>(s.stage), tile);
   for (; tile < ntiles; tile += gridDim.x) {
     cp_async_wait_all();
     __syncthreads();
     const int next = tile + gridDim.x;
-    rxf_tile<R, NC>(g, X, RB, dLG, s, tile, [&]() {
-      if (next < ntiles) rxf_load<R, NC>(g, in, RB, cs, vec16, s, next);
+    rxf_tile<T, NC, PL>(g, X, RB, dLG, s, tile, [&]() {
+      if (next < ntiles) rxf_load<typename LineT<T>::R, NC>(g, in, RB, cs, vec16, line_smem_at<typename LineT<T>::R>(s.stage), next);
     });
   }
   cp_async_wait_all();
 }
 
-template <typename R, int NC>
-__global__ void __launch_bounds__(RL_THREADS, RMinBlocks<R>::v) k_rxfwd_batch(BatchWork bw, BatchIo io) {
+template <typename T, int NC>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS) k_rxfwd_batch(BatchWork bw, BatchIo bio) {
+  typedef typename LineT<T>::R R;
   typedef typename cplx_t<R>::type C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ PassDesc<R> sd;
-  RxSmem<R> s;
+  XSmem s;
   int cur = -1, i0, i1, staged = -1;
   while (batch_next(bw, i0, i1)) {
     for (int it = i0; it < i1; it++) {
@@ -927,17 +1117,17 @@ __global__ void __launch_bounds__(RL_THREADS, RMinBlocks<R>::v) k_rxfwd_batch(Ba
         staged = -1;
       }
       if (batch_patch<R>(bw, it, sd, cur)) {
-        s = rx_setup<R, NC>(sd.g, sd.RB, false, smem_raw);
+        s = x_setup<T, NC>(sd.g, sd.RB, false);
         __syncthreads();
       }
-      const R *in = reinterpret_cast<const R *>(io.p[cur]);
-      if (staged != it) rxf_load<R, NC>(sd.g, in, sd.RB, sd.cs, sd.vec16, s, it - sd.first);
+      const R *in = reinterpret_cast<const R *>(bio.p[sd.patch]);
+      if (staged != it) rxf_load<R, NC>(sd.g, in, sd.RB, sd.cs, sd.vec16, line_smem_at<R>(s.stage), it - sd.first);
       cp_async_wait_all();
       __syncthreads();
       const int next = it + 1;
       const bool pre = next < i1 && next < sd.first + sd.ntiles;
-      rxf_tile<R, NC>(sd.g, reinterpret_cast<C *>(sd.out), sd.RB, sd.dLG, s, it - sd.first, [&]() {
-        if (pre) rxf_load<R, NC>(sd.g, in, sd.RB, sd.cs, sd.vec16, s, next - sd.first);
+      rxf_tile<T, NC, RtPlan>(sd.g, reinterpret_cast<C *>(sd.out), sd.RB, sd.dLG, s, it - sd.first, [&]() {
+        if (pre) rxf_load<R, NC>(sd.g, in, sd.RB, sd.cs, sd.vec16, line_smem_at<R>(s.stage), next - sd.first);
       });
       staged = pre ? next : -1;
     }
@@ -945,139 +1135,177 @@ __global__ void __launch_bounds__(RL_THREADS, RMinBlocks<R>::v) k_rxfwd_batch(Ba
   cp_async_wait_all();
 }
 
-// x inverse: spectrum rows of tile `tile` into the stage (cp.async, committed)
-template <typename R, int NC>
-__device__ __forceinline__ void rxi_load(const SolveGeom<R> &g, const typename cplx_t<R>::type *__restrict__ X, int RB,
-                                         const RxSmem<R> &s, int tile) {
-  typedef typename cplx_t<R>::type C;
-  const size_t rowc = (size_t)g.Hp * NC;
-  const int nrows = g.P[1] * g.P[2];
-  const int row0 = tile * RB;
-  const int nr = min(RB, nrows - row0);
-  const size_t nch = (size_t)nr * rowc * sizeof(C) / 16;
-  const char *src = reinterpret_cast<const char *>(X + (size_t)row0 * rowc);
-  for (size_t c = threadIdx.x; c < nch; c += blockDim.x)
-    cp_async16(reinterpret_cast<char *>(s.stage) + 16 * c, src + 16 * c);
-  cp_async_commit();
+// spectral vector v of a row: the values of its (one or two) kx
+__device__ __forceinline__ void spec_row(const float2 *row, size_t v, float2 *o) {
+  const float4 q = __ldg(reinterpret_cast<const float4 *>(row) + v);
+  o[0] = make_float2(q.x, q.z);
+  o[1] = make_float2(q.y, q.w);
 }
+__device__ __forceinline__ void spec_row(const double2 *row, size_t v, double2 *o) { o[0] = __ldg(row + v); }
 
-// x inverse of a staged tile (the caller waited for its copies and synchronised);
-// `prefetch` runs once the stage has been read.  Ends with a barrier.
-template <typename R, int NC, typename Prefetch>
-__device__ __forceinline__ void rxi_tile(const SolveGeom<R> &g, R *__restrict__ outp, int RB, int cs,
-                                         const FastDiv &dLG, const RxSmem<R> &s, int tile, Prefetch prefetch) {
+// one tile of the x inverse pass (ends with a barrier)
+template <typename T, int NC, typename PL>
+__device__ __forceinline__ void rxi_tile(const SolveGeom<typename LineT<T>::R> &g,
+                                         const typename cplx_t<typename LineT<T>::R>::type *__restrict__ X,
+                                         typename LineT<T>::R *__restrict__ outp, int RB, int cs, const FastDiv &dLG,
+                                         const XSmem &s, int tile) {
+  typedef typename LineT<T>::R R;
   typedef typename cplx_t<R>::type C;
-  constexpr int G = RVec<R>::G;
-  const RegPlan &pl = g.rx;
+  constexpr int G = LineT<T>::G;
+  constexpr int XG = sizeof(R) == 4 ? 2 : 1;
+  const LinePlan &pl = g.lx;
   const bool blue = pl.bl != 0;
-  const int N = blue ? pl.bn : pl.n, L = NC * RB, LG = L / G;
-  const size_t rowc = (size_t)g.Hp * NC;
-  const int nrows = g.P[1] * g.P[2];
-  const C *Sc = reinterpret_cast<const C *>(s.stage);
-  C *Bc = reinterpret_cast<C *>(s.buf);
-  const int row0 = tile * RB;
-  for (int t = threadIdx.x; t < RB * N; t += blockDim.x) {
-    const int rr = t / N, m = t - rr * N;
-    const C w = cconj(s.ext[m]);
-    const bool ok = row0 + rr < nrows;
-    const int pm = s.xpos[m];
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-      C z = mk(R(0), R(0));
-      if (ok) {
-        C xm = Sc[rr * rowc + (size_t)m * NC + c];
-        C xn = Sc[rr * rowc + (size_t)(N - m) * NC + c];
-        if (m == 0) {
-          xm.y = R(0);
-          xn.y = R(0);
-        }  // DC and Nyquist are real
-        const C a = cadd(xm, cconj(xn));
-        const C b = csub(xm, cconj(xn));
-        const C wb = cmul(w, b);
-        z = mk(a.x - wb.y, a.y + wb.x);  // a + i W^{-m} b
-      }
-      Bc[pm * L + rr * NC + c] = z;
-    }
-  }
-  __syncthreads();
-  prefetch();
-  PhaseGlobal gl;
-  gl.in = nullptr;
-  gl.out = nullptr;
-  gl.rs_in = gl.rs_out = 0;
-  gl.rows_in = gl.rows_out = N;
-  const int P0 = g.P[0];
-  const int nout = (P0 + 1) / 2;
-  if (blue) bfft<R, true>(pl, s.buf, LG, dLG, s.tw, s.chirp, s.bpos, false, false, gl, N, nout);
-  else rfft_inv<R>(pl, s.buf, LG, dLG, s.tw, false, false, gl);
-  for (int t = threadIdx.x; t < RB * nout; t += blockDim.x) {
-    const int rr = t / nout, m = t - rr * nout;
+  const int N = g.N2, LG = NC * RB / G, P0 = g.P[0];
+  const RtPlan rp{pl, LG, dLG};
+  const int *xpos = line_smem_at<int>(s.xpos);
+  const C *ext = line_smem_at<C>(s.ext);
+  const int nrows = g.P[1] * g.P[2], row0 = tile * RB;
+  long long *srow = line_smem_at<long long>(s.srow);
+  for (int rr = threadIdx.x; rr < RB; rr += blockDim.x) {
     const int row = row0 + rr;
-    if (row >= nrows) continue;
+    srow[rr] = spec_row0<R, NC>(g, row < nrows ? row : row0);
     const int y = row % g.P[1], z = row / g.P[1];
-    R *dst = outp + (((size_t)(z + g.off[2]) * g.ext[1] + (y + g.off[1])) * g.ext[0] + g.off[0]) * cs;
-    const int x0 = 2 * m, x1 = 2 * m + 1;
+    line_smem_at<long long>(s.rows)[rr] = row < nrows ? (long long)((((size_t)(z + g.off[2]) * g.ext[1] + (y + g.off[1])) * g.ext[0] + g.off[0]) * cs)
+                             : -1;
+  }
+  // the twist: Z[k] and Z[N-k] from X[k] and X[N-k]; k <= N/2 from this side, k > N/2 from
+  // its mirror
+  const int nh = N / 2 / XG + 1, nv = nh * NC;
+  constexpr int BV = spec_block<R>() * NC / XG;
+  const int nrg = PL::RT ? RB / G : x_groups<PL, NC>(), nrs = __ffs(nrg) - 1, nb = (nv + BV - 1) / BV;
+  const long long kbs = spec_kb<R, NC>(g);
+  __syncthreads();
+  {
+    for (int t = threadIdx.x; t < nb * nrg * BV; t += blockDim.x) {
+      const int w0 = t / BV, kb = w0 >> nrs, rho = w0 - (kb << nrs);
+      const int v = kb * BV + (t - w0 * BV);
+      if (v >= nv) continue;
+      typename LineT<T>::V *b = line_smem_at<typename LineT<T>::V>(s.tabs.buf) + rho * NC;
+      const int kv = v / NC, c = v - kv * NC;
+      // vector w of the row at base r
+      auto at = [&](long long r, int w) { return (size_t)(r + (w / BV) * kbs + w % BV); };
+      C xk[G][XG], xn[G][XG];
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-      const C v = Bc[m * L + rr * NC + c];
-      dst[(size_t)x0 * cs + c] = v.x;
-      if (x1 < P0) dst[(size_t)x1 * cs + c] = v.y;
+      for (int q = 0; q < G; q++) {
+        const long long r = srow[rho * G + q];
+        spec_row(X, at(r, v), xk[q]);
+        if constexpr (XG == 2) {
+          // X[N - 2 kv] is the even, X[N - 2 kv - 1] the odd value of a pair when N is even,
+          // both lie in one pair when it is odd
+          C m0[XG], m1[XG];
+          const int n0 = N - 2 * kv, n1 = max(n0 - 1, 0);
+          spec_row(X, at(r, (n0 >> 1) * NC + c), m0);
+          spec_row(X, at(r, (n1 >> 1) * NC + c), m1);
+          xn[q][0] = (n0 & 1) ? m0[1] : m0[0];
+          xn[q][1] = (n1 & 1) ? m1[1] : m1[0];
+        } else {
+          spec_row(X, at(r, (N - kv) * NC + c), xn[q]);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < XG; h++) {
+        const int k = kv * XG + h;
+        if (2 * k > N) continue;
+        LV<T> a, m;
+        if constexpr (G == 2) {
+          a = {make_float2(xk[0][h].x, xk[1][h].x), make_float2(xk[0][h].y, xk[1][h].y)};
+          m = {make_float2(xn[0][h].x, xn[1][h].x), make_float2(xn[0][h].y, xn[1][h].y)};
+        } else {
+          a = {xk[0][h].x, xk[0][h].y};
+          m = {xn[0][h].x, xn[0][h].y};
+        }
+        if (k == 0) a.im = m.im = pset(T(), R(0));  // DC and Nyquist are real
+        const LV<T> sum = {padd(a.re, m.re), psub(a.im, m.im)}, dif = {psub(a.re, m.re), padd(a.im, m.im)};
+        const C w = ext[k];
+        const LV<T> t = lmulc<T>(dif, pset(T(), w.x), pset(T(), w.y));  // W^-k (X[k] - conj X[N-k])
+        b[xpos[k] * LG + c] = vput(ladd_i(sum, t));
+        if (k > 0 && 2 * k < N) {
+          const LV<T> z = lsub_i(sum, t);
+          b[xpos[N - k] * LG + c] = vput(LV<T>{z.re, pneg(z.im)});
+        }
+      }
     }
   }
   __syncthreads();
-}
-
-template <typename R, int NC>
-__global__ void __launch_bounds__(RL_THREADS, RMinBlocks<R>::v) k_rxinv(SolveGeom<R> g,
-                                                         const typename cplx_t<R>::type *__restrict__ X,
-                                                         R *__restrict__ outp, int RB, int cs, FastDiv dLG) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const RxSmem<R> s = rx_setup<R, NC>(g, RB, true, smem_raw);
-  const int nrows = g.P[1] * g.P[2];
-  const int ntiles = (nrows + RB - 1) / RB;
-  int tile = blockIdx.x;
-  if (tile < ntiles) rxi_load<R, NC>(g, X, RB, s, tile);
-  for (; tile < ntiles; tile += gridDim.x) {
-    cp_async_wait_all();
+  XRowIo<T, NC> io;
+  io.out = outp;
+  io.rows = s.rows;
+  io.P0 = P0;
+  io.cs = cs;
+  io.rows_in = N;
+  io.rows_out = (P0 + 1) / 2;
+  if constexpr (!PL::RT) {
+    if constexpr (PL::NP > 2) x_phase_ct<T, XRowIo<T, NC>, PL, true, 2>(s.tabs, io);
+    if constexpr (PL::NP > 1) x_phase_ct<T, XRowIo<T, NC>, PL, true, 1>(s.tabs, io);
+    x_phase_ct<T, XRowIo<T, NC>, PL, true, 0>(s.tabs, io);
+  } else {
+  if (blue) {
+    lchirp_in<T>(s.tabs.buf, pl.n, LG, dLG, s.chirp, N, true, false, io);
     __syncthreads();
-    const int next = tile + gridDim.x;
-    rxi_tile<R, NC>(g, outp, RB, cs, dLG, s, tile, [&]() {
-      if (next < ntiles) rxi_load<R, NC>(g, X, RB, s, next);
-    });
+    for (int p = 0; p < pl.np; p++) {
+      lphase_any<false, false, T>(rp, p, s.tabs, io, false, false, false);
+      __syncthreads();
+    }
+    lchirp_mul<T>(s.tabs.buf, pl.n, LG, dLG, line_smem_at<C>(s.bpos));
+    __syncthreads();
   }
-  cp_async_wait_all();
+  for (int p = pl.np - 1; p >= 0; p--) {
+    lphase_any<true, false, T>(rp, p, s.tabs, io, !blue, false, false);
+    __syncthreads();
+  }
+  if (blue) {
+    lchirp_out<T>(s.tabs.buf, pl.n, LG, dLG, s.chirp, io.rows_out, true, true, io);
+    __syncthreads();
+  }
+  }
 }
 
-template <typename R, int NC>
-__global__ void __launch_bounds__(RL_THREADS, RMinBlocks<R>::v) k_rxinv_batch(BatchWork bw, BatchIo io) {
+template <typename T, int NC, typename PL = RtPlan>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS)
+    k_rxinv(SolveGeom<typename LineT<T>::R> g, const typename cplx_t<typename LineT<T>::R>::type *__restrict__ X,
+            typename LineT<T>::R *__restrict__ outp, int RB, int cs, FastDiv dLG) {
+  const XSmem s = x_setup<T, NC>(g, RB, true);
+  __syncthreads();
+  const int ntiles = (g.P[1] * g.P[2] + RB - 1) / RB;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) rxi_tile<T, NC, PL>(g, X, outp, RB, cs, dLG, s, tile);
+}
+
+template <typename T, int NC>
+__global__ void __launch_bounds__(LINE_THREADS_MAX, LINE_CTAS) k_rxinv_batch(BatchWork bw, BatchIo bio) {
+  typedef typename LineT<T>::R R;
   typedef typename cplx_t<R>::type C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ PassDesc<R> sd;
-  RxSmem<R> s;
-  int cur = -1, i0, i1, staged = -1;
+  XSmem s;
+  int cur = -1, i0, i1;
   while (batch_next(bw, i0, i1)) {
     for (int it = i0; it < i1; it++) {
-      if (cur >= 0 && (it < sd.first || it >= sd.first + sd.ntiles)) {
-        cp_async_wait_all();
-        staged = -1;
-      }
       if (batch_patch<R>(bw, it, sd, cur)) {
-        s = rx_setup<R, NC>(sd.g, sd.RB, true, smem_raw);
+        s = x_setup<T, NC>(sd.g, sd.RB, true);
         __syncthreads();
       }
-      const C *X = reinterpret_cast<const C *>(sd.in);
-      if (staged != it) rxi_load<R, NC>(sd.g, X, sd.RB, s, it - sd.first);
-      cp_async_wait_all();
-      __syncthreads();
-      const int next = it + 1;
-      const bool pre = next < i1 && next < sd.first + sd.ntiles;
-      rxi_tile<R, NC>(sd.g, (R *)io.p[cur], sd.RB, sd.cs, sd.dLG, s, it - sd.first, [&]() {
-        if (pre) rxi_load<R, NC>(sd.g, X, sd.RB, s, next - sd.first);
-      });
-      staged = pre ? next : -1;
+      rxi_tile<T, NC, RtPlan>(sd.g, reinterpret_cast<const C *>(sd.in), (R *)bio.p[sd.patch], sd.RB, sd.cs, sd.dLG, s,
+                      it - sd.first);
     }
   }
-  cp_async_wait_all();
+}
+
+// Vector v of a spectral row: two neighbouring kx of one component in FP32, as
+// (re, re, im, im); one complex value in FP64.
+template <typename R>
+__device__ __forceinline__ void spec_put(typename cplx_t<R>::type *row, size_t v, typename cplx_t<R>::type a,
+                                         typename cplx_t<R>::type b) {
+  if constexpr (sizeof(R) == 4) reinterpret_cast<float4 *>(row)[v] = make_float4(a.x, b.x, a.y, b.y);
+  else row[v] = a;
+}
+// component c at kx index m of a spectral row
+template <typename R, int NC>
+__device__ __forceinline__ typename cplx_t<R>::type spec_get(const typename cplx_t<R>::type *row, int m, int c) {
+  if constexpr (sizeof(R) == 4) {
+    const float *p = reinterpret_cast<const float *>(row) + 4 * ((m >> 1) * NC + c) + (m & 1);
+    return make_float2(p[0], p[2]);
+  } else {
+    return row[(size_t)m * NC + c];
+  }
 }
 
 // ---------------------------------------------------------------- x forward (R2C)
@@ -1137,7 +1365,6 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xfwd(SolveGeom<R> g, const 
     __syncthreads();
     const int row0 = tile * RB;
     // pack the staged reals into complex lines
-    C *Ac = reinterpret_cast<C *>(A);
     for (int t = threadIdx.x; t < RB * N; t += blockDim.x) {
       const int rr = t / N, m = t - rr * N;
       const R *xr = Sr + (size_t)rr * P0 * NC;
@@ -1146,38 +1373,43 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xfwd(SolveGeom<R> g, const 
       for (int c = 0; c < NC; c++) {
         const R a = (x0 < P0 && row0 + rr < nrows) ? xr[x0 * NC + c] : R(0);
         const R b = (x1 < P0 && row0 + rr < nrows) ? xr[x1 * NC + c] : R(0);
-        Ac[m * L + rr * NC + c] = mk(a, b);
+        line_set(A, m * L + rr * NC + c, mk(a, b));
       }
     }
     __syncthreads();
     const int next = tile + gridDim.x;
     if (next < ntiles) load(next);
     V *res = vfft_chain<false, R>(A, A, B, LG, sd, tw, lm, NoHook());
-    const C *Z = reinterpret_cast<const C *>(res);
     const C *W = tw + sd.extoff;  // exp(-2 pi i k / Mx), k < H
-    for (int t = threadIdx.x; t < RB * g.Hp; t += blockDim.x) {
-      const int rr = t / g.Hp, k = t - rr * g.Hp;
+    constexpr int XG = sizeof(R) == 4 ? 2 : 1;
+    const int nkv = g.Hp / XG;
+    for (int t = threadIdx.x; t < RB * nkv; t += blockDim.x) {
+      const int rr = t / nkv, kv = t - rr * nkv;
       const int row = row0 + rr;
       if (row >= nrows) continue;
-      C o[NC];
-      if (k < g.H) {
-        const int kk = (k == N) ? 0 : k;
-        const int km = (k == 0 || k == N) ? 0 : N - k;
-        const C w = W[k];
+      C o[XG][NC];
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-          const C zk = Z[kk * L + rr * NC + c];
-          const C zn = cconj(Z[km * L + rr * NC + c]);
-          const C a = cadd(zk, zn), bb = csub(zk, zn);
-          const C wb = cmul(w, bb);
-          o[c] = mk(R(0.5) * (a.x + wb.y), R(0.5) * (a.y - wb.x));  // (a - i W^k b) / 2
+      for (int h = 0; h < XG; h++) {
+        const int k = kv * XG + h;
+        if (k < g.H) {
+          const int kk = (k == N) ? 0 : k;
+          const int km = (k == 0 || k == N) ? 0 : N - k;
+          const C w = W[k];
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            const C zk = line_at(res, kk * L + rr * NC + c);
+            const C zn = cconj(line_at(res, km * L + rr * NC + c));
+            const C a = cadd(zk, zn), bb = csub(zk, zn);
+            const C wb = cmul(w, bb);
+            o[h][c] = mk(R(0.5) * (a.x + wb.y), R(0.5) * (a.y - wb.x));  // (a - i W^k b) / 2
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < NC; c++) o[h][c] = mk(R(0), R(0));
         }
-      } else {
-#pragma unroll
-        for (int c = 0; c < NC; c++) o[c] = mk(R(0), R(0));
       }
 #pragma unroll
-      for (int c = 0; c < NC; c++) X[((size_t)row * g.Hp + k) * NC + c] = o[c];
+      for (int c = 0; c < NC; c++) spec_put<R>(X, spec_vec<R, NC>(g, row, kv * NC + c), o[0][c], o[XG - 1][c]);
     }
     __syncthreads();
   }
@@ -1210,10 +1442,12 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xinv(SolveGeom<R> g, const 
   auto load = [&](int tile) {
     const int row0 = tile * RB;
     const int nr = min(RB, nrows - row0);
-    const size_t nch = (size_t)nr * rowc * sizeof(C) / 16;
-    const char *src = reinterpret_cast<const char *>(X + (size_t)row0 * rowc);
-    for (size_t c = threadIdx.x; c < nch; c += blockDim.x)
-      cp_async16(reinterpret_cast<char *>(Sc) + 16 * c, src + 16 * c);
+    const int rch = (int)(rowc * sizeof(C) / 16);  // 16-byte vectors of a row
+    for (int c = threadIdx.x; c < nr * rch; c += blockDim.x) {
+      const int rr = c / rch, v = c - rr * rch;
+      cp_async16(reinterpret_cast<char *>(Sc) + 16 * (size_t)c,
+                 reinterpret_cast<const char *>(X) + 16 * spec_vec<R, NC>(g, row0 + rr, v));
+    }
     cp_async_commit();
   };
   int tile = blockIdx.x;
@@ -1223,7 +1457,6 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xinv(SolveGeom<R> g, const 
     __syncthreads();
     const int row0 = tile * RB;
     const C *W = tw + sd.extoff;
-    C *Ac = reinterpret_cast<C *>(A);
     for (int t = threadIdx.x; t < RB * N; t += blockDim.x) {
       const int rr = t / N, m = t - rr * N;
       const C w = cconj(W[m]);
@@ -1232,8 +1465,8 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xinv(SolveGeom<R> g, const 
       for (int c = 0; c < NC; c++) {
         C z = mk(R(0), R(0));
         if (ok) {
-          C xm = Sc[rr * rowc + (size_t)m * NC + c];
-          C xn = Sc[rr * rowc + (size_t)(N - m) * NC + c];
+          C xm = spec_get<R, NC>(Sc + rr * rowc, m, c);
+          C xn = spec_get<R, NC>(Sc + rr * rowc, N - m, c);
           if (m == 0) {
             xm.y = R(0);
             xn.y = R(0);
@@ -1243,14 +1476,13 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xinv(SolveGeom<R> g, const 
           const C wb = cmul(w, b);
           z = mk(a.x - wb.y, a.y + wb.x);  // a + i W^{-m} b
         }
-        Ac[m * L + rr * NC + c] = z;
+        line_set(A, m * L + rr * NC + c, z);
       }
     }
     __syncthreads();
     const int next = tile + gridDim.x;
     if (next < ntiles) load(next);
     V *res = vfft_chain<true, R>(A, A, B, LG, sd, tw, lm, NoHook());
-    const C *Rc = reinterpret_cast<const C *>(res);
     for (int t = threadIdx.x; t < RB * N; t += blockDim.x) {
       const int rr = t / N, m = t - rr * N;
       const int row = row0 + rr;
@@ -1260,7 +1492,7 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_xinv(SolveGeom<R> g, const 
       const int x0 = 2 * m, x1 = 2 * m + 1;
 #pragma unroll
       for (int c = 0; c < NC; c++) {
-        const C v = Rc[m * L + rr * NC + c];
+        const C v = line_at(res, m * L + rr * NC + c);
         if (x0 < g.P[0]) dst[(size_t)x0 * cs + c] = v.x;
         if (x1 < g.P[0]) dst[(size_t)x1 * cs + c] = v.y;
       }
