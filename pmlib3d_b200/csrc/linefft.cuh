@@ -59,7 +59,7 @@ __host__ __device__ constexpr bool reg_radix(int r) {
   return r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 7 || r == 8 || r == 9 || r == 10 || r == 11 ||
          r == 12 || r == 13 || r == 16 || r == 17;
 }
-// further composite radices: FP32 schedules, and the convolutions of Bluestein lines
+// further composite radices, FP32 schedules only
 __host__ __device__ constexpr bool reg_radix_wide(int r) { return r == 18 || r == 20 || r == 22 || r == 24; }
 
 constexpr int LP_MAX = 3;
@@ -530,7 +530,7 @@ __device__ __forceinline__ void lphase(const PL &pl, int p, const LineTabs &tb, 
   }
 }
 
-// WIDE: the radices above 17 too (y and z passes)
+// WIDE: the radices above 17 too (FP32 schedules of the y and z passes)
 template <bool INV, bool WIDE, typename T, typename IO>
 __device__ __forceinline__ void lphase_any(const RtPlan &rp, int p, const LineTabs &tb, const IO &io, bool glob,
                                            bool gin, bool gout) {
@@ -540,7 +540,7 @@ __device__ __forceinline__ void lphase_any(const RtPlan &rp, int p, const LineTa
     PMGPU_LP(1) PMGPU_LP(2) PMGPU_LP(3) PMGPU_LP(4) PMGPU_LP(5) PMGPU_LP(6) PMGPU_LP(7) PMGPU_LP(8) PMGPU_LP(9)
     PMGPU_LP(10) PMGPU_LP(11) PMGPU_LP(12) PMGPU_LP(13) PMGPU_LP(16) PMGPU_LP(17)
     default:
-      if constexpr (WIDE) {
+      if constexpr (WIDE && sizeof(typename LineT<T>::R) == 4) {
         switch (pl.rad[p]) {
           PMGPU_LP(18) PMGPU_LP(20) PMGPU_LP(22) PMGPU_LP(24)
           default: break;  // plans only hold register radices
@@ -566,18 +566,30 @@ __device__ __forceinline__ void lchirp_in(unsigned boff, int n, int LG, const Fa
   typename LineT<T>::V *const buf = line_smem_at<typename LineT<T>::V>(boff);
   const typename cplx_t<typename LineT<T>::R>::type *chirp =
       line_smem_at<typename cplx_t<typename LineT<T>::R>::type>(coff);
+  // four values a thread at a time, so that their loads are in flight together
+  constexpr int U = 4;
   const unsigned total = (unsigned)n * (unsigned)LG;
-  for (unsigned t = threadIdx.x; t < total; t += blockDim.x) {
-    const unsigned j = fdiv(t, dLG);
-    const int g = (int)(t - j * (unsigned)LG);
-    LV<T> v = lzero<T>();
-    if ((int)j < nin) {
-      v = gsrc ? io.load((int)j, g) : vget(buf[t]);
-      if (conj_in) v.im = pneg(v.im);
-      const auto c = chirp[j];
-      v = lmul<T>(v, pset(T(), c.x), pset(T(), c.y));
+  for (unsigned t0 = threadIdx.x; t0 < total; t0 += U * blockDim.x) {
+    LV<T> v[U];
+    unsigned j[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const unsigned t = t0 + u * blockDim.x;
+      j[u] = fdiv(t, dLG);
+      v[u] = lzero<T>();
+      if (t < total && (int)j[u] < nin) v[u] = gsrc ? io.load((int)j[u], (int)(t - j[u] * (unsigned)LG)) : vget(buf[t]);
     }
-    buf[t] = vput(v);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const unsigned t = t0 + u * blockDim.x;
+      if (t >= total) break;
+      if ((int)j[u] < nin) {
+        if (conj_in) v[u].im = pneg(v[u].im);
+        const auto c = chirp[j[u]];
+        v[u] = lmul<T>(v[u], pset(T(), c.x), pset(T(), c.y));
+      }
+      buf[t] = vput(v[u]);
+    }
   }
 }
 template <typename T>

@@ -1,6 +1,6 @@
 // passes_ct_x_f32.cu -- compile-time x passes (float fields of 3 components), and the choice among
 // the compile-time line passes.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

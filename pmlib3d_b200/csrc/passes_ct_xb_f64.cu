@@ -1,5 +1,5 @@
 // passes_ct_xb_f64.cu -- batched compile-time x passes (double fields of 3 components).
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

@@ -1,5 +1,5 @@
 // passes_ct_z_f64.cu -- compile-time line passes (z, double fields of 3 components).
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

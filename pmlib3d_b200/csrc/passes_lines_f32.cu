@@ -1,5 +1,5 @@
 // passes_lines_f32.cu -- the register-engine line pass kernel for float fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

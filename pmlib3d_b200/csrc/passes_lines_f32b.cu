@@ -1,5 +1,5 @@
 // passes_lines_f32b.cu -- the register-engine batched line pass kernel for float fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

@@ -1,5 +1,5 @@
 // passes_lines_f64.cu -- the register-engine line pass kernel for double fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

@@ -1,5 +1,5 @@
 // passes_lines_f64b.cu -- the register-engine batched line pass kernel for double fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

@@ -1,5 +1,5 @@
 // passes_x_f32_1.cu -- x passes of float fields of 1 component.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

@@ -1,5 +1,5 @@
 // passes_x_f32_3.cu -- x passes of float fields of 3 components (two rows a vector).
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

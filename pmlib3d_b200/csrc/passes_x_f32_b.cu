@@ -1,5 +1,5 @@
 // passes_x_f32_b.cu -- batched x passes of float fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

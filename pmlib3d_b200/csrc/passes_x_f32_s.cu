@@ -1,5 +1,5 @@
 // passes_x_f32_s.cu -- x passes of float fields whose rows are too long for two rows a vector.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

@@ -1,5 +1,5 @@
 // passes_x_f64.cu -- x passes of double fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

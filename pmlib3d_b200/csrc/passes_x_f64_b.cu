@@ -1,5 +1,5 @@
 // passes_x_f64_b.cu -- batched x passes of double fields.
-#include "passes.cuh"
+#include "kernels.cuh"
 
 namespace pmgpu {
 

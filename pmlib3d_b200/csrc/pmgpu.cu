@@ -451,7 +451,7 @@ static std::vector<RadixSeq> line_candidates(int n, int split, int axis, int rsi
     }
     out.push_back(q);
   };
-  auto ok = [&](int r) { return reg_radix(r) || ((rsize == 4 || one_group) && axis != 0 && reg_radix_wide(r)); };
+  auto ok = [&](int r) { return reg_radix(r) || (rsize == 4 && axis != 0 && !one_group && reg_radix_wide(r)); };
   for (int a : S) {
     if (n % a || !ok(a)) continue;
     const int n1 = n / a;
