@@ -944,13 +944,13 @@ __global__ void k_m2p(PartGeom<R> g, const R *__restrict__ pos, const int *__res
 // conflicts only where the warp spans two bin rows.  The particles of one bin row
 // are one contiguous range of the sorted order.  Same index and weight rules as
 // k_m2p; particles with the sentinel key (outside every bin) are left to k_m2p.
-constexpr int M2P_TX = 32, M2P_TY = 8, M2P_TZ = 8, M2P_THREADS = 256;
+constexpr int M2P_TX = 32, M2P_THREADS = 256;
 
-template <typename R, int W> __host__ __device__ constexpr size_t m2p_tile_smem() {
-  return (size_t)(M2P_TX + W - 1) * (M2P_TY + W - 1) * (M2P_TZ + W - 1) * 3 * sizeof(R);
+template <typename R, int W, int TY, int TZ> __host__ __device__ constexpr size_t m2p_tile_smem() {
+  return (size_t)(M2P_TX + W - 1) * (TY + W - 1) * (TZ + W - 1) * 3 * sizeof(R);
 }
 
-template <typename R, int W>
+template <typename R, int W, int M2P_TY, int M2P_TZ>
 __global__ void __launch_bounds__(M2P_THREADS) k_m2p_tile(PartGeom<R> g, const R *__restrict__ pos,
                                                           const unsigned *__restrict__ start,
                                                           const int *__restrict__ perm, const R *__restrict__ f,

@@ -869,22 +869,36 @@ static int run_m2p(const pmgpu_topo *t, int order, const R *pos, const int *ord,
 // M2P of one field for particles already sorted by bin (perm, start of the
 // deposition with the same positions): tiles of bins through shared memory, then
 // the particles outside every bin (the tail of perm) one by one.
-template <typename R, int W>
-static int run_m2p_sorted_w(const pmgpu_topo *t, const R *pos, const unsigned *start, const int *perm, int n,
-                            const R *f, R *o, cudaStream_t st, const char *caller) {
-  PartGeom<R> g = part_geom<R>(t, W);
-  const size_t sm = m2p_tile_smem<R, W>();
-  if (smem_attr((const void *)k_m2p_tile<R, W>, sm, caller)) return -1;
+template <typename R, int W, int TY, int TZ>
+static int launch_m2p_tile(const PartGeom<R> &g, const R *pos, const unsigned *start, const int *perm, const R *f, R *o,
+                           cudaStream_t st, const char *caller) {
+  const size_t sm = m2p_tile_smem<R, W, TY, TZ>();
+  if (smem_attr((const void *)k_m2p_tile<R, W, TY, TZ>, sm, caller)) return -1;
   // tile edges on the bin of interior cell 1 (bin 1 - blo) along each axis
   auto org = [&](int e, int T) {
     const int r = (1 - g.blo[e]) % T;
     return r ? r - T : 0;
   };
-  const int3 o3 = make_int3(org(0, M2P_TX), org(1, M2P_TY), org(2, M2P_TZ));
-  dim3 grid((g.nb[0] - o3.x + M2P_TX - 1) / M2P_TX, (g.nb[1] - o3.y + M2P_TY - 1) / M2P_TY,
-            (g.nb[2] - o3.z + M2P_TZ - 1) / M2P_TZ);
-  { KTimer kt_(KC_M2P, st); k_m2p_tile<R, W><<<grid, M2P_THREADS, sm, st>>>(g, pos, start, perm, f, o, o3); }
+  const int3 o3 = make_int3(org(0, M2P_TX), org(1, TY), org(2, TZ));
+  dim3 grid((g.nb[0] - o3.x + M2P_TX - 1) / M2P_TX, (g.nb[1] - o3.y + TY - 1) / TY, (g.nb[2] - o3.z + TZ - 1) / TZ);
+  { KTimer kt_(KC_M2P, st); k_m2p_tile<R, W, TY, TZ><<<grid, M2P_THREADS, sm, st>>>(g, pos, start, perm, f, o, o3); }
   PM_LAUNCHED();
+  CKL(caller);
+  return 0;
+}
+template <typename R, int W>
+static int run_m2p_sorted_w(const pmgpu_topo *t, const R *pos, const unsigned *start, const int *perm, int n,
+                            const R *f, R *o, cudaStream_t st, const char *caller) {
+  PartGeom<R> g = part_geom<R>(t, W);
+  // 8 x 8 bin rows a tile, or 4 x 4 where few tiles would leave SMs idle or where a tile's
+  // cells (FP64, M6*: 75 to 150 KB) would leave room for one or two CTAs.  Microseconds, 8 x 8
+  // against 4 x 4: 64^3 FP32 56 / 37, 256^3 FP32 792 / 904, 256^3 FP64 1468 / 1414,
+  // 104 x 104 x 136 FP64 (two fields) 353 / 320, 150 x 121 x 95 M6* FP32 251 / 230
+  const long long tiles = (long long)((g.nb[0] + 31) / 32) * ((g.nb[1] + 7) / 8) * ((g.nb[2] + 7) / 8);
+  const bool small = sizeof(R) == 8 || W == 6 || tiles < 4 * (long long)num_sms();
+  if (small ? launch_m2p_tile<R, W, 4, 4>(g, pos, start, perm, f, o, st, caller)
+            : launch_m2p_tile<R, W, 8, 8>(g, pos, start, perm, f, o, st, caller))
+    return -1;
   const int nblk = std::min((n + 127) / 128, 148 * 8);
   { KTimer kt_(KC_M2P, st);
     k_m2p<R, W><<<nblk, 128, 0, st>>>(g, pos, perm, n, start + g.nbins, nullptr, nullptr, f, nullptr, nullptr, o); }
