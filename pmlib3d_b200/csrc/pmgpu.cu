@@ -795,7 +795,7 @@ static int run_bin_sort(const pmgpu_topo *t, int order, const R *pos, int n, Par
 // One deposition launch: a persistent grid of one CTA per SM (fewer for small
 // grids), each taking an equal share of the cells.
 template <typename R, int W, int NV>
-static int launch_deposit(const PartGeom<R> &g, const R *pos, const R *vp, int vstride, PartScratchRefs s,
+static int launch_deposit(const PartGeom<R> &g, const R *pos, const R *vp, int vstride, int n, PartScratchRefs s,
                           const int *perm, R *mp, int mstride, int clear_mode, cudaStream_t st, const char *caller) {
   const size_t smem = deposit_smem<R, W>();
   const int threads = dep_threads<R, W>();
@@ -807,8 +807,22 @@ static int launch_deposit(const PartGeom<R> &g, const R *pos, const R *vp, int v
   const long long units = ntx * nty * g.ext[2];
   const int grid = (int)std::max<long long>(1, std::min<long long>(num_sms(), units));
   KTimer kt_(KC_DEPOSIT, st);
+  // fewer particles than half the cells sit unevenly (vortex cores): shares by their
+  // particles.  The counts' buffer is free after the scan: unit costs, then the shares.
+  int *shares = nullptr;
+  const long long cells = (long long)g.nint[0] * g.nint[1] * g.nint[2];
+  if (2 * (long long)n < cells && units >= DEP_SHARE_UNITS && units + grid + 1 <= (long long)g.nbins) {
+    unsigned *cost = s.counts->as<unsigned>();
+    shares = reinterpret_cast<int *>(cost + units);
+    const int nblk = (int)std::min<long long>((units + 7) / 8, 148 * 8);
+    k_dep_cost<<<nblk, 256, 0, st>>>(s.start->as<unsigned>(), g.ext[0], g.ext[1], g.ext[2], g.nb[0], g.nb[1], g.nb[2],
+                                     tw, th, W, (int)units, cost);
+    PM_LAUNCHED();
+    k_dep_shares<<<1, SCAN_THREADS, 0, st>>>(cost, (int)units, grid, shares);
+    PM_LAUNCHED();
+  }
   k_deposit<R, W, NV><<<grid, threads, smem, st>>>(g, pos, vp, vstride, s.start->as<unsigned>(), perm, mp, mstride,
-                                                    clear_mode, tw, th);
+                                                    clear_mode, tw, th, shares);
   PM_LAUNCHED();
   CKL(caller);
   return 0;
@@ -830,10 +844,10 @@ static int run_p2m(const pmgpu_topo *t, int order, const R *pos, const R *val, i
     const R *vp = val + c0;
     R *mp = mesh + c0;
     int rc = 0;
-    if (W == 4) rc = (nv == 3) ? launch_deposit<R, 4, 3>(g, pos, vp, nvar, s, perm, mp, nvar_mesh, clear_mode, st, caller)
-                               : launch_deposit<R, 4, 1>(g, pos, vp, nvar, s, perm, mp, nvar_mesh, clear_mode, st, caller);
-    else rc = (nv == 3) ? launch_deposit<R, 6, 3>(g, pos, vp, nvar, s, perm, mp, nvar_mesh, clear_mode, st, caller)
-                        : launch_deposit<R, 6, 1>(g, pos, vp, nvar, s, perm, mp, nvar_mesh, clear_mode, st, caller);
+    if (W == 4) rc = (nv == 3) ? launch_deposit<R, 4, 3>(g, pos, vp, nvar, n, s, perm, mp, nvar_mesh, clear_mode, st, caller)
+                               : launch_deposit<R, 4, 1>(g, pos, vp, nvar, n, s, perm, mp, nvar_mesh, clear_mode, st, caller);
+    else rc = (nv == 3) ? launch_deposit<R, 6, 3>(g, pos, vp, nvar, n, s, perm, mp, nvar_mesh, clear_mode, st, caller)
+                        : launch_deposit<R, 6, 1>(g, pos, vp, nvar, n, s, perm, mp, nvar_mesh, clear_mode, st, caller);
     if (rc) return -1;
     c0 += nv;
   }
