@@ -645,7 +645,7 @@ struct pmgpu_plan {
   pmgpu_topo topo;
   pmgpu_params par;
   Geometry g;
-  FftDesc fx, fy, fz;
+  FftDesc fx{}, fy{}, fz{};
   DevBuf twx, twy, twz;
   DevBuf kxt, kyt, kzt;
   DevBuf green;  // view of green_own (shared between plans of the same grid)
@@ -1081,6 +1081,7 @@ static void attach_green(pmgpu_plan *pl, const std::shared_ptr<DevBuf> &sp) {
 }
 
 template <typename R> static int reg_tables(pmgpu_plan *pl, const char *caller, bool tune_ok);
+template <typename R> static int stockham_tables(pmgpu_plan *pl, int nc, const char *caller);
 
 template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller) {
   const Geometry &G = pl->g;
@@ -1141,16 +1142,12 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
   tmp.perm = nullptr;
   tmp.perm_n = 0;
   tmp.gM1 = tmp.gM2 = 0;
-  std::vector<cld> tw;
   // temporaries are stream-ordered on the legacy stream, so a set-up does not wait
   // for (or stall) solves running on other streams
   DevBuf gr, gX, gY, yinv, zinv;
   int rc = -1;
   do {
-    if (!make_fft(G.N2, G.M[0], tmp.fx, tw) || upload_tw<double>(tw, tmp.twx, caller)) break;
-    if (!make_fft(G.M[1], 0, tmp.fy, tw) || upload_tw<double>(tw, tmp.twy, caller)) break;
-    if (!make_fft(G.M[2], 0, tmp.fz, tw) || upload_tw<double>(tw, tmp.twz, caller)) break;
-    if (reg_tables<double>(&tmp, caller, false)) break;
+    if (reg_tables<double>(&tmp, caller, false) || stockham_tables<double>(&tmp, 1, caller)) break;
     SolveGeom<double> gg = solve_geom<double>(&tmp);
     // spectrum rows after the y and z transforms: frequency -> row
     std::vector<int> yi(G.M[1]), zi(G.M[2]);
@@ -1613,16 +1610,31 @@ template <typename R> static int apply_tuning(pmgpu_plan *pl, const char *caller
   return fresh ? reg_tables<R>(pl, caller, true) : 0;
 }
 
+// Tables of the Stockham passes, when a pass of nc components takes them: an axis without a
+// register plan, or whose smallest tile exceeds the shared memory (passes.cuh: line_shape,
+// x_shape)
+template <typename R> static int stockham_tables(pmgpu_plan *pl, int nc, const char *caller) {
+  const Geometry &G = pl->g;
+  auto fits_x = [&](bool inverse) {
+    return x_smem(pl->lx, G.N2, G.H, G.P[0], nc, 1, sizeof(R), false, inverse) <= PASS_SMEM_BUDGET;
+  };
+  if (pl->rx_ok && pl->ry_ok && pl->rz_ok && fits_x(false) && fits_x(true) &&
+      line_smem(pl->ly, nc, 1, sizeof(R)) <= PASS_SMEM_BUDGET && line_smem(pl->lz, nc, 1, sizeof(R)) <= PASS_SMEM_BUDGET)
+    return 0;
+  std::vector<cld> tw;
+  return !make_fft(G.N2, G.M[0], pl->fx, tw) || upload_tw<R>(tw, pl->twx, caller) ||
+                 !make_fft(G.M[1], 0, pl->fy, tw) || upload_tw<R>(tw, pl->twy, caller) ||
+                 !make_fft(G.M[2], 0, pl->fz, tw) || upload_tw<R>(tw, pl->twz, caller)
+             ? -1
+             : 0;
+}
+
 template <typename R> static int plan_tables(pmgpu_plan *pl, const char *caller) {
   typedef typename cplx_t<R>::type C;
-  std::vector<cld> tw;
-  if (!make_fft(pl->g.N2, pl->g.M[0], pl->fx, tw) || upload_tw<R>(tw, pl->twx, caller)) return -1;
-  if (!make_fft(pl->g.M[1], 0, pl->fy, tw) || upload_tw<R>(tw, pl->twy, caller)) return -1;
-  if (!make_fft(pl->g.M[2], 0, pl->fz, tw) || upload_tw<R>(tw, pl->twz, caller)) return -1;
   if (upload_wavenumbers<R>(pl, caller)) return -1;
   pl->gM1 = pl->g.M[1] / 2 + 1;
   pl->gM2 = pl->g.M[2] / 2 + 1;
-  if (reg_tables<R>(pl, caller, true)) return -1;
+  if (reg_tables<R>(pl, caller, true) || stockham_tables<R>(pl, 3, caller)) return -1;
   if (setup_green<R>(pl, caller)) return -1;
   // the work spectra of a three-component solve, so that a plan's first solve (often
   // queued from another thread than the set-up) allocates nothing
