@@ -1000,10 +1000,15 @@ __global__ void k_m2p(PartGeom<R> g, const R *__restrict__ pos, const int *__res
 // conflicts only where the warp spans two bin rows.  The particles of one bin row
 // are one contiguous range of the sorted order.  Same index and weight rules as
 // k_m2p; particles with the sentinel key (outside every bin) are left to k_m2p.
-constexpr int M2P_TX = 32, M2P_THREADS = 256;
+constexpr int M2P_THREADS = 256;
+// bins along x.  29 for W = 4: a staged row is then 32 cells, a multiple of the banks, and the
+// rows of a tile fill whole 128-byte lines.  Microseconds with 32 / 29: 256^3 FP64 1414 / 1403,
+// 104 x 104 x 136 FP64 (two fields) 319 / 311, 192^3 FP32 (two fields) 825 / 798, 256^3 FP32
+// 792 / 790.  M6* takes 32 (150 x 121 x 95: 228; 27, the same row, 235)
+template <int W> __host__ __device__ constexpr int m2p_tx() { return W == 4 ? 29 : 32; }
 
 template <typename R, int W, int TY, int TZ> __host__ __device__ constexpr size_t m2p_tile_smem() {
-  return (size_t)(M2P_TX + W - 1) * (TY + W - 1) * (TZ + W - 1) * 3 * sizeof(R);
+  return (size_t)(m2p_tx<W>() + W - 1) * (TY + W - 1) * (TZ + W - 1) * 3 * sizeof(R);
 }
 
 template <typename R, int W, int M2P_TY, int M2P_TZ>
@@ -1012,6 +1017,7 @@ __global__ void __launch_bounds__(M2P_THREADS) k_m2p_tile(PartGeom<R> g, const R
                                                           const int *__restrict__ perm, const R *__restrict__ f,
                                                           R *__restrict__ o, int3 org) {
   constexpr int off = Stencil<W>::off;
+  constexpr int M2P_TX = m2p_tx<W>();
   constexpr int CX = M2P_TX + W - 1, CY = M2P_TY + W - 1, CZ = M2P_TZ + W - 1, NR = M2P_TY * M2P_TZ;
   constexpr int PLANE = CZ * CY * CX;
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -894,6 +894,7 @@ static int launch_m2p_tile(const PartGeom<R> &g, const R *pos, const unsigned *s
     return r ? r - T : 0;
   };
   const int3 o3 = make_int3(org(0, M2P_TX), org(1, TY), org(2, TZ));
+  constexpr int M2P_TX = m2p_tx<W>();
   dim3 grid((g.nb[0] - o3.x + M2P_TX - 1) / M2P_TX, (g.nb[1] - o3.y + TY - 1) / TY, (g.nb[2] - o3.z + TZ - 1) / TZ);
   { KTimer kt_(KC_M2P, st); k_m2p_tile<R, W, TY, TZ><<<grid, M2P_THREADS, sm, st>>>(g, pos, start, perm, f, o, o3); }
   PM_LAUNCHED();
@@ -908,7 +909,8 @@ static int run_m2p_sorted_w(const pmgpu_topo *t, const R *pos, const unsigned *s
   // cells (FP64, M6*: 75 to 150 KB) would leave room for one or two CTAs.  Microseconds, 8 x 8
   // against 4 x 4: 64^3 FP32 56 / 37, 256^3 FP32 792 / 904, 256^3 FP64 1468 / 1414,
   // 104 x 104 x 136 FP64 (two fields) 353 / 320, 150 x 121 x 95 M6* FP32 251 / 230
-  const long long tiles = (long long)((g.nb[0] + 31) / 32) * ((g.nb[1] + 7) / 8) * ((g.nb[2] + 7) / 8);
+  constexpr int M2P_TX = m2p_tx<W>();
+  const long long tiles = (long long)((g.nb[0] + M2P_TX - 1) / M2P_TX) * ((g.nb[1] + 7) / 8) * ((g.nb[2] + 7) / 8);
   const bool small = sizeof(R) == 8 || W == 6 || tiles < 4 * (long long)num_sms();
   if (small ? launch_m2p_tile<R, W, 4, 4>(g, pos, start, perm, f, o, st, caller)
             : launch_m2p_tile<R, W, 8, 8>(g, pos, start, perm, f, o, st, caller))
