@@ -116,6 +116,9 @@ struct BatchLayout {
 template <typename R, int NC>
 int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y, cudaStream_t st,
            const char *caller, int cs = NC);
+// periodic ghosts of a mesh of nv components
+template <typename R>
+int ghost_fill_all(const pmgpu_topo *topo, R *mesh, int nv, cudaStream_t st, const char *caller);
 // z pass on rows_y spectrum rows: Z_VEL / Z_VORT / Z_VECPOT / Z_REGULARISE / Z_FORWARD
 template <typename R, int NC>
 int zpass(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typename cplx_t<R>::type *out, int mode, int reproj,

@@ -1042,19 +1042,7 @@ static int run_regularise(pmgpu_plan *pl, R *mesh, int nvar, int reg_order, doub
     for (int c = 0; c < nvar; c++)
       if (run_regularise_nc<R, 1>(pl, mesh + c, nvar, reg_order, fw, st, caller)) return -1;
   }
-  const pmgpu_topo *topo = &pl->topo;
-  for (int d = 0; d < 3; d++) {
-    if (topo->bound_cond[2 * d] == 0 || topo->bound_cond[2 * d + 1] == 0) continue;
-    const int ext[3] = {pl->g.ext[0], pl->g.ext[1], pl->g.ext[2]};
-    const int S = topo->nghost[2 * d] + topo->nghost[2 * d + 1];
-    const long long total = (long long)S * ext[(d + 1) % 3] * ext[(d + 2) % 3];
-    const int nblk = (int)std::min<long long>((total + 255) / 256, 148 * 16);
-    { KTimer kt_(KC_GFILL, st); k_ghost_fill<R><<<std::max(nblk, 1), 256, 0, st>>>(mesh, ext[0], ext[1], ext[2], nvar, d, topo->ncell[d],
-                                                        topo->nghost[2 * d], topo->nghost[2 * d + 1]); }
-    PM_LAUNCHED();
-    CKL(caller);
-  }
-  return 0;
+  return ghost_fill_all<R>(&pl->topo, mesh, nvar, st, caller);
 }
 
 // ------------------------------------------------------------------ Green's function
@@ -2812,18 +2800,7 @@ static int run_deriv_vorticity(const pmgpu_topo *t, int fd_order, double visc, c
     PM_LAUNCHED();
     CKL(caller);
   }
-  for (int d = 0; d < 3; d++) {
-    if (t->bound_cond[2 * d] == 0 || t->bound_cond[2 * d + 1] == 0) continue;
-    const int S = t->nghost[2 * d] + t->nghost[2 * d + 1];
-    const long long total = (long long)S * g.ext[(d + 1) % 3] * g.ext[(d + 2) % 3];
-    const int nblk = (int)std::min<long long>((total + 255) / 256, 148 * 16);
-    { KTimer kt_(KC_GFILL, st); k_ghost_fill<R><<<std::max(nblk, 1), 256, 0, st>>>(dvort, g.ext[0], g.ext[1], g.ext[2], 3, d,
-                                                                                    t->ncell[d], t->nghost[2 * d],
-                                                                                    t->nghost[2 * d + 1]); }
-    PM_LAUNCHED();
-    CKL(caller);
-  }
-  return 0;
+  return ghost_fill_all<R>(t, dvort, 3, st, caller);
 }
 
 // Runge-Kutta coefficients of source/particles/pmlib_particles_advance.f:49-88 in the
@@ -3296,19 +3273,7 @@ static int run_penal(pmgpu_plan *pm, pmgpu_plan *pp, const R *solid, const R *sv
   }
   // :345-360 box vorticity added to the main vorticity, then the main ghost map
   if (launch_mesh_map<R>(to_main, pvort, vort, 1, st, caller)) return -1;
-  const pmgpu_topo *t = &pm->topo;
-  for (int d = 0; d < 3; d++) {
-    if (t->bound_cond[2 * d] == 0 || t->bound_cond[2 * d + 1] == 0) continue;
-    const int ext[3] = {to_main.er[0], to_main.er[1], to_main.er[2]};
-    const int S = t->nghost[2 * d] + t->nghost[2 * d + 1];
-    const long long total = (long long)S * ext[(d + 1) % 3] * ext[(d + 2) % 3];
-    const int nblk = (int)std::min<long long>((total + 255) / 256, 148 * 16);
-    { KTimer kt_(KC_GFILL, st);
-      k_ghost_fill<R><<<std::max(nblk, 1), 256, 0, st>>>(vort, ext[0], ext[1], ext[2], 3, d, t->ncell[d],
-                                                         t->nghost[2 * d], t->nghost[2 * d + 1]); }
-    PM_LAUNCHED();
-    CKL(caller);
-  }
+  if (ghost_fill_all<R>(&pm->topo, vort, 3, st, caller)) return -1;
   // :364-419 main solve (vorticity reprojected when asked), free-stream velocity
   if (run_solve<R>(pm, vort, vel, reproject ? vort : nullptr, nullptr, 0, reproject ? 1 : 0, 0, st, caller))
     return -1;

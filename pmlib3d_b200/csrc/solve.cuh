@@ -1550,6 +1550,39 @@ __global__ void k_ghost_fill_batch(const GhostDesc *__restrict__ d, int npatch, 
     int lo = 0, hi = npatch - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
+// All periodic ghosts of a mesh in one launch: every point of a periodic axis's ghost strips
+// copies its image in the interior of all periodic axes, which is what filling the axes in
+// turn leaves there (a point in two strips is written twice, with the same value).
+struct GhostAll {
+  int ext[3], per[3], n[3], ngl[3], ngh[3], nv;
+  long long first[4];  // strip points of axes 0, 1, 2 in one index space
+};
+template <typename R> __global__ void k_ghost_fill_all(GhostAll q, R *__restrict__ mesh) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < q.first[3];
+       t += (long long)gridDim.x * blockDim.x) {
+    const int axis = t >= q.first[2] ? 2 : t >= q.first[1] ? 1 : 0;
+    long long r = t - q.first[axis];
+    int id[3];
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      const int len = e == axis ? q.ngl[e] + q.ngh[e] : q.ext[e];
+      const long long d = r / len;
+      id[e] = (int)(r - d * len);
+      r = d;
+      if (e == axis && id[e] >= q.ngl[e]) id[e] += q.n[e];
+    }
+    size_t di = 0, si = 0;
+#pragma unroll
+    for (int e = 2; e >= 0; e--) {
+      int i = id[e];
+      if (q.per[e]) i += i < q.ngl[e] ? q.n[e] : i >= q.ngl[e] + q.n[e] ? -q.n[e] : 0;
+      di = di * q.ext[e] + id[e];
+      si = si * q.ext[e] + i;
+    }
+    for (int c = 0; c < q.nv; c++) mesh[di * q.nv + c] = mesh[si * q.nv + c];
+  }
+}
+
       if (d[mid].first <= t) lo = mid;
       else hi = mid - 1;
     }
