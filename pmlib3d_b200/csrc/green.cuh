@@ -119,14 +119,18 @@ __device__ __forceinline__ double green_k1(const GreenParams &gp, double r) {
   }
 }
 
-// real kernel on the shifted M0 x M1 x M2 grid, x fastest
-__global__ void k_green_real(GreenParams gp, double *__restrict__ gr) {
-  const size_t total = (size_t)gp.M[0] * gp.M[1] * gp.M[2];
+// real kernel on the shifted grid, x fastest.  It is even in every axis (transform
+// lengths are even): the rows y <= M1 / 2, z <= M2 / 2 are written (even_forward reads the
+// others from their mirror), and a thread writes a point and its mirror in x, an eighth of
+// the evaluations.  full: all rows
+__global__ void k_green_real(GreenParams gp, int full, double *__restrict__ gr) {
+  const int hx = gp.M[0] / 2 + 1, ny = full ? gp.M[1] : gp.M[1] / 2 + 1, nz = full ? gp.M[2] : gp.M[2] / 2 + 1;
+  const size_t total = (size_t)hx * ny * nz;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     int s[3];
-    s[0] = (int)(t % gp.M[0]);
-    s[1] = (int)((t / gp.M[0]) % gp.M[1]);
-    s[2] = (int)(t / ((size_t)gp.M[0] * gp.M[1]));
+    s[0] = (int)(t % hx);
+    s[1] = (int)((t / hx) % ny);
+    s[2] = (int)(t / ((size_t)hx * ny));
     double p0[3];
     for (int e = 0; e < 3; e++) {
       const int h = gp.M[e] / 2;
@@ -142,7 +146,9 @@ __global__ void k_green_real(GreenParams gp, double *__restrict__ gr) {
           const double pz = p0[2] + gp.plen[2] * (double)kk;
           acc += green_k1(gp, sqrt(px * px + py * py + pz * pz));
         }
-    gr[t] = acc;
+    double *row = gr + ((size_t)s[2] * ny + s[1]) * gp.M[0];
+    row[s[0]] = acc;
+    if (s[0] > 0 && 2 * s[0] < gp.M[0]) row[gp.M[0] - s[0]] = acc;
   }
 }
 

@@ -116,6 +116,9 @@ struct BatchLayout {
 template <typename R, int NC>
 int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y, cudaStream_t st,
            const char *caller, int cs = NC);
+template <typename R, int NC>
+int even_forward(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y,
+                 typename cplx_t<R>::type *Z, cudaStream_t st, const char *caller);
 // periodic ghosts of a mesh of nv components
 template <typename R>
 int ghost_fill_all(const pmgpu_topo *topo, R *mesh, int nv, cudaStream_t st, const char *caller);

@@ -226,9 +226,9 @@ static int launch_lines(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typ
   return 0;
 }
 
+// x forward: real cuboid (component stride cs) -> X
 template <typename R, int NC>
-int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y,
-           cudaStream_t st, const char *caller, int cs) {
+static int xfwd(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, cudaStream_t st, const char *caller, int cs) {
   typedef typename cplx_t<R>::type C;
   const bool vec16r = cs == NC && ((size_t)g.ext[0] * NC * sizeof(R)) % 16 == 0 &&
                       ((size_t)g.off[0] * NC * sizeof(R)) % 16 == 0 && ((size_t)g.P[0] * NC * sizeof(R)) % 16 == 0;
@@ -255,8 +255,7 @@ int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename c
       }
     }
     if (launch(kern, sh.pairs ? 2 : 1)) return -1;
-    KTimer kt_(KC_YFWD, st);
-    return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, line_tiles(g, 1, L_FWD, 0, 0), st, caller);
+    return 0;
   }
   const int ntwx = g.fx.ntw + g.fx.next;
   const int RB = pick_rb(g.N2, g.P[0], g.Hp, NC, sizeof(C), sizeof(R), ntwx, false);
@@ -275,8 +274,35 @@ int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename c
     k_xfwd<R, NC><<<persistent_grid(k_xfwd<R, NC>, sm, ntiles), PASS_THREADS, sm, st>>>(g, in, X, RB, cs, vec16 ? 1 : 0); }
   PM_LAUNCHED();
   CKL(caller);
+  return 0;
+}
+
+template <typename R, int NC>
+int fwd_xy(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y,
+           cudaStream_t st, const char *caller, int cs) {
+  if (xfwd<R, NC>(g, in, X, st, caller, cs)) return -1;
   KTimer kt_(KC_YFWD, st);
   return launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, line_tiles(g, 1, L_FWD, 0, 0), st, caller);
+}
+
+// Transform of a real sequence even in y and z (M1 / 2 + 1 rows of M2 / 2 + 1 planes of M0 reals
+// in `in`): x on those rows, y on those planes with the other rows read from their mirror
+// -> Y, z the same way for the spectrum rows of ky <= M1 / 2 -> Z (M2 planes).  Needs the
+// register engine on every axis.
+template <typename R, int NC>
+int even_forward(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y,
+                 typename cplx_t<R>::type *Z, cudaStream_t st, const char *caller) {
+  SolveGeom<R> h = g;
+  for (int e = 1; e < 3; e++) h.ext[e] = h.P[e] = g.M[e] / 2 + 1;
+  if (xfwd<R, NC>(h, in, X, st, caller, NC)) return -1;
+  LineTiles ty = line_tiles(h, 1, L_FWD, 0, 0), tz = line_tiles(h, 2, L_Z, g.M[1], g.M[2]);
+  ty.rows_in = g.M[1];
+  tz.rows_in = g.M[2];
+  ty.even = tz.even = 1;
+  { KTimer kt_(KC_YFWD, st);
+    if (launch_lines<R, NC>(g, X, Y, 1, L_FWD, 0, 0, 0, ty, st, caller)) return -1; }
+  KTimer kt_(KC_ZPASS, st);
+  return launch_lines<R, NC>(g, Y, Z, 2, L_FWD, Z_FORWARD, 0, 0, tz, st, caller);
 }
 
 // one forward (or inverse) pass along y over the X layout -> Y layout, as in fwd_xy
@@ -544,6 +570,8 @@ int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters,
                             cudaStream_t, const char *);                                                       \
   template int inv_yx<R, NC>(SolveGeom<R> &, const pmgpu_topo *, cplx_t<R>::type *, cplx_t<R>::type *, R *,    \
                              cudaStream_t, const char *, int, bool);                                           \
+  template int even_forward<R, NC>(SolveGeom<R> &, const R *, cplx_t<R>::type *, cplx_t<R>::type *,             \
+                                   cplx_t<R>::type *, cudaStream_t, const char *);                              \
   template int ypass<R, NC>(SolveGeom<R> &, const cplx_t<R>::type *, cplx_t<R>::type *, int, cudaStream_t,      \
                             const char *);                                                                     \
   int upload_cs_##NAME(const void *t32, const void *t64) { return upload_cs_local(t32, t64); }                 \
@@ -551,10 +579,10 @@ int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters,
 
 #define PMGPU_INSTANTIATE_BATCH(R, NC)                                                                         \
   namespace pmgpu {                                                                                            \
+  template int ghost_fill_all<R>(const pmgpu_topo *, R *, int, cudaStream_t, const char *);                    \
   template int batch_layout<R, NC>(int, const SolveGeom<R> *, cplx_t<R>::type *const *,                        \
                                    cplx_t<R>::type *const *, const pmgpu_topo *const *,                        \
                                    std::vector<unsigned char> &, BatchLayout &, const char *);                 \
   template int batch_launch<R, NC>(const BatchLayout &, const void *, unsigned *, const void *const *,          \
                                    void *const *, cudaStream_t, const char *);                                 \
   }
-  template int ghost_fill_all<R>(const pmgpu_topo *, R *, int, cudaStream_t, const char *);                    \

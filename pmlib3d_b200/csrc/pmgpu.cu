@@ -655,6 +655,7 @@ struct pmgpu_plan {
   DevBuf X, Y, Y2, Y3;
   // register-engine plans along y and z (in-place, digit-reversed spectra)
   int rx_ok, ry_ok, rz_ok;
+  bool stockham = false;  // an axis takes the Stockham passes
   LinePlan lx, ly, lz;
   int tky = 0, tkz = 0;  // tuned kx tiles (0: chosen by shared memory)
   DevBuf rtwx, rtwy, rtwz, rtsx, rtsy, rtsz, rbx0, rby0, rbz0, yk, zk, rextx, xpos;
@@ -893,8 +894,8 @@ static int launch_m2p_tile(const PartGeom<R> &g, const R *pos, const unsigned *s
     const int r = (1 - g.blo[e]) % T;
     return r ? r - T : 0;
   };
-  const int3 o3 = make_int3(org(0, M2P_TX), org(1, TY), org(2, TZ));
   constexpr int M2P_TX = m2p_tx<W>();
+  const int3 o3 = make_int3(org(0, M2P_TX), org(1, TY), org(2, TZ));
   dim3 grid((g.nb[0] - o3.x + M2P_TX - 1) / M2P_TX, (g.nb[1] - o3.y + TY - 1) / TY, (g.nb[2] - o3.z + TZ - 1) / TZ);
   { KTimer kt_(KC_M2P, st); k_m2p_tile<R, W, TY, TZ><<<grid, M2P_THREADS, sm, st>>>(g, pos, start, perm, f, o, o3); }
   PM_LAUNCHED();
@@ -1134,7 +1135,7 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
   tmp.gM1 = tmp.gM2 = 0;
   // temporaries are stream-ordered on the legacy stream, so a set-up does not wait
   // for (or stall) solves running on other streams
-  DevBuf gr, gX, gY, yinv, zinv;
+  DevBuf gr, gX, gY, gH, yinv, zinv;
   int rc = -1;
   do {
     if (reg_tables<double>(&tmp, caller, false) || stockham_tables<double>(&tmp, 1, caller)) break;
@@ -1159,10 +1160,18 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
     if (yinv.ensure(sizeof(int) * G.M[1], caller) || zinv.ensure(sizeof(int) * G.M[2], caller)) break;
     if (!cuda_ok(cudaMemcpy(yinv.p, yi.data(), sizeof(int) * G.M[1], cudaMemcpyHostToDevice), caller)) break;
     if (!cuda_ok(cudaMemcpy(zinv.p, zi.data(), sizeof(int) * G.M[2], cudaMemcpyHostToDevice), caller)) break;
-    const size_t npts = (size_t)G.M[0] * G.M[1] * G.M[2];
+    // kernel 1 is even in every axis (transform lengths are even): an eighth of its values, a
+    // quarter of the x rows, half of the y planes and half of the z rows make its octant, and
+    // the temporaries are that much smaller.  Through the Stockham passes, which read every
+    // row, all of it.  Set-up, one solve and release of a 120 x 88 x 72 FP32 grid 1003 us with
+    // all of it, 550 with the octant's share; set-up alone at 120^3 1155 / 468
+    const bool even = pl->green_mode == 0 && gp.kernel == 1 && !tmp.stockham;
+    const size_t npts = even ? (size_t)G.M[0] * pl->gM1 * pl->gM2 : (size_t)G.M[0] * G.M[1] * G.M[2];
     const size_t nspec = (size_t)G.M[2] * G.M[1] * G.Hp;
-    if (gr.ensure(sizeof(double) * npts, caller) || gX.ensure(sizeof(double2) * nspec, caller) ||
-        gY.ensure(sizeof(double2) * nspec, caller))
+    if (gr.ensure(sizeof(double) * npts, caller) ||
+        gX.ensure(sizeof(double2) * (even ? (size_t)pl->gM2 * pl->gM1 * G.Hp : nspec), caller) ||
+        gY.ensure(sizeof(double2) * nspec, caller) ||
+        (even && gH.ensure(sizeof(double2) * (size_t)pl->gM2 * G.M[1] * G.Hp, caller)))
       break;
     const size_t noct = (size_t)pl->gM2 * pl->gM1 * G.Hp;
     const double f = pl->patch.dx[0] * pl->patch.dx[1] * pl->patch.dx[2] /
@@ -1201,11 +1210,16 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
       PM_LAUNCHED();
       if (!cuda_ok(cudaGetLastError(), caller)) break;
     } else if (gp.kernel == 1) {
-      k_green_real<<<nb_real, 256>>>(gp, gr.as<double>());
+      k_green_real<<<nb_real, 256>>>(gp, even ? 0 : 1, gr.as<double>());
       PM_LAUNCHED();
       if (!cuda_ok(cudaGetLastError(), caller)) break;
-      if (fwd_xy<double, 1>(gg, gr.as<double>(), gX.as<double2>(), gY.as<double2>(), 0, caller)) break;
-      if (zpass<double, 1>(gg, gY.as<double2>(), gY.as<double2>(), Z_FORWARD, 0, 0, G.M[1], 0, caller)) break;
+      if (even) {
+        if (even_forward<double, 1>(gg, gr.as<double>(), gX.as<double2>(), gH.as<double2>(), gY.as<double2>(), 0, caller))
+          break;
+      } else {
+        if (fwd_xy<double, 1>(gg, gr.as<double>(), gX.as<double2>(), gY.as<double2>(), 0, caller)) break;
+        if (zpass<double, 1>(gg, gY.as<double2>(), gY.as<double2>(), Z_FORWARD, 0, 0, G.M[1], 0, caller)) break;
+      }
       if (!cuda_ok(cudaStreamSynchronize(0), caller)) break;
       if (own->ensure(sizeof(R) * noct, caller)) break;
       attach_green(pl, own);
@@ -1239,7 +1253,7 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
     g_green_cache[key] = own;
     rc = 0;
   } while (0);
-  gr.release(); gX.release(); gY.release(); yinv.release(); zinv.release();
+  gr.release(); gX.release(); gY.release(); gH.release(); yinv.release(); zinv.release();
   cudaStreamSynchronize(0);
   return rc;
 }
@@ -1611,6 +1625,7 @@ template <typename R> static int stockham_tables(pmgpu_plan *pl, int nc, const c
   if (pl->rx_ok && pl->ry_ok && pl->rz_ok && fits_x(false) && fits_x(true) &&
       line_smem(pl->ly, nc, 1, sizeof(R)) <= PASS_SMEM_BUDGET && line_smem(pl->lz, nc, 1, sizeof(R)) <= PASS_SMEM_BUDGET)
     return 0;
+  pl->stockham = true;
   std::vector<cld> tw;
   return !make_fft(G.N2, G.M[0], pl->fx, tw) || upload_tw<R>(tw, pl->twx, caller) ||
                  !make_fft(G.M[1], 0, pl->fy, tw) || upload_tw<R>(tw, pl->twy, caller) ||

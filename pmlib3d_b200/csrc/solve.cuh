@@ -146,6 +146,9 @@ struct LineTiles {
   long long in_kb, out_kb;  // strides between kx blocks
   int nouter, nkt, TK;
   int ofast;      // consecutive tiles: outer index fastest (z pass) or kx tile fastest
+  // even input of n rows (the Green's function): rows beyond n / 2 are read from their
+  // mirror, and z tiles of the mirrored half of ky are left out
+  int even;
   FastDiv dLG;    // division by the line vectors per row (register engine)
 };
 // kx of a block of the spectral arrays: 192 bytes of three components
@@ -572,6 +575,14 @@ __device__ __forceinline__ LineSmem line_setup(const SolveGeom<typename LineT<T>
                    : line_tables<T>(g.lz, g.rtwz, g.rtsz, g.rbz0, g.rchz, g.rbz, lmode == L_INV);
 }
 
+// rows whose second half mirrors the first (mirror = number of rows; 0: plain rows)
+template <typename T> struct EvenIo : LineIo<T> {
+  int mirror;
+  __device__ __forceinline__ LV<T> load(int row, int g) const {
+    return LineIo<T>::load(2 * row > mirror && mirror ? mirror - row : row, g);
+  }
+};
+
 // the rows of tile (o, k0) of a line pass
 template <typename T>
 __device__ __forceinline__ LineIo<T> line_io(const LineTiles &lt, const typename cplx_t<typename LineT<T>::R>::type *in,
@@ -605,14 +616,17 @@ __device__ __forceinline__ void line_tile(const SolveGeom<typename LineT<T>::R> 
                                           typename cplx_t<typename LineT<T>::R>::type *out, int nc, int axis, int lmode,
                                           int zmode, int reproj, int use_zeta, const LineSmem &s, int tile) {
   typedef typename LineT<T>::V V;
-  typedef LineIo<T> IO;
+  typedef EvenIo<T> IO;
   const LinePlan &pl = (axis == 1) ? g.ly : g.lz;
   const int LG = nc * lt.TK / LineT<T>::G;
   const RtPlan rp{pl, LG, lt.dLG};
   const bool blue = pl.bl != 0;
   int o, k0;
   line_tile_at(lt, tile, lt.TK, o, k0);
-  const IO io = line_io<T>(lt, in, out, nc, o, k0);
+  if (lt.even && axis == 2 && 2 * (g.yk ? g.yk[o] : o) > g.M[1]) return;
+  IO io;
+  static_cast<LineIo<T> &>(io) = line_io<T>(lt, in, out, nc, o, k0);
+  io.mirror = lt.even ? lt.n : 0;
   V *const buf = line_smem_at<V>(s.tabs.buf);
   const int y = g.yk ? g.yk[o] : o;  // z pass: the spectrum row's ky
   const bool zvel = lmode == L_Z && zmode == Z_VEL && nc == 3 && z_plain(g, use_zeta);
@@ -1536,20 +1550,6 @@ __global__ void k_ghost_fill(R *__restrict__ mesh, int ex, int ey, int ez, int n
     ghost_fill_point<R>(mesh, ex, ey, ez, nv, axis, N, ngl, ngh, t);
 }
 
-// the ghost fill along one axis of every patch of a batch that is periodic there:
-// patch i's ghost points are items [first, first + total) of one index space
-struct GhostDesc {
-  long long first, total;
-  int patch, ext[3], nv, N, ngl, ngh;
-};
-template <typename R>
-__global__ void k_ghost_fill_batch(const GhostDesc *__restrict__ d, int npatch, long long total, int axis,
-                                   BatchIo io) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = npatch - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
 // All periodic ghosts of a mesh in one launch: every point of a periodic axis's ghost strips
 // copies its image in the interior of all periodic axes, which is what filling the axes in
 // turn leaves there (a point in two strips is written twice, with the same value).
@@ -1583,6 +1583,20 @@ template <typename R> __global__ void k_ghost_fill_all(GhostAll q, R *__restrict
   }
 }
 
+// the ghost fill along one axis of every patch of a batch that is periodic there:
+// patch i's ghost points are items [first, first + total) of one index space
+struct GhostDesc {
+  long long first, total;
+  int patch, ext[3], nv, N, ngl, ngh;
+};
+template <typename R>
+__global__ void k_ghost_fill_batch(const GhostDesc *__restrict__ d, int npatch, long long total, int axis,
+                                   BatchIo io) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    int lo = 0, hi = npatch - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
       if (d[mid].first <= t) lo = mid;
       else hi = mid - 1;
     }
