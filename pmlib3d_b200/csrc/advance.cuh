@@ -97,24 +97,40 @@ constexpr int ADV_PASSES = 2;  // map passes per axis the key holds
 // axis 4 bits (bits 0-1 the class in pass 1, bits 2-3 in pass 2; 2 = inside), bit 31
 // dropped.  stats[0] |= 1 when a particle leaves or is dropped, stats[1 + d] = the
 // most passes axis d needs, stats[4] = 1 when a particle needs more than ADV_PASSES.
+// Bound by HBM (ten arrays of three values a particle, 124 bytes in FP32) and, a particle a
+// thread, by its stores of every third value: the update runs over a CTA's values in memory
+// order (whole lines a warp), the wraps a particle a thread with the new positions in shared
+// memory.  8.0 M particles FP32 207 -> 153 us (6.5 TB/s), 1.5 M FP64 76 -> 55.
+constexpr int ADV_THREADS = 256;
 template <typename R>
-__global__ void k_advance(AdvanceCoef<R> c, int n, R *__restrict__ pos, R *__restrict__ vort,
-                          const R *__restrict__ vel, const R *__restrict__ dvort, R *__restrict__ vel_rk,
-                          R *__restrict__ dvort_rk, unsigned *__restrict__ code, unsigned *__restrict__ stats) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int p0 = blockIdx.x * blockDim.x; p0 < n; p0 += stride) {
-    const int p = p0 + (int)threadIdx.x;
+__global__ void __launch_bounds__(ADV_THREADS)
+    k_advance(AdvanceCoef<R> c, int n, R *__restrict__ pos, R *__restrict__ vort, const R *__restrict__ vel,
+              const R *__restrict__ dvort, R *__restrict__ vel_rk, R *__restrict__ dvort_rk,
+              unsigned *__restrict__ code, unsigned *__restrict__ stats) {
+  __shared__ R sx[3 * ADV_THREADS];
+  const int stride = gridDim.x * ADV_THREADS;
+  for (int p0 = blockIdx.x * ADV_THREADS; p0 < n; p0 += stride) {
+    const int p = p0 + (int)threadIdx.x, len = 3 * min(ADV_THREADS, n - p0);
+    const size_t q0 = (size_t)3 * p0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const int f = i * ADV_THREADS + (int)threadIdx.x;
+      if (f < len) {
+        const size_t q = q0 + f;
+        const R vr = add_rn(mul_rn(c.a1, vel_rk[q]), mul_rn(c.b1dt, vel[q]));
+        const R dr = add_rn(mul_rn(c.a2, dvort_rk[q]), mul_rn(c.b2dt, dvort[q]));
+        sx[f] = add_rn(pos[q], mul_rn(c.c1, vr));
+        vort[q] = add_rn(vort[q], mul_rn(c.c2, dr));
+        vel_rk[q] = c.zero_rk ? R(0) : vr;
+        dvort_rk[q] = c.zero_rk ? R(0) : dr;
+      }
+    }
+    __syncthreads();
     unsigned cd = 0, np[3] = {0, 0, 0}, bad = 0;
     if (p < n) {
 #pragma unroll
       for (int e = 0; e < 3; e++) {
-        const size_t q = (size_t)3 * p + e;
-        const R vr = add_rn(mul_rn(c.a1, vel_rk[q]), mul_rn(c.b1dt, vel[q]));
-        const R dr = add_rn(mul_rn(c.a2, dvort_rk[q]), mul_rn(c.b2dt, dvort[q]));
-        R x = add_rn(pos[q], mul_rn(c.c1, vr));
-        vort[q] = add_rn(vort[q], mul_rn(c.c2, dr));
-        vel_rk[q] = c.zero_rk ? R(0) : vr;
-        dvort_rk[q] = c.zero_rk ? R(0) : dr;
+        R x = sx[3 * threadIdx.x + e];
         unsigned cls = 0xAu;  // both passes "inside"
         // pass t + 1 over this axis (a particle dropped on an earlier axis is gone)
         for (int t = 0; t <= ADV_PASSES && !(cd & ADV_REMOVED); t++) {
@@ -133,11 +149,14 @@ __global__ void k_advance(AdvanceCoef<R> c, int n, R *__restrict__ pos, R *__res
           cls = (cls & ~(3u << (2 * t))) | (side << (2 * t));
           np[e] = t + 1;
         }
-        pos[q] = x;
+        sx[3 * threadIdx.x + e] = x;
         cd |= cls << (4 * e);
       }
       code[p] = cd;
     }
+    __syncthreads();
+    for (int f = threadIdx.x; f < len; f += ADV_THREADS) pos[q0 + f] = sx[f];
+    __syncthreads();
     const unsigned moved = ((cd & ADV_REMOVED) || np[0] || np[1] || np[2]) ? 1u : 0u;
     const unsigned anym = __reduce_or_sync(0xffffffffu, moved | (bad << 1));
     if (anym) {

@@ -1003,7 +1003,7 @@ __global__ void k_m2p(PartGeom<R> g, const R *__restrict__ pos, const int *__res
 constexpr int M2P_THREADS = 256;
 // bins along x.  29 for W = 4: a staged row is then 32 cells, a multiple of the banks, and the
 // rows of a tile fill whole 128-byte lines.  Microseconds with 32 / 29: 256^3 FP64 1414 / 1403,
-// 104 x 104 x 136 FP64 (two fields) 319 / 311, 192^3 FP32 (two fields) 825 / 798, 256^3 FP32
+// 104 x 104 x 136 FP64 (two fields) 319 / 311, 200^3 FP32 (two fields) 825 / 798, 256^3 FP32
 // 792 / 790.  M6* takes 32 (150 x 121 x 95: 228; 27, the same row, 235)
 template <int W> __host__ __device__ constexpr int m2p_tx() { return W == 4 ? 29 : 32; }
 

@@ -1163,7 +1163,7 @@ template <typename R> static int setup_green(pmgpu_plan *pl, const char *caller)
     // kernel 1 is even in every axis (transform lengths are even): an eighth of its values, a
     // quarter of the x rows, half of the y planes and half of the z rows make its octant, and
     // the temporaries are that much smaller.  Through the Stockham passes, which read every
-    // row, all of it.  Set-up, one solve and release of a 120 x 88 x 72 FP32 grid 1003 us with
+    // row, all of it.  Set-up, one solve and release of a 136 x 104 x 88 FP32 grid 1003 us with
     // all of it, 550 with the octant's share; set-up alone at 120^3 1155 / 468
     const bool even = pl->green_mode == 0 && gp.kernel == 1 && !tmp.stockham;
     const size_t npts = even ? (size_t)G.M[0] * pl->gM1 * pl->gM2 : (size_t)G.M[0] * G.M[1] * G.M[2];
@@ -2895,8 +2895,8 @@ static int run_advance(const pmgpu_patch *pa, pmgpu_topo *t, int order, int stag
     return -1;
   unsigned *stats = s.adv_stats.as<unsigned>();
   CK(cudaMemsetAsync(stats, 0, sizeof(unsigned) * 8, st), caller);
-  const int nblk = std::min((n + 255) / 256, 148 * 16);
-  { KTimer kt_(KC_ADVANCE, st); k_advance<R><<<nblk, 256, 0, st>>>(c, n, pos, vort, vel, dvort, vel_rk, dvort_rk,
+  const int nblk = std::min((n + ADV_THREADS - 1) / ADV_THREADS, 148 * 16);
+  { KTimer kt_(KC_ADVANCE, st); k_advance<R><<<nblk, ADV_THREADS, 0, st>>>(c, n, pos, vort, vel, dvort, vel_rk, dvort_rk,
                                                                    s.adv_code.as<unsigned>(), stats); }
   PM_LAUNCHED();
   CKL(caller);
