@@ -23,7 +23,7 @@ OUT = os.path.join(HERE, "libpmgpu.so")
 BUILD = os.path.join(HERE, "_build")
 UNITS = ([os.path.join(CSRC, "pmgpu.cu")] + sorted(glob.glob(os.path.join(CSRC, "passes_*.cu"))) +
          [os.path.join(CSRC, "output.cu")])
-HEADERS = sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h"))) + [
+HEADERS = sorted(p for e in ("cuh", "h", "inc") for p in glob.glob(os.path.join(CSRC, "*." + e))) + [
     os.path.join(os.path.dirname(HERE), "include", "pmlib_gpu.h")]
 
 

@@ -47,6 +47,16 @@ constexpr size_t PASS_SMEM_BUDGET = 220 * 1024;
 // which 1 KB a CTA is the system's)
 constexpr size_t LINE_SMEM_4 = 56 * 1024;
 constexpr size_t LINE_SMEM_2 = 113 * 1024;
+// shared memory the batched kernels keep for their own bookkeeping (the patch
+// descriptor copy and the chunk counter), taken off the per-CTA budgets so that as
+// many CTAs fit on an SM as in the passes of a single plan
+constexpr size_t BATCH_SMEM_SLACK = 3 * 1024;
+// A line tile takes its whole kx block (rows of 192 bytes) if its `bytes` of shared memory
+// fit: on two CTAs an SM for Bluestein and the z pass of a single plan, which spend their
+// time on the transforms, else on four; longer y lines take half of it (three CTAs an SM)
+constexpr bool line_whole_block(size_t bytes, bool two_ctas) {
+  return bytes <= (two_ctas ? LINE_SMEM_2 : LINE_SMEM_4);
+}
 
 static inline size_t tw_bytes(int ntw, size_t csize) { return (size_t)((ntw + 7) & ~7) * csize; }
 

@@ -360,6 +360,7 @@ template <int N_, int SPLIT_, int LGV, int R0, int R1 = 1, int R2 = 1> struct Ct
   }
   __host__ __device__ static constexpr int tin(int p) { return str(p) / inner(p); }
   __host__ __device__ static constexpr int tmul(int p) { return inner(p) > 1 ? N / (rad(p) * inner(p)) : 0; }
+  __host__ __device__ static constexpr bool twiddles() { return tmul(0) || (NP > 1 && tmul(1)) || (NP > 2 && tmul(2)); }
   __host__ __device__ static constexpr int rstep() {
     return N / (rad(0) * inner(0)) * inner(0) % N;
   }

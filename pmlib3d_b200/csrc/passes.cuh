@@ -71,10 +71,7 @@ static LineShape line_shape(const SolveGeom<R> &g, int axis, size_t slack) {
     return LineShape{tk, line_threads(pl, lg, bytes(tk))};
   };
   if (tuned > 0 && tuned <= top && bytes(tuned) <= PASS_SMEM_BUDGET) return shape(tuned);
-  // the whole block (rows of 192 bytes) for short lines, Bluestein and the z pass, which spend
-  // their time on the transforms; half of it (three CTAs an SM) for longer y lines
-  const size_t whole = (axis == 2 || pl.bl) && slack == 0 ? LINE_SMEM_2 : LINE_SMEM_4;
-  if (bytes(top) <= whole) return shape(top);
+  if (line_whole_block(bytes(top), (axis == 2 || pl.bl) && slack == 0)) return shape(top);
   for (size_t budget : {LINE_SMEM_2, PASS_SMEM_BUDGET})
     if (bytes(top / 2) <= budget) return shape(top / 2);
   for (int tk = top / 4; tk >= 1; tk /= 2)
@@ -379,11 +376,6 @@ int inv_yx(SolveGeom<R> &g, const pmgpu_topo *topo, typename cplx_t<R>::type *Y,
 
 
 // ---------------------------------------------------------------- batches of patches
-// shared memory the batched kernels keep for their own bookkeeping (the patch
-// descriptor copy and the chunk counter), taken off the per-CTA budgets so that as
-// many CTAs fit on an SM as in the passes of a single plan
-constexpr size_t BATCH_SMEM_SLACK = 3 * 1024;
-
 template <typename R, int NC>
 int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *X,
                  typename cplx_t<R>::type *const *Y, const pmgpu_topo *const *topo, std::vector<unsigned char> &desc,
@@ -429,8 +421,7 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
       q.out = inv ? nullptr : X[i];  // x inverse writes the caller's velocity
       q.ntiles = (gi.P[1] * gi.P[2] + RB - 1) / RB;
       const int lg = NC * RB / (sizeof(R) == 4 ? 2 : 1);
-      const bool ct = g_fft_ct && (inv ? rxinv_kernel_ct<R>(gi.lx, lg) != nullptr : rxfwd_kernel_ct<R>(gi.lx, lg) != nullptr);
-      add(f, i, ct ? plan_class(gi.lx.n, gi.lx.split, lg) : 0, sm, q);
+      add(f, i, g_fft_ct ? rx_batch_class<R>(gi.lx, lg) : 0, sm, q);
     }
     // y forward, z pass, y inverse (run_solve's launch_lines arguments)
     for (int f = 1; f <= 3; f++) {
@@ -451,8 +442,8 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
       q.out = f == 3 ? X[i] : Y[i];
       q.ntiles = lt.nouter * lt.nkt;
       const int lmode = f == 3 ? L_INV : f == 2 ? L_Z : L_FWD, lg = NC * TK / (sizeof(R) == 4 ? 2 : 1);
-      const bool ct = g_fft_ct && (f != 2 || z_plain(gi, 0)) && lines_kernel_ct<R>(lmode, pl, lg) != nullptr;
-      add(f, i, ct ? plan_class(pl.n, pl.split, lg) : 0, line_smem(pl, NC, TK, sizeof(R)), q);
+      const bool plain = f != 2 || z_plain(gi, 0);
+      add(f, i, g_fft_ct && plain ? lines_batch_class<R>(lmode, pl, lg) : 0, line_smem(pl, NC, TK, sizeof(R)), q);
     }
     // periodic ghosts of the velocity (x, then y, then z)
     for (int a = 0; a < 3; a++) {

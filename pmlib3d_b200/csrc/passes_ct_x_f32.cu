@@ -1,22 +1,7 @@
-// passes_ct_x_f32.cu -- compile-time x passes (float fields of 3 components), and the choice among
-// the compile-time line passes.
+// passes_ct_x_f32.cu -- compile-time x passes (float fields of 3 components).
 #include "kernels.cuh"
 
 namespace pmgpu {
-
-LinesKernel<float> ct_yf_f32_kernel(const LinePlan &pl, int lg);
-LinesKernel<float> ct_yi_f32_kernel(const LinePlan &pl, int lg);
-LinesKernel<float> ct_z_f32_kernel(const LinePlan &pl, int lg);
-template <> LinesKernel<float> lines_kernel_ct<float>(int lmode, const LinePlan &pl, int lg) {
-  return lmode == L_FWD ? ct_yf_f32_kernel(pl, lg) : lmode == L_INV ? ct_yi_f32_kernel(pl, lg) : ct_z_f32_kernel(pl, lg);
-}
-
-LinesBatchCt ct_yf_f32_batch();
-LinesBatchCt ct_yi_f32_batch();
-LinesBatchCt ct_z_f32_batch();
-template <> LinesBatchCt lines_batch_ct<float>(int lmode) {
-  return lmode == L_FWD ? ct_yf_f32_batch() : lmode == L_INV ? ct_yi_f32_batch() : ct_z_f32_batch();
-}
 
 #define PMGPU_PLAN_X_F32(S, N, A, B, C)                                                    \
   if (lg == 12 && CtPlan<N, S, 12, A, B, C>::is(pl)) return K<float2, 3, CtPlan<N, S, 12, A, B, C>>; \

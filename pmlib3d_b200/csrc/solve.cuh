@@ -520,16 +520,16 @@ __host__ __device__ inline bool plan_twiddles(const LinePlan &p) {
   for (int i = 0; i < p.np; i++) t = t || p.tmul[i] != 0;
   return t;
 }
-// bytes of the tables of a line pass in shared memory; wsize / csize: a twiddle, a
-// complex value
+// bytes of the tables of a line pass in shared memory (a direct plan of n points and first
+// radix r0); wsize / csize: a twiddle, a complex value
+__host__ __device__ constexpr size_t line_tab_bytes(int n, bool twiddles, bool split, int r0, size_t wsize) {
+  return (((twiddles + split) * (size_t)n * wsize + 15) & ~(size_t)15) +
+         (((size_t)(n / r0) * sizeof(int) + 15) & ~(size_t)15);
+}
 __host__ __device__ inline size_t line_tab_bytes(const LinePlan &p, size_t wsize, size_t csize) {
-  size_t b = 0;
-  if (plan_twiddles(p)) b += (size_t)p.n * wsize;
-  if (p.split) b += (size_t)p.n * wsize;
-  b = (b + 15) & ~(size_t)15;
-  if (!p.bl) b += ((size_t)(p.n / p.rad[0]) * sizeof(int) + 15) & ~(size_t)15;
-  else b += ((size_t)(p.bn + p.n) * csize + 15) & ~(size_t)15;
-  return b;
+  if (!p.bl) return line_tab_bytes(p.n, plan_twiddles(p), p.split != 0, p.rad[0], wsize);
+  return (((plan_twiddles(p) + (p.split != 0)) * (size_t)p.n * wsize + 15) & ~(size_t)15) +
+         (((size_t)(p.bn + p.n) * csize + 15) & ~(size_t)15);
 }
 
 // carves the tables of plan pl out of shared memory and stages them (Bluestein: the product
