@@ -59,6 +59,8 @@ __host__ __device__ constexpr bool reg_radix(int r) {
   return r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 7 || r == 8 || r == 9 || r == 10 || r == 11 ||
          r == 12 || r == 13 || r == 16 || r == 17;
 }
+// first digits of a split plan: a thread holds both halves of such a butterfly
+__host__ __device__ constexpr bool split_radix(int r) { return r <= 13 || r == 17; }
 // further composite radices, FP32 schedules only
 __host__ __device__ constexpr bool reg_radix_wide(int r) { return r == 18 || r == 20 || r == 22 || r == 24; }
 
@@ -400,8 +402,7 @@ __device__ __forceinline__ void lphase(const PL &pl, int p, const LineTabs &tb, 
   const int s = pl.str(p), n = pl.n(), tm = pl.tmul(p), LG = pl.LG();
   const int sv = s * LG;
   V *const buf = line_smem_at<V>(tb.buf);
-  // (digit 0 of a split plan is at most 13, or 17)
-  constexpr bool SPLIT0 = RAD <= 13 || RAD == 17;
+  constexpr bool SPLIT0 = split_radix(RAD);
   if (SPLIT0 && p == 0 && glob && pl.split()) {
     // both halves of a butterfly in one thread: its rows are read (written) once
     if constexpr (SPLIT0) {

@@ -21,6 +21,7 @@
 #include <deque>
 #include <map>
 #include <memory>
+#include <set>
 #include <tuple>
 #include <mutex>
 #include <string>
@@ -282,9 +283,10 @@ template <typename R> static int upload_tw(const std::vector<cld> &tw, DevBuf &b
   return 0;
 }
 
-// Autotuned schedules: (length, precision, axis) -> radix sequence and kx tile, the
-// fastest measured forward pass among the candidates (process-wide, filled when
-// plans are created while tuning is on).
+// Autotuned schedules: (length, precision, axis) -> radix sequence of the whole line and kx
+// tile, the fastest measured forward pass among the candidates (process-wide, filled when
+// plans are created while tuning is on).  Padded and periodic lines of a length share the
+// entry, so its radices are always ones that either can run (schedule_radices).
 struct TunedSchedule {
   int np;
   int r[3];
@@ -292,6 +294,9 @@ struct TunedSchedule {
   double ms;
 };
 static std::map<std::tuple<int, int, int>, TunedSchedule> g_tuned;
+// lines (length, precision, axis, split) whose default plan was measured fastest and has no
+// such radices: they keep it, without an entry
+static std::set<std::tuple<int, int, int, int>> g_tuned_default;
 static int g_tune = 0;
 
 // ------------------------------------------------------------------ line plans (y and z)
@@ -470,25 +475,49 @@ static std::vector<RadixSeq> line_candidates(int n, int split, int axis, int rsi
   return out;
 }
 
+// radices of the whole-line schedules
+static bool schedule_radix(int r, int rsize) { return reg_radix(r) || (rsize == 4 && reg_radix_wide(r)); }
+
 // The digits of a schedule (radices of the whole line, as the schedule table holds them)
 // for a split plan: the padding's factor 2 comes off the first radix if that leaves a
-// digit, else off the largest even radix, which then comes first.
-static bool schedule_digits(const int *r, int np, int split, int *d, int &nd) {
+// digit, else off the largest even radix, which then comes first.  false: the engine has no
+// such digits, and the line keeps its default plan.
+static bool schedule_digits(const int *r, int np, int split, int rsize, int *d, int &nd) {
   nd = 0;
-  if (!split) {
-    for (int i = 0; i < np; i++) d[nd++] = r[i];
-    return true;
-  }
   int h = -1;
-  if (r[0] % 2 == 0 && r[0] > 2) h = 0;
-  else
-    for (int i = 0; i < np; i++)
-      if (r[i] % 2 == 0 && (h < 0 || r[i] > r[h])) h = i;
-  if (h < 0) return false;
-  if (r[h] > 2) d[nd++] = r[h] / 2;
+  if (split) {
+    if (r[0] % 2 == 0 && r[0] > 2) h = 0;
+    else
+      for (int i = 0; i < np; i++)
+        if (r[i] % 2 == 0 && (h < 0 || r[i] > r[h])) h = i;
+    if (h < 0) return false;
+    if (r[h] > 2) d[nd++] = r[h] / 2;
+  }
   for (int i = 0; i < np; i++)
     if (i != h) d[nd++] = r[i];
-  return nd > 0;
+  for (int i = 0; i < nd; i++)
+    if (!schedule_radix(d[i], rsize)) return false;
+  return nd > 0 && (!split || split_radix(d[0]));
+}
+
+// Whole-line radices that stand for a plan's digits in the schedule table: radices of the
+// schedules (a periodic line of the length can run them, and they can be set again) from
+// which schedule_digits makes the same digits.  false: there are none (a first digit 7, whose
+// double is no radix, with an even digit after it).
+static bool schedule_radices(const int *d, int nd, int split, int rsize, int *r, int &np) {
+  auto same = [&](std::initializer_list<int> q) {
+    np = 0;
+    for (int v : q)
+      if (v > 1) r[np++] = v;
+    for (int i = 0; i < np; i++)
+      if (!schedule_radix(r[i], rsize)) return false;
+    int e[LP_MAX + 1], ne = 0;
+    if (np > LP_MAX || !schedule_digits(r, np, split, rsize, e, ne) || ne != nd) return false;
+    return std::equal(d, d + nd, e);
+  };
+  const int d1 = nd > 1 ? d[1] : 1, d2 = nd > 2 ? d[2] : 1;
+  if (!split) return same({d[0], d1, d2});
+  return same({2 * d[0], d1, d2}) || (nd < LP_MAX && (same({d[0], d1, 2}) || same({2, d[0], d1})));
 }
 
 // the plan of a line of M points along `axis`; half: the second half is zero padding
@@ -1344,15 +1373,23 @@ static int zvel_upload(const pmgpu_plan *pl, const LinePlan &, LineBufs &t, cons
 
 // Times the pass along `axis` of this plan's geometry (y: the forward pass; z: the
 // fused transform / multiply / inverse pass of the velocity solve) for the candidate
-// radix sequences (the five best by the model) and kx tiles, on scratch arrays; the
-// fastest goes to the tuning table.  The plan's Green's function must exist.
+// radix sequences (the eight best by the model of those that the table can hold) and kx
+// tiles, on scratch arrays; the fastest goes to the tuning table.  best.np = 0: the default
+// plan, which the table cannot hold, is faster than all of them.  The plan's Green's
+// function must exist.
 template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedule &best, const char *caller) {
   typedef typename cplx_t<R>::type C;
   const Geometry &G = pl->g;
-  const int n = G.M[axis];
-  const int split = G.M[axis] == 2 * G.P[axis] && n >= 4 ? 1 : 0, m = split ? n / 2 : n;
-  std::vector<RadixSeq> cands = line_candidates(m, split, axis, (int)sizeof(R));
+  const LinePlan now = axis == 1 ? pl->ly : pl->lz;
+  const int split = now.split, m = now.n, rsize = (int)sizeof(R);
+  int whole[LP_MAX], np = 0;
+  std::vector<RadixSeq> cands = line_candidates(m, split, axis, rsize);
+  cands.erase(std::remove_if(cands.begin(), cands.end(),
+                             [&](const RadixSeq &c) { return !schedule_radices(c.r, c.np, split, rsize, whole, np); }),
+              cands.end());
   if (cands.size() > 8) cands.resize(8);
+  if (!schedule_radices(now.rad, now.np, split, rsize, whole, np))
+    cands.push_back(RadixSeq{now.np, {now.rad[0], now.rad[1], now.rad[2]}, 0.0});
   DevBuf A, B;
   LineBufs tabs;
   const size_t nx = (size_t)G.P[1] * G.P[2] * G.Hp * 3;
@@ -1364,13 +1401,15 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
   CK(cudaEventCreate(&e0), caller);
   CK(cudaEventCreate(&e1), caller);
   best.ms = 1e30;
-  best.np = 0;
+  best.np = -1;
   for (const RadixSeq &c : cands) {
     LinePlan lp;
     lineplan_from(m, split, c.r, c.np, false, lp);
     if (line_upload<R>(lp, tabs, caller)) break;
-    for (int tk : {8, 4, 2}) {
-      if (tk > spec_block<R>() || line_smem(lp, 3, tk, sizeof(R)) > PASS_SMEM_BUDGET) continue;
+    const bool held = schedule_radices(c.r, c.np, split, rsize, whole, np);
+    for (int tk : {8, 4, 2, 0}) {  // 0: the tile that the plan chooses
+      if (held ? tk == 0 || tk > spec_block<R>() || line_smem(lp, 3, tk, sizeof(R)) > PASS_SMEM_BUDGET : tk != 0)
+        continue;
       SolveGeom<R> g = solve_geom<R>(pl);
       if (axis == 1) {
         g.ly = lp;
@@ -1406,10 +1445,8 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
       cudaEventElapsedTime(&ms, e0, e1);
       if (ms / 3 < best.ms) {
         best.ms = ms / 3;
-        best.np = c.np;
-        // the table holds radices of the whole line
-        for (int i = 0; i < 3; i++) best.r[i] = i < c.np ? c.r[i] : 0;
-        if (split) best.r[0] *= 2;
+        best.np = held ? np : 0;
+        for (int i = 0; i < 3; i++) best.r[i] = i < best.np ? whole[i] : 0;
         best.tk = tk;
       }
     }
@@ -1417,7 +1454,7 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaGetLastError();
-  return best.np > 0 ? 0 : -1;
+  return best.np >= 0 ? 0 : -1;
 }
 
 // Device tables of the register engine, shared by every plan of the same transform
@@ -1536,7 +1573,7 @@ template <typename R> static int reg_tables(pmgpu_plan *pl, const char *caller, 
       // a schedule measured or set earlier for this length
       auto it = g_tuned.find(std::make_tuple(n, pb, axis));
       int d[LP_MAX], nd = 0;
-      if (it != g_tuned.end() && schedule_digits(it->second.r, it->second.np, lp.split, d, nd)) {
+      if (it != g_tuned.end() && schedule_digits(it->second.r, it->second.np, lp.split, pb, d, nd)) {
         lineplan_from(lp.n, lp.split, d, nd, false, lp);
         (axis == 1 ? pl->tky : pl->tkz) = it->second.tk;
       }
@@ -1602,11 +1639,16 @@ template <typename R> static int apply_tuning(pmgpu_plan *pl, const char *caller
   if (!g_tune || g_force_stockham) return 0;
   bool fresh = false;
   for (int axis = 1; axis <= 2; axis++) {
-    if (!(axis == 1 ? pl->ry_ok : pl->rz_ok) || (axis == 1 ? pl->ly : pl->lz).bl) continue;
+    const LinePlan &lp = axis == 1 ? pl->ly : pl->lz;
+    if (!(axis == 1 ? pl->ry_ok : pl->rz_ok) || lp.bl) continue;
     const auto key = std::make_tuple(pl->g.M[axis], (int)sizeof(R), axis);
-    if (g_tuned.count(key)) continue;
+    const auto kept = std::make_tuple(pl->g.M[axis], (int)sizeof(R), axis, lp.split);
+    if (g_tuned.count(key) || g_tuned_default.count(kept)) continue;
     TunedSchedule ts;
-    if (tune_axis<R>(pl, axis, ts, caller) == 0) {
+    if (tune_axis<R>(pl, axis, ts, caller)) continue;
+    if (ts.np == 0) {
+      g_tuned_default.insert(kept);
+    } else {
       g_tuned.emplace(key, ts);
       fresh = true;
     }
@@ -2719,9 +2761,11 @@ int pmgpu_fft_set_schedule(int length, int precision, int axis, const int *radic
     set_error(caller, "length, precision or axis out of range.");
     return -1;
   }
-  const auto key = std::make_tuple(length, precision == PMGPU_FP64 ? 8 : 4, axis);
+  const int rsize = precision == PMGPU_FP64 ? 8 : 4;
+  const auto key = std::make_tuple(length, rsize, axis);
   if (!radices) {
     g_tuned.erase(key);
+    for (int split = 0; split < 2; split++) g_tuned_default.erase(std::make_tuple(length, rsize, axis, split));
     return 0;
   }
   TunedSchedule ts;
@@ -2729,7 +2773,7 @@ int pmgpu_fft_set_schedule(int length, int precision, int axis, const int *radic
   long long prod = 1;
   for (int i = 0; i < 3 && radices[i] > 0; i++) {
     const int r = radices[i];
-    if (!(reg_radix(r) || (precision == PMGPU_FP32 && reg_radix_wide(r)))) {
+    if (!schedule_radix(r, rsize)) {
       set_error(caller, "radix not available.");
       return -1;
     }
