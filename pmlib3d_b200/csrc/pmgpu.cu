@@ -1400,7 +1400,11 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
   if (cands.size() > 8) cands.resize(8);
   if (!schedule_radices(now.rad, now.np, split, rsize, whole, np))
     cands.push_back(RadixSeq{now.np, {now.rad[0], now.rad[1], now.rad[2]}, 0.0});
-  DevBuf A, B;
+  struct Spectra {
+    DevBuf a, b;
+    ~Spectra() { a.release(); b.release(); }
+  } spectra;
+  DevBuf &A = spectra.a, &B = spectra.b;
   LineBufs tabs;
   const size_t nx = (size_t)G.P[1] * G.P[2] * G.Hp * 3;
   const size_t ny = (size_t)G.M[1] * G.P[2] * G.Hp * 3;

@@ -65,3 +65,21 @@ def test_padded_then_periodic(length, axis, prec):
         for e in P.fft_tuned():
             if (e["length"], e["precision"], e["axis"]) not in before:
                 P.fft_set_schedule(e["length"], _prec(e), e["axis"], None)
+
+
+def test_tuning_returns_its_memory():
+    """The tuner's scratch spectra (80 MB for these grids) go back to the pool: tuning three more
+    z lengths, each a little shorter, takes no further device memory.  Bound: half of one
+    length's spectrum of 50 MB."""
+    import torch
+    lengths = (128, 124, 120, 116)
+    for n in lengths:
+        P.fft_set_schedule(n, P.FP32, 2, None)
+    free = []
+    for n in lengths:
+        _solve((112, 112, n // 2 - 8), (0, 0, 0), P.FP32, tune=True)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    for n in lengths:
+        P.fft_set_schedule(n, P.FP32, 2, None)
+    assert free[0] - free[-1] < 25e6, free
