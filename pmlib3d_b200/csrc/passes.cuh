@@ -86,14 +86,19 @@ struct XShape {
   int rb, threads;
   bool pairs;
 };
-template <typename R, int NC> static XShape x_shape(const SolveGeom<R> &g, bool inverse, size_t slack) {
+// rows: all rows of the launch.
+template <typename R, int NC>
+static XShape x_shape(const SolveGeom<R> &g, bool inverse, size_t slack, long long rows) {
   if (!g.rx_ok) return XShape{0, 0, false};
   auto bytes = [&](int rb, bool pairs) {
     return x_smem(g.lx, g.N2, g.H, g.P[0], NC, rb, sizeof(R), pairs, inverse) + slack;
   };
   const bool f32 = sizeof(R) == 4;
-  // rows shorter than those of the compile-time plans: more of them, to fill the CTA
-  const int most = (f32 ? 8 : 4) * (plan_points(g.lx) < 32 ? 4 : 1);
+  // rows shorter than those of the compile-time plans: more of them, to fill the CTA, while
+  // that leaves two tiles an SM.  Solves in microseconds, always four times the rows / so many:
+  // 16^3 fff FP32 50.7 / 40.3, 40 x 40 x 40 ppf 57 / 47, 20 x 48 x 48 pff 61 / 56
+  int most = f32 ? 8 : 4;
+  for (int i = 0; i < 2 && plan_points(g.lx) < 32 && rows >= 2 * (2 * most) * (long long)num_sms(); i++) most *= 2;
   for (size_t budget : {LINE_SMEM_4, LINE_SMEM_2, PASS_SMEM_BUDGET})
     for (int rb = most; rb >= (budget == PASS_SMEM_BUDGET ? (f32 ? 2 : 1) : most / 2); rb /= 2)
       if (bytes(rb, f32) <= budget)
@@ -229,7 +234,7 @@ static int xfwd(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, cudaS
   typedef typename cplx_t<R>::type C;
   const bool vec16r = cs == NC && ((size_t)g.ext[0] * NC * sizeof(R)) % 16 == 0 &&
                       ((size_t)g.off[0] * NC * sizeof(R)) % 16 == 0 && ((size_t)g.P[0] * NC * sizeof(R)) % 16 == 0;
-  const XShape sh = x_shape<R, NC>(g, false, 0);
+  const XShape sh = x_shape<R, NC>(g, false, 0, (long long)g.P[1] * g.P[2]);
   if (sh.rb > 0) {
     const size_t sm = x_smem(g.lx, g.N2, g.H, g.P[0], NC, sh.rb, sizeof(R), sh.pairs, false);
     auto launch = [&](auto kern, int G) -> int {
@@ -332,7 +337,7 @@ int inv_yx(SolveGeom<R> &g, const pmgpu_topo *topo, typename cplx_t<R>::type *Y,
       return -1;
   }
   const int rows = g.P[1] * g.P[2];
-  const XShape sh = x_shape<R, NC>(g, true, 0);
+  const XShape sh = x_shape<R, NC>(g, true, 0, rows);
   if (sh.rb > 0) {
     const size_t sm = x_smem(g.lx, g.N2, g.H, g.P[0], NC, sh.rb, sizeof(R), sh.pairs, true);
     auto launch = [&](auto kern, int G) -> int {
@@ -385,19 +390,16 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
   if (n <= 0 || n > BATCH_MAX) return -1;
   lay = BatchLayout();
   lay.npatch = n;
-  std::vector<PassDesc<R>> d[5][2];  // by pass family and part
-  // the descriptor of patch i in family f: in the part of its plan
-  auto add = [&](int f, int i, int cls, size_t smem, PassDesc<R> &q) {
-    const int part = cls ? 0 : 1;
-    BatchPart &bp = lay.pass[f].part[part];
+  std::vector<PassDesc<R>> all[5], d[5][2];  // by pass family, and by part of it
+  std::vector<size_t> smem[5];
+  auto add = [&](int f, int i, int cls, size_t sm, PassDesc<R> &q) {
     q.patch = i;
     q.cls = cls;
-    q.first = bp.nitems;
-    bp.nitems += q.ntiles;
-    bp.npatch++;
-    bp.smem = std::max(bp.smem, smem);
-    d[f][part].push_back(q);
+    all[f].push_back(q);
+    smem[f].push_back(sm);
   };
+  long long rows = 0;
+  for (int i = 0; i < n; i++) rows += (long long)g[i].P[1] * g[i].P[2];
   std::vector<GhostDesc> gd[3];
   for (int i = 0; i < n; i++) {
     const SolveGeom<R> &gi = g[i];
@@ -405,7 +407,7 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
     // x forward and x inverse (rows per tile as the single-plan passes, within the slack)
     for (int inv = 0; inv < 2; inv++) {
       const int f = inv ? 4 : 0;
-      const XShape sh = x_shape<R, NC>(gi, inv != 0, BATCH_SMEM_SLACK);
+      const XShape sh = x_shape<R, NC>(gi, inv != 0, BATCH_SMEM_SLACK, rows);
       if (sh.rb <= 0 || sh.pairs != (sizeof(R) == 4)) return -1;
       const int RB = sh.rb;
       const size_t sm = x_smem(gi.lx, gi.N2, gi.H, gi.P[0], NC, RB, sizeof(R), sh.pairs, inv != 0);
@@ -461,6 +463,28 @@ int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *
       q.first = lay.ghost[a].total;
       lay.ghost[a].total += q.total;
       gd[a].push_back(q);
+    }
+  }
+  // A patch goes to the part of its plan.  A family whose tiles all fit on the GPU at once runs
+  // as one part, of run-time plans: its time is that of a tile, and a second launch adds
+  // another.  Microseconds, two parts / one: 2 patches of up to 64 cells 84 / 66, of up to 40
+  // 93 / 83; with four tiles an SM for the limit 12 patches 224 / 228
+  for (int f = 0; f < 5; f++) {
+    long long items = 0, compiled = 0;
+    for (const PassDesc<R> &q : all[f]) {
+      items += q.ntiles;
+      if (q.cls) compiled += q.ntiles;
+    }
+    const bool one = compiled < items && items <= 3ll * num_sms();
+    for (size_t k = 0; k < all[f].size(); k++) {
+      PassDesc<R> &q = all[f][k];
+      if (one) q.cls = 0;
+      BatchPart &bp = lay.pass[f].part[q.cls ? 0 : 1];
+      q.first = bp.nitems;
+      bp.nitems += q.ntiles;
+      bp.npatch++;
+      bp.smem = std::max(bp.smem, smem[f][k]);
+      d[f][q.cls ? 0 : 1].push_back(q);
     }
   }
   // chunks of work items: about eight per CTA slot of the GPU
