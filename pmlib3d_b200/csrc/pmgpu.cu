@@ -429,8 +429,9 @@ static void lineplan_tables(const LinePlan &pl, std::vector<int> &freq, std::vec
 // half a cycle of the SM an instruction).  Along z (axis 2) the last digit is done
 // together with the multiply when it is small enough (z_mid_radix): worth its round
 // trip; an even one pays four instructions for its bank conflicts.  Split plans hold
-// both halves of a first-phase butterfly, so digit 0 is at most 12 (FP64: 8).
-static std::vector<RadixSeq> line_candidates(int n, int split, int axis, int rsize, bool one_group = false) {
+// both halves of a first-phase butterfly, so digit 0 is at most `first`.
+static int split_limit(int axis, int rsize) { return rsize == 4 || axis == 0 ? 12 : 8; }
+static std::vector<RadixSeq> line_candidates(int n, int split, int axis, int rsize, bool one_group, int first) {
   static const int S[] = {24, 22, 20, 18, 17, 16, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
   std::vector<RadixSeq> out;
   auto add = [&](int np, int a, int b, int c) {
@@ -439,7 +440,7 @@ static std::vector<RadixSeq> line_candidates(int n, int split, int axis, int rsi
     q.r[0] = a;
     q.r[1] = b;
     q.r[2] = c;
-    if (split && a > (rsize == 4 || axis == 0 ? 12 : 8)) return;
+    if (split && a > first) return;
     LinePlan pl;
     lineplan_from(n, split, q.r, np, one_group, pl);
     q.cost = 0.0;
@@ -538,17 +539,19 @@ static bool make_lineplan(int M, bool half, int axis, int rsize, LinePlan &pl) {
       lineplan_from(n, split, q.r, q.r[2] > 1 ? 3 : q.r[1] > 1 ? 2 : 1, false, pl);
       return true;
     }
-  // A half whose factors leave only first digits that spill over two halves (FP64 y and z: 11,
-  // 13, 17, 121, ... 289; else 13, 17, 169, 221, 289): the whole line, which skips the zero
-  // rows, and not a convolution of 1.5 times it.  Solves of thin grids in microseconds, whole
-  // line / convolution: FP64 121 points along y 177 / 288, along z 169 / 434; 289 along z FP64
-  // 210 / 603, FP32 106 / 239; 442 along x FP32 265 / 355.  Split digits all the same: within
-  // 8 % of the whole line at 11 and 13, up to 30 % slower at 17
-  for (const int sp : {split, 0}) {
-    const int len = sp ? n : M;
-    const std::vector<RadixSeq> c = line_candidates(len, sp, axis, rsize);
+  // A half without a first digit inside the limit (13, 17, 169, 221, 289 points; FP64 along y
+  // and z also 11, 121, 143, 187): first digits up to 13, at some spilling, then (17, 289) the
+  // whole line, which skips the zero rows; not a convolution of 1.5 times the line.  Solves in
+  // microseconds, split / whole / convolution on thin grids: 121 points along y FP64 167 / 177 /
+  // 288, along z 178 / 169 / 434; 289 along z FP32 139 / 106 / 239.  Split / whole on 112 x 152
+  // cells by 113 (121 points) FP64: 730 / 725, with reprojection 1359 / 1443; by 281 (289) 2412 /
+  // 1979
+  const int tries[][2] = {{split, split_limit(axis, rsize)}, {split, 13}, {0, 0}};
+  for (const auto &t : tries) {
+    const int len = t[0] ? n : M;
+    const std::vector<RadixSeq> c = line_candidates(len, t[0], axis, rsize, false, t[1]);
     if (c.empty()) continue;
-    lineplan_from(len, sp, c[0].r, c[0].np, false, pl);
+    lineplan_from(len, t[0], c[0].r, c[0].np, false, pl);
     return true;
   }
   return false;
@@ -585,7 +588,7 @@ static bool make_bluestein(int n, int rows, int axis, int rsize, LinePlan &pl) {
   const int least = n + rows - 1;
   double best = 1e30;
   for (int m = least; m <= 2 * least && (m <= least + least / 3 || best > 1e29); m++) {
-    const std::vector<RadixSeq> c = line_candidates(m, 0, axis ? 1 : 0, rsize, true);
+    const std::vector<RadixSeq> c = line_candidates(m, 0, axis ? 1 : 0, rsize, true, 0);
     if (c.empty() || m * (c[0].cost + 16.0) >= best) continue;
     best = m * (c[0].cost + 16.0);
     lineplan_from(m, 0, c[0].r, c[0].np, true, pl);
@@ -1393,12 +1396,14 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
   const LinePlan now = axis == 1 ? pl->ly : pl->lz;
   const int split = now.split, m = now.n, rsize = (int)sizeof(R);
   int whole[LP_MAX], np = 0;
-  std::vector<RadixSeq> cands = line_candidates(m, split, axis, rsize);
+  std::vector<RadixSeq> cands = line_candidates(m, split, axis, rsize, false, split_limit(axis, rsize));
   cands.erase(std::remove_if(cands.begin(), cands.end(),
                              [&](const RadixSeq &c) { return !schedule_radices(c.r, c.np, split, rsize, whole, np); }),
               cands.end());
   if (cands.size() > 8) cands.resize(8);
-  if (!schedule_radices(now.rad, now.np, split, rsize, whole, np))
+  // and the plan as it is
+  auto current = [&](const RadixSeq &c) { return c.np == now.np && std::equal(c.r, c.r + c.np, now.rad); };
+  if (std::none_of(cands.begin(), cands.end(), current))
     cands.push_back(RadixSeq{now.np, {now.rad[0], now.rad[1], now.rad[2]}, 0.0});
   struct Spectra {
     DevBuf a, b;
