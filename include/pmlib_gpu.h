@@ -237,18 +237,22 @@ int pmgpu_batch_mode(int fused);
 int pmgpu_batch_fused(const pmgpu_batch *batch);
 
 /* Selects the line-FFT engine of plans created afterwards (no counterpart in the
- * reference): 0 = in-place register passes wherever the y / z lengths factor into
- * radices up to 17 (default), 1 = out-of-place Stockham passes everywhere.  Both give
- * the same results to round-off; returns the previous setting. */
+ * reference): 0 = in-place register passes, directly where a length factors into
+ * radices up to 17 and by Bluestein's algorithm elsewhere (default), 1 = out-of-place
+ * Stockham passes everywhere.  Both give the same results to round-off; returns the
+ * previous setting. */
 int pmgpu_fft_engine(int engine);
 
 /* Lets the line passes of 3-component fields run kernels compiled for their plan
- * where one exists (y / z: length, radices and kx tile; x: the packed transform's
- * plan, rows per tile, row length and spectrum pitch known to the compiler): 1 = on
- * (default), 0 = the run-time register engine only (no counterpart in the
- * reference).  The arithmetic is the same either way (results agree to round-off);
- * returns the previous setting. */
+ * where one exists (length, radices and the lines of a tile known to the compiler):
+ * 1 = on (default), 0 = the run-time register engine only (no counterpart in the
+ * reference).  The arithmetic is the same either way (bit-identical results); returns
+ * the previous setting. */
 int pmgpu_fft_specialised(int on);
+
+/* Which passes of the plan's plain velocity solve run a kernel compiled for their plan
+ * at the present setting: x forward, y forward, z, y inverse, x inverse (1 or 0). */
+int pmgpu_plan_compiled(const pmgpu_plan *plan, int compiled[5]);
 
 /* Global particle diagnostics accumulated in FP64 for FP32 or FP64 particle arrays
  * (device pointers, (3, npart) component fastest), the quantities of
@@ -264,9 +268,12 @@ int pmgpu_particle_diagnostics(const double dx[3], const void *d_pos, const void
 /* Schedule autotuner (no counterpart in the reference).  While on, creating a plan
  * times, for every y / z transform length and precision not measured before, the y
  * forward pass and the fused z pass with the best few radix sequences (by the
- * engine's cost model) and kx tiles of 8, 4 and 2, and keeps the fastest for this and
- * later plans of that length (process-wide; plans made with tuning off also use the
- * table).  Tuning adds tens of milliseconds per new length to plan creation.  pmgpu_fft_tune returns the previous setting; pmgpu_fft_tuned reads
+ * engine's cost model) and kx tiles of 8 (FP32), 4 and 2, and keeps the fastest for this
+ * and later plans of that length (process-wide; plans made with tuning off also use the
+ * table).  An entry holds radices of the whole line, which pmgpu_fft_set_schedule takes
+ * and any line of the length can run; a length whose default plan has no such radices
+ * and is fastest gets none.  Tuning adds tens of milliseconds per new length to plan
+ * creation.  pmgpu_fft_tune returns the previous setting; pmgpu_fft_tuned reads
  * entry `index` of the table (radices[3], 0-padded), -1 past the end. */
 int pmgpu_fft_tune(int on);
 int pmgpu_fft_tuned(int index, int *length, int *precision, int *axis, int *radices, int *tile,
@@ -274,8 +281,9 @@ int pmgpu_fft_tuned(int index, int *length, int *precision, int *axis, int *radi
 /* Puts a schedule into the table for plans created afterwards (a saved tuning, or a
  * schedule to test): radices[3] outermost first, 0-padded, multiplying to `length`;
  * FP32 may also use the wide composite radices 18, 20, 22, 24 (two-phase schedules
- * such as 528 = 22 x 24); tile 0 lets the plan choose.  radices = NULL removes the
- * entry. */
+ * such as 528 = 22 x 24); tile 0 lets the plan choose.  A line padded with zeros is
+ * transformed as two halves, and the factor 2 comes off the first radix (or off the
+ * largest even one).  radices = NULL removes the entry. */
 int pmgpu_fft_set_schedule(int length, int precision, int axis, const int *radices, int tile);
 
 /* ---- allocation-free deposition (no counterpart in the reference) ----

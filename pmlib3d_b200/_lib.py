@@ -27,7 +27,7 @@ EXPORTS = (
     "pmgpu_output_mesh", "pmgpu_output_pvti", "pmgpu_output_topology", "pmgpu_output_particles",
     "pmgpu_input_particles", "pmgpu_poisson_setup_ppf", "pmgpu_p2m_sort_order",
     "pmgpu_poisson_setup_pff", "pmgpu_inject_alloc_failure", "pmgpu_batch_mode", "pmgpu_batch_fused",
-    "pmgpu_penalisation_stage_dev",
+    "pmgpu_penalisation_stage_dev", "pmgpu_plan_compiled",
 )
 
 
@@ -96,6 +96,7 @@ def lib():
         "pmgpu_interp_particle_mesh_noalloc": [TP, QP, vp, vp, C.c_int, C.c_int, vp, C.c_int, C.c_int, C.c_int, vp],
         "pmgpu_fft_engine": [C.c_int],
         "pmgpu_fft_specialised": [C.c_int],
+        "pmgpu_plan_compiled": [vp, ip],
         "pmgpu_inject_alloc_failure": [C.c_longlong],
         "pmgpu_poisson_solve_dev": [vp, vp, vp, vp, C.c_int, C.c_int, C.c_int, vp],
         "pmgpu_batch_create": [C.c_int, PP, TP, QP, C.c_int, C.POINTER(vp)],

@@ -141,7 +141,6 @@ template <typename R, int NC>
 int inv_yx(SolveGeom<R> &g, const pmgpu_topo *topo, typename cplx_t<R>::type *Y, typename cplx_t<R>::type *X, R *out,
            cudaStream_t st, const char *caller, int cs = NC, bool ghosts = true);
 
-// one pass along y (forward X -> Y, or inverse Y -> X)
 // fills `desc` (host bytes) and `lay` for the velocity solve of n patches of
 // geometries g[i] with work spectra X[i], Y[i] (run_solve's layout); -1 if a patch
 // needs a pass the batched kernels do not run (the Stockham fallback)
@@ -149,13 +148,20 @@ template <typename R, int NC>
 int batch_layout(int n, const SolveGeom<R> *g, typename cplx_t<R>::type *const *X,
                  typename cplx_t<R>::type *const *Y, const pmgpu_topo *const *topo, std::vector<unsigned char> &desc,
                  BatchLayout &lay, const char *caller);
-// queues the batched solve: d_desc holds the descriptors, counters 5 zeroed words
+// queues the batched solve: d_desc holds the descriptors; counters: BATCH_COUNTERS words, two
+// parts a pass family, cleared here
+constexpr int BATCH_COUNTERS = 10;
 template <typename R, int NC>
 int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters, const void *const *vort,
                  void *const *vel, cudaStream_t st, const char *caller);
+// one pass along y (forward X -> Y, or inverse Y -> X)
 template <typename R, int NC>
 int ypass(SolveGeom<R> &g, const typename cplx_t<R>::type *X, typename cplx_t<R>::type *Y, int inverse,
           cudaStream_t st, const char *caller);
+
+// whether the passes of a plain velocity solve (x forward, y forward, z, y inverse, x inverse)
+// run kernels compiled for their plan
+template <typename R, int NC> void compiled_passes(const SolveGeom<R> &g, int compiled[5]);
 
 // each pass unit holds its own copy of the DFT constant tables
 int upload_cs_f32_1(const void *t32, const void *t64);

@@ -530,7 +530,7 @@ __device__ inline DepPos dep_share_start(long long s, long long nshare, int ntx,
 // the bin layer in the middle of its stencil that reach the tile, plus half a full tile for
 // the staging round trip; k_dep_shares cuts the units (tile by tile, layer by layer) into
 // ranges of equal cost, shares[s] = first unit of share s.  The shares move only the
-// boundaries between CTAs: a cell's sum and its order stay the same.  192 x 168 x 184 cells
+// boundaries between CTAs: a cell's sum and its order stay the same.  200 x 168 x 184 cells
 // with particles in two vortex cores, FP32: deposit 361 us with shares by cells, 209 us.
 constexpr int DEP_SHARE_UNITS = 1024;
 __global__ void __launch_bounds__(256) k_dep_cost(const unsigned *__restrict__ start, int ext0, int ext1, int ext2,
@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(M2P_THREADS) k_m2p_tile(PartGeom<R> g, const R
   R *cells = reinterpret_cast<R *>(smem_raw);
   __shared__ int rs[NR + 1], rg[NR];
   // tile origin in bins; org (<= 0) puts the tile edges on the first interior bin, so
-  // that one particle per cell fills whole 32-bin rows (warp-aligned, no empty tiles)
+  // that one particle per cell fills the first tile's rows (no tile of ghost bins alone)
   const int x0 = blockIdx.x * M2P_TX + org.x, y0 = blockIdx.y * M2P_TY + org.y, z0 = blockIdx.z * M2P_TZ + org.z;
   const int cx0 = x0 - (W - 1), cy0 = y0 - (W - 1), cz0 = z0 - (W - 1);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;

@@ -178,6 +178,52 @@ template <typename R> static LineTiles line_tiles(const SolveGeom<R> &g, int axi
   return lt;
 }
 
+// The kernel of a register-engine line pass of shape sh; compiled: one of its plan's own.
+template <typename R, int NC>
+static LinesKernel<R> pick_lines(const SolveGeom<R> &g, int axis, int lmode, int zmode, int use_zeta, const LineShape &sh,
+                                 bool &compiled) {
+  const bool pairs = sizeof(R) == 4 && sh.tk > 1;
+  LinesKernel<R> kern = nullptr;
+  if constexpr (NC == 3) {
+    const bool plain = lmode != L_Z || (zmode == Z_VEL && z_plain(g, use_zeta));
+    if (g_fft_ct && plain && (pairs || sizeof(R) == 8))
+      kern = lines_kernel_ct<R>(lmode, axis == 1 ? g.ly : g.lz, NC * sh.tk / (pairs ? 2 : 1));
+  }
+  compiled = kern != nullptr;
+  return compiled ? kern : lines_kernel<R>(pairs);
+}
+// The kernels of register-engine x passes, the same way.
+template <typename R, int NC> static RxfKernel<R> pick_xfwd(const SolveGeom<R> &g, const XShape &sh, bool &compiled) {
+  RxfKernel<R> kern = nullptr;
+  if constexpr (NC == 3)
+    if (g_fft_ct && (sh.pairs || sizeof(R) == 8)) kern = rxfwd_kernel_ct<R>(g.lx, NC * sh.rb / (sh.pairs ? 2 : 1));
+  compiled = kern != nullptr;
+  return compiled ? kern : rxfwd_kernel<R, NC>(sh.pairs);
+}
+template <typename R, int NC> static RxiKernel<R> pick_xinv(const SolveGeom<R> &g, const XShape &sh, bool &compiled) {
+  RxiKernel<R> kern = nullptr;
+  if constexpr (NC == 3)
+    if (g_fft_ct && (sh.pairs || sizeof(R) == 8)) kern = rxinv_kernel_ct<R>(g.lx, NC * sh.rb / (sh.pairs ? 2 : 1));
+  compiled = kern != nullptr;
+  return compiled ? kern : rxinv_kernel<R, NC>(sh.pairs);
+}
+
+template <typename R, int NC> void compiled_passes(const SolveGeom<R> &g, int compiled[5]) {
+  const long long rows = (long long)g.P[1] * g.P[2];
+  bool c[5] = {false, false, false, false, false};
+  for (int inv = 0; inv < 2; inv++) {
+    const XShape sh = x_shape<R, NC>(g, inv != 0, 0, rows);
+    if (sh.rb > 0 && inv) pick_xinv<R, NC>(g, sh, c[4]);
+    else if (sh.rb > 0) pick_xfwd<R, NC>(g, sh, c[0]);
+  }
+  for (int f = 1; f <= 3; f++) {
+    const int axis = f == 2 ? 2 : 1;
+    const LineShape sh = line_shape<R, NC>(g, axis, 0);
+    if (sh.tk > 0) pick_lines<R, NC>(g, axis, f == 1 ? L_FWD : f == 2 ? L_Z : L_INV, Z_VEL, 0, sh, c[f]);
+  }
+  for (int f = 0; f < 5; f++) compiled[f] = c[f];
+}
+
 template <typename R, int NC>
 static int launch_lines(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typename cplx_t<R>::type *out, int axis,
                         int lmode, int zmode, int reproj, int use_zeta, const LineTiles &tiles, cudaStream_t st,
@@ -193,13 +239,8 @@ static int launch_lines(SolveGeom<R> &g, const typename cplx_t<R>::type *in, typ
     lt.TK = sh.tk;
     lt.dLG = make_fastdiv((unsigned)(NC * sh.tk / (pairs ? 2 : 1)));
     const size_t sm = line_smem(pl, NC, sh.tk, sizeof(R));
-    const int lg = NC * sh.tk / (pairs ? 2 : 1);
-    LinesKernel<R> kern = nullptr;
-    if constexpr (NC == 3) {
-      const bool plain = lmode != L_Z || (zmode == Z_VEL && z_plain(g, use_zeta));
-      if (g_fft_ct && plain && (pairs || sizeof(R) == 8)) kern = lines_kernel_ct<R>(lmode, pl, lg);
-    }
-    if (!kern) kern = lines_kernel<R>(pairs);
+    bool compiled;
+    const LinesKernel<R> kern = pick_lines<R, NC>(g, axis, lmode, zmode, use_zeta, sh, compiled);
     if (smem_attr((const void *)kern, sm, caller)) return -1;
     int per = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, sh.threads, sm) != cudaSuccess || per < 1) per = 1;
@@ -249,14 +290,8 @@ static int xfwd(SolveGeom<R> &g, const R *in, typename cplx_t<R>::type *X, cudaS
       CKL(caller);
       return 0;
     };
-    auto kern = rxfwd_kernel<R, NC>(sh.pairs);
-    if constexpr (NC == 3) {
-      if (g_fft_ct && (sh.pairs || sizeof(R) == 8)) {
-        const auto ck = rxfwd_kernel_ct<R>(g.lx, NC * sh.rb / (sh.pairs ? 2 : 1));
-        if (ck) kern = ck;
-      }
-    }
-    if (launch(kern, sh.pairs ? 2 : 1)) return -1;
+    bool compiled;
+    if (launch(pick_xfwd<R, NC>(g, sh, compiled), sh.pairs ? 2 : 1)) return -1;
     return 0;
   }
   const int ntwx = g.fx.ntw + g.fx.next;
@@ -352,14 +387,8 @@ int inv_yx(SolveGeom<R> &g, const pmgpu_topo *topo, typename cplx_t<R>::type *Y,
       CKL(caller);
       return 0;
     };
-    auto kern = rxinv_kernel<R, NC>(sh.pairs);
-    if constexpr (NC == 3) {
-      if (g_fft_ct && (sh.pairs || sizeof(R) == 8)) {
-        const auto ck = rxinv_kernel_ct<R>(g.lx, NC * sh.rb / (sh.pairs ? 2 : 1));
-        if (ck) kern = ck;
-      }
-    }
-    if (launch(kern, sh.pairs ? 2 : 1)) return -1;
+    bool compiled;
+    if (launch(pick_xinv<R, NC>(g, sh, compiled), sh.pairs ? 2 : 1)) return -1;
   } else {
     const int ntwx = g.fx.ntw + g.fx.next;
     const int RB = pick_rb(g.N2, g.P[0], g.Hp, NC, sizeof(C), sizeof(R), ntwx, true);
@@ -526,7 +555,7 @@ int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters,
     vin.p[i] = vort[i];
     vout.p[i] = vel[i];
   }
-  CK(cudaMemsetAsync(counters, 0, 10 * sizeof(unsigned), st), caller);
+  CK(cudaMemsetAsync(counters, 0, BATCH_COUNTERS * sizeof(unsigned), st), caller);
   const char *base = reinterpret_cast<const char *>(d_desc);
   // one part of a pass family; a family's patches differ in their phases: four CTAs of 128
   // threads where they fit
@@ -595,6 +624,7 @@ int batch_launch(const BatchLayout &lay, const void *d_desc, unsigned *counters,
 #define PMGPU_INSTANTIATE_BATCH(R, NC)                                                                         \
   namespace pmgpu {                                                                                            \
   template int ghost_fill_all<R>(const pmgpu_topo *, R *, int, cudaStream_t, const char *);                    \
+  template void compiled_passes<R, NC>(const SolveGeom<R> &, int[5]);                                          \
   template int batch_layout<R, NC>(int, const SolveGeom<R> *, cplx_t<R>::type *const *,                        \
                                    cplx_t<R>::type *const *, const pmgpu_topo *const *,                        \
                                    std::vector<unsigned char> &, BatchLayout &, const char *);                 \

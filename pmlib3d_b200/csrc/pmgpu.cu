@@ -1032,7 +1032,6 @@ template <typename R> static SolveGeom<R> solve_geom(const pmgpu_plan *pl) {
   g.kxv = pl->kxv.as<R>();
   g.kzv = pl->kzv.as<R>();
   g.zoff = pl->zoff.as<int>();
-  g.gH = pl->g.Hp;
   g.yk = pl->ry_ok ? pl->yk.as<int>() : nullptr;
   g.zk = pl->rz_ok ? pl->zk.as<int>() : nullptr;
   return g;
@@ -1377,7 +1376,7 @@ template <typename R> static int line_upload(const LinePlan &lp, LineBufs &t, co
              : 0;
 }
 template <typename R>
-static int zvel_upload(const pmgpu_plan *pl, const LinePlan &, LineBufs &t, const char *caller) {
+static int zvel_upload(const pmgpu_plan *pl, LineBufs &t, const char *caller) {
   std::vector<R> kzv;
   std::vector<int> zoff;
   zvel_tables<R>(pl, t.hfreq, kzv, zoff);
@@ -1439,7 +1438,7 @@ template <typename R> static int tune_axis(pmgpu_plan *pl, int axis, TunedSchedu
         g.yk = tabs.freq.as<int>();
         g.tky = tk;
       } else {
-        if (zvel_upload<R>(pl, lp, tabs, caller)) break;
+        if (zvel_upload<R>(pl, tabs, caller)) break;
         g.lz = lp;
         g.rz_ok = 1;
         g.rtwz = tabs.tw.as<C>();
@@ -2530,6 +2529,17 @@ int pmgpu_fft_specialised(int on) {
   return old;
 }
 
+int pmgpu_plan_compiled(const pmgpu_plan *plan, int compiled[5]) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  if (!plan || !compiled) {
+    set_error("pmgpu_plan_compiled", "missing argument.");
+    return -1;
+  }
+  if (plan->prec == PMGPU_FP64) compiled_passes<double, 3>(solve_geom<double>(plan), compiled);
+  else compiled_passes<float, 3>(solve_geom<float>(plan), compiled);
+  return 0;
+}
+
 // ------------------------------------------------------------------ batches of patches
 // Independent solves of patches of uneven sizes and boundary types.  Each patch has
 // its own plan (work buffers; the Green's spectra are shared through the cache when
@@ -2589,7 +2599,7 @@ template <typename R> static int batch_fuse(pmgpu_batch *b, const char *caller) 
   }
   std::vector<unsigned char> host;
   if (batch_layout<R, 3>(n, geo.data(), X.data(), Y.data(), topo.data(), host, b->lay, caller)) return 0;
-  if (b->desc.ensure(host.size(), caller) || b->counters.ensure(10 * sizeof(unsigned), caller)) return -1;
+  if (b->desc.ensure(host.size(), caller) || b->counters.ensure(BATCH_COUNTERS * sizeof(unsigned), caller)) return -1;
   CK(cudaMemcpy(b->desc.p, host.data(), host.size(), cudaMemcpyHostToDevice), caller);
   b->fused = true;
   return 0;

@@ -6,9 +6,10 @@
 // transforms back and keeps REAL().  The 3-D DFT is separable, so the result does
 // not depend on the axis order; here the passes always run x, y, z:
 //
-//   x_fwd : real cuboid -> X[z][y][kx][c], kx < H = Mx/2+1   (R2C, zero-pad fused)
-//   y_fwd : X -> Y[z][ky][kx][c], ky < My                      (C2C, zero-pad fused)
-// (the kx extent of X and Y is padded to Hp, a multiple of 8, for aligned tiles)
+//   x_fwd : real cuboid -> X, kx < H = Mx/2+1                 (R2C, zero-pad fused)
+//   y_fwd : X -> Y, ky < My                                     (C2C, zero-pad fused)
+// (X is stored [z][kx block][y][kx in block][c], Y the same with the ky rows, in blocks of
+// spec_block kx; the kx extent is padded to Hp, a multiple of 8)
 //   z_pass: Y -> Y (or another buffer): pad, FFT, multiply+curl, iFFT, truncate
 //   y_inv : Y -> X (truncate to the pencil extent)
 //   x_inv : X -> real cuboid                                     (C2R, truncate fused)
@@ -38,7 +39,7 @@ template <typename R> struct SolveGeom {
   FftDesc fx, fy, fz;
   const C *twx, *twy, *twz;
   const R *kxt, *kyt, *kzt;  // wavenumbers (cycles / length), Nyquist index included
-  const R *green;            // real octant G(kx, |ky|, |kz|) * dx dy dz / (Mx My Mz)
+  const R *green;            // real octant G(kx, |ky|, |kz|) * dx dy dz / (Mx My Mz), rows of Hp
   int gM1, gM2;              // My / 2 + 1, Mz / 2 + 1
   int kernel2;               // derivative kernel (3 components); green holds its spectrum
   R scale;                   // 1 / (Mx My Mz)
@@ -64,7 +65,6 @@ template <typename R> struct SolveGeom {
   // offset of the octant plane |kz|
   const R *kxv, *kzv;
   const int *zoff;
-  int gH;                    // row pitch of the octants (kx entries beyond H are zero)
 };
 
 enum ZMode { Z_VEL = 0, Z_VORT = 1, Z_VECPOT = 2, Z_REGULARISE = 3, Z_FORWARD = 4 };
@@ -137,7 +137,7 @@ struct NoHook {
 
 // ---------------------------------------------------------------- y and z passes
 // Tile t = (outer o, kx-tile kt): L = NC * TK lines of n points.  Row r of the tile
-// starts at complex offset ((o * os + kt * TK) + r * rs) * NC and holds L complex.
+// starts at complex offset (spec_off(o * os, kb, kt * TK) + r * rs) * NC and holds L complex.
 struct LineTiles {
   int n;          // transform length
   int rows_in;    // rows read (the rest is zero padding)
@@ -235,9 +235,9 @@ __device__ __forceinline__ void z_point(const SolveGeom<R> &g, typename cplx_t<R
       // i S_c + (-1)^(k_c) E_c, S_c odd along axis c and even along the others
       // (stored for |ky|, |kz| with the sign of the odd axis applied here), E_c the
       // spectrum of the kernel's plane at -M_c/2 dx_c
-      const size_t noct = (size_t)g.gM2 * g.gM1 * g.gH;
+      const size_t noct = (size_t)g.gM2 * g.gM1 * g.Hp;
       const int iz = min(z, g.M[2] - z);
-      const size_t oc = ((size_t)iz * g.gM1 + iy) * g.gH + kx_i;
+      const size_t oc = ((size_t)iz * g.gM1 + iy) * g.Hp + kx_i;
       const R *E = g.green + 3 * noct;
       R sx = g.green[oc], sy = g.green[noct + oc], sz = g.green[2 * noct + oc];
       if (2 * y > g.M[1]) sy = -sy;
@@ -344,7 +344,7 @@ __device__ __forceinline__ void z_multiply(const SolveGeom<typename LineT<T>::R>
     for (int h = 0; h < G; h++) {
       const int kx_i = k0 + kk * G + h;
       const R kxp = kx_i < g.H ? g.kxt[kx_i] : R(0);
-      const R Gp = pre ? g.green[((size_t)min(z, g.M[2] - z) * g.gM1 + iy) * g.gH + kx_i] : R(0);
+      const R Gp = pre ? g.green[((size_t)min(z, g.M[2] - z) * g.gM1 + iy) * g.Hp + kx_i] : R(0);
       typename cplx_t<R>::type v[NC];
 #pragma unroll
       for (int c = 0; c < NC; c++) v[c] = lane_get(a[c], h);
@@ -373,7 +373,7 @@ __device__ __forceinline__ void z_mid_vel(const SolveGeom<typename LineT<T>::R> 
   constexpr int G = LineT<T>::G;
   const int nk = LG / 3, nks = __ffs(nk) - 1;
   const T ky = pset(T(), (2 * y == g.M[1]) ? R(0) : R(6.283185307179586476925286766559) * g.kyt[y]);
-  const R *green = g.green + (size_t)min(y, g.M[1] - y) * g.gH + k0;
+  const R *green = g.green + (size_t)min(y, g.M[1] - y) * g.Hp + k0;
   const int total = (npts / RL) << nks;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
     const int beta = t >> nks, kk = t - (beta << nks);
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(PASS_THREADS, 1) k_lines(SolveGeom<R> g, LineT
 // position (row -> ky through g.yk); the z pass keeps its spectrum by position in shared
 // memory (position -> kz through g.zk).  Several CTAs share an SM so that one CTA's loads
 // overlap another's transforms.
-constexpr int LINE_THREADS_MAX = 256;   // 128 or 256 threads, at most 128 registers
+constexpr int LINE_THREADS_MAX = 256;   // 96 to 256 threads (pass_threads), at most 128 registers
 constexpr int LINE_CTAS = 2;
 
 struct LineSmem {

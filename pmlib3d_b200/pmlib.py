@@ -367,10 +367,19 @@ def fft_engine(engine: int) -> int:
 
 
 def fft_specialised(on: bool) -> int:
-    """Lets the y / z line passes run the kernels compiled for their plan where one
+    """Lets the x, y and z passes run the kernels compiled for their plan where one
     exists (default on); off: the run-time register engine only.  The results are
     bit-identical either way.  Returns the previous setting."""
     return lib().pmgpu_fft_specialised(1 if on else 0)
+
+
+def plan_compiled(plan) -> list:
+    """Which passes of the plan's plain velocity solve run a compiled kernel: x forward,
+    y forward, z, y inverse, x inverse."""
+    out = (C.c_int * 5)()
+    if lib().pmgpu_plan_compiled(plan.handle, out) != 0:
+        raise RuntimeError(last_error())
+    return [bool(v) for v in out]
 
 
 def step(plan: Plan, pos, part_vort, part_vel) -> int:

@@ -1,14 +1,15 @@
-"""Compile-time-plan line passes against the run-time register engine.
+"""Compile-time-plan passes against the run-time register engine.
 
-The y / z passes of 3-component fields run kernels compiled for their plan (length,
-radices, kx tile) where one exists, and so do the x passes (plan of the packed
-half-length transform, rows per tile); they do the arithmetic of the run-time engine
-in the same order, so the solves agree to round-off (the compiler may fuse a
-different multiply and add of an expression in the two builds).  The grids have y
-and z lines of 528 points (256 cells, four ghost layers, free), the length of the
-256^3 step, and the schedules are set to the compiled plans; the x-pass grid has 256
-free cells along x (264 reals a row, a 264-point packed transform).
+Every plan of line_plans.inc (x, y and z lines of three-component fields, FP32 and FP64, padded
+and periodic) on a thin grid with its length along its axis: the plan reports that the
+axis's passes run compiled kernels, none with them turned off, and velocity and reprojected
+vorticity agree bit for bit (the kernels do the run-time engine's arithmetic in its order,
+with products that are never contracted).  The last test takes the lengths of the 256^3 and
+512 x 512 x 256 steps together with several tiles along every axis.
 """
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -17,95 +18,64 @@ from tests.helpers import gaussian_field
 
 pytestmark = pytest.mark.gpu
 
-# (precision, y schedule, z schedule, kx tile)
-CASES = [
-    (P.FP32, (24, 22), (12, 11, 4), 8),
-    (P.FP32, (24, 22), (22, 24), 8),
-    (P.FP32, (22, 24), (12, 11, 4), 4),
-    (P.FP64, (12, 11, 4), (12, 11, 4), 8),
-    (P.FP64, (12, 11, 4), (8, 6, 11), 8),
-    (P.FP64, (12, 11, 4), (8, 6, 11), 4),
-]
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+H = 1.0 / 128
+AXES = "XYZ"
+PASSES = {0: (0, 4), 1: (1, 3), 2: (2,)}  # x forward and inverse, y forward and inverse, z
 
 
-YZ_BOX = ((-0.0625, -1.0, -1.0), (0.0625, 1.0, 1.0))
-X_BOX = ((-1.0, -0.0625, -0.0625), (1.0, 0.0625, 0.0625))
+def _plans():
+    txt = open(os.path.join(ROOT, "pmlib3d_b200", "csrc", "line_plans.inc")).read()
+    out = re.findall(r"^PMGPU_PLAN_([XYZ])_F(32|64)\((\d), (\d+),", txt, re.M)
+    return [(AXES.index(a), P.FP32 if p == "32" else P.FP64, int(s), int(n)) for a, p, s, n in out]
 
 
-def _solve(prec, sched, specialised, w, reproj, box=YZ_BOX, tile=8, length=528, h=1.0 / 128, bc=(0, 0, 0)):
+def _solve(n, bc, prec, specialised, w):
     old = P.fft_specialised(specialised)
     try:
-        for axis, rad in sched.items():
-            assert P.fft_set_schedule(length, prec, axis, rad, tile) == 0, P.last_error()
-        patch = P.make_patch(box[0], box[1], (h,) * 3, bound_cond=bc, nghost=4)
-        ierr, topo = P.pmlib_topology_cuboid(patch, 3)
+        pa = P.make_patch([-0.5 * H * c for c in n], [0.5 * H * c for c in n], (H,) * 3, bound_cond=bc, nghost=4)
+        ierr, topo = P.pmlib_topology_cuboid(pa, 3)
         assert ierr == 0
         params = P.make_params(order=6, kernel=1, radius=2.0, interp=3)
-        ierr, plan = P.pmlib_poisson_setup(patch, topo, params, prec)
+        for axis in (1, 2):  # the default plans, not a schedule measured earlier in the process
+            P.fft_set_schedule(n[axis] if bc[axis] else 2 * (n[axis] + 8), prec, axis, None)
+        ierr, plan = P.pmlib_poisson_setup(pa, topo, params, prec)
         assert ierr == 0, P.last_error()
-        dt = np.float32 if prec == P.FP32 else np.float64
-        wg = w.astype(dt)
-        vel = np.zeros(w.shape, dt)
-        assert P.pmlib_poisson_solve(plan, wg, vel, reproj=reproj) == 0, P.last_error()
+        wg = w(topo).astype(np.float32 if prec == P.FP32 else np.float64)
+        vel = np.zeros_like(wg)
+        assert P.pmlib_poisson_solve(plan, wg, vel, reproj=True) == 0, P.last_error()
+        compiled = P.plan_compiled(plan)
         plan.close()
-        return vel, wg, topo
+        return vel, wg, compiled
     finally:
         P.fft_specialised(old)
-        for axis in sched:
-            P.fft_set_schedule(length, prec, axis, None)
 
 
-@pytest.mark.parametrize("prec,ysched,zsched,tile", CASES)
-@pytest.mark.parametrize("reproj", [False, True])
-def test_specialised_equals_runtime_engine(prec, ysched, zsched, tile, reproj):
-    sched = {1: ysched, 2: zsched}
-    patch = P.make_patch((-0.0625, -1.0, -1.0), (0.0625, 1.0, 1.0), (1.0 / 128,) * 3, bound_cond=(0, 0, 0), nghost=4)
-    ierr, topo = P.pmlib_topology_cuboid(patch, 3)
-    w = gaussian_field(topo, seed=5, noise=0.05)
-    v1, w1, t1 = _solve(prec, sched, True, w, reproj, tile=tile)
-    v0, w0, _ = _solve(prec, sched, False, w, reproj, tile=tile)
-    assert np.abs(v1).max() > 0
-    tol = 2e-6 if prec == P.FP32 else 1e-14
-    for a, b in ((v1, v0), (w1, w0)):
-        d = np.linalg.norm((a.astype(np.float64) - b).ravel()) / np.linalg.norm(b.astype(np.float64).ravel())
-        assert d < tol, d
+def _compare(n, bc, prec, passes):
+    seed = sum(n)
+    v1, w1, c1 = _solve(n, bc, prec, True, lambda t: gaussian_field(t, seed=seed, noise=0.05))
+    v0, w0, c0 = _solve(n, bc, prec, False, lambda t: gaussian_field(t, seed=seed, noise=0.05))
+    assert all(c1[p] for p in passes), c1
+    assert not any(c0)
+    assert np.abs(v0).max() > 0 and np.abs(w0).max() > 0
+    assert np.array_equal(v1, v0) and np.array_equal(w1, w0)
 
 
-@pytest.mark.parametrize("prec", [P.FP32, P.FP64])
-@pytest.mark.parametrize("reproj", [False, True])
-def test_specialised_x_passes_equal_runtime_engine(prec, reproj):
-    patch = P.make_patch(X_BOX[0], X_BOX[1], (1.0 / 128,) * 3, bound_cond=(0, 0, 0), nghost=4)
-    ierr, topo = P.pmlib_topology_cuboid(patch, 3)
-    assert topo.ncell[0] == 256
-    w = gaussian_field(topo, seed=9, noise=0.05)
-    v1, w1, _ = _solve(prec, {}, True, w, reproj, box=X_BOX)
-    v0, w0, _ = _solve(prec, {}, False, w, reproj, box=X_BOX)
-    assert np.abs(v1).max() > 0
-    tol = 2e-6 if prec == P.FP32 else 1e-14
-    for a, b in ((v1, v0), (w1, w0)):
-        d = np.linalg.norm((a.astype(np.float64) - b).ravel()) / np.linalg.norm(b.astype(np.float64).ravel())
-        assert d < tol, d
+def test_all_plans_listed():
+    assert len(_plans()) == 154
 
 
-# the periodic 512-point lines of the 512 x 512 x 256 ppf grid: y lines under a
-# compiled schedule, and x rows of 512 periodic cells (a 256-point packed transform)
-PPF_Y_BOX = ((-0.0625, -1.0, -0.0625), (0.0625, 1.0, 0.0625))
-PPF_X_BOX = ((-1.0, -0.0625, -0.0625), (1.0, 0.0625, 0.0625))
+@pytest.mark.parametrize("axis,prec,split,points", _plans())
+def test_plan_equals_runtime_engine(axis, prec, split, points):
+    length = points * (1 + split) * (2 if axis == 0 else 1)  # x: the packed half-length transform
+    n, bc = [8, 8, 8], [0, 0, 0]
+    n[axis], bc[axis] = (length // 2 - 8, 0) if split else (length, 1)
+    _compare(n, tuple(bc), prec, PASSES[axis])
 
 
 @pytest.mark.parametrize("prec", [P.FP32, P.FP64])
-@pytest.mark.parametrize("case", ["y", "x"])
-def test_specialised_periodic_512_lines_equal_runtime_engine(prec, case):
-    h, bc = 1.0 / 256, (1, 1, 0)
-    box = PPF_Y_BOX if case == "y" else PPF_X_BOX
-    sched = {1: (8, 8, 8)} if case == "y" else {}
-    patch = P.make_patch(box[0], box[1], (h,) * 3, bound_cond=bc, nghost=4)
-    ierr, topo = P.pmlib_topology_cuboid(patch, 3)
-    assert topo.ncell[1 if case == "y" else 0] == 512
-    w = gaussian_field(topo, seed=11, noise=0.05)
-    v1, w1, _ = _solve(prec, sched, True, w, False, box=box, length=512, h=h, bc=bc)
-    v0, w0, _ = _solve(prec, sched, False, w, False, box=box, length=512, h=h, bc=bc)
-    assert np.abs(v1).max() > 0
-    tol = 2e-6 if prec == P.FP32 else 1e-14
-    d = np.linalg.norm((v1.astype(np.float64) - v0).ravel()) / np.linalg.norm(v0.astype(np.float64).ravel())
-    assert d < tol, d
+@pytest.mark.parametrize("n,bc,passes", [
+    ((256, 16, 56), (0, 0, 0), (0, 2, 4)), ((24, 256, 56), (0, 0, 0), (1, 2, 3)), ((24, 56, 256), (0, 0, 0), (1, 2, 3)),
+    ((512, 64, 56), (1, 1, 0), (0, 1, 2, 3, 4)), ((64, 512, 56), (1, 1, 0), (0, 1, 2, 3, 4))])
+def test_step_lengths_equal_runtime_engine(n, bc, passes, prec):
+    _compare(n, bc, prec, passes)
